@@ -4,52 +4,73 @@
 // Replaces gemm_w4a16 of the reference (src/kernels/gemm_w4a16.cu:63-88), which expands a
 // weight tile to bf16 in a 256 MB workspace (k_dequant_rows) and calls cublasGemmEx. Here no
 // bf16 copy of the weights ever touches global or shared memory:
-//   * one CTA per SM; a tile is 128 output rows x 256 tokens, its fp32 accumulator lives in 256
-//     columns of tensor memory;
-//   * a producer thread streams the packed int4 weight stream of the row tile through a ring of
+//   * a pair of CTAs (cta_group::2) computes a tile of 256 output rows x TN tokens: each CTA holds the weights
+//     and the fp32 accumulator of its own 128 rows in tensor memory and HALF of the tile's tokens in shared
+//     memory. A CTA alone (128 rows x 256 tokens) pulls 72 KB through L2 per k group and 1024 tensor
+//     cycles; a pair's CTA pulls 41 KB for the same math, which leaves room for four
+//     group stages of activations instead of two;
+//   * a producer thread per CTA streams the packed int4 blocks of its row tile through a ring of
 //     shared-memory stages with 1-D bulk async copies (cp.async.bulk + mbarrier);
-//   * eight dequant warps (one output row per thread, two k-halves) turn 16 bytes of nibbles
-//     into bf16 weights in registers - (128+q) by LOP3, minus (128+zp) and times the group
-//     scale with packed bf16 arithmetic, which is exactly bf16(float(q-zp)*float(s)), the value
-//     w4a16_dequant_rows produces - and store them as the A operand into tensor memory
-//     (tcgen05.st);
-//   * a second producer thread brings the activation tile in with tiled TMA loads
-//     (cp.async.bulk.tensor, 128-byte swizzle), which is the K-major B operand as is;
-//   * one thread issues tcgen05.mma (128 x 256 x 16, kind::f16) per 16-k slab, A from tensor
-//     memory, B from shared memory, and commits to mbarriers that recycle the A columns and the
-//     activation buffers;
-//   * the epilogue reads the accumulator back with tcgen05.ld, rounds to bf16 and stores C.
+//   * sixteen dequant warps per CTA (one output row and half a k group per thread; two teams take alternate
+//     groups) turn 32 bytes of nibbles into bf16 weights in registers - (128+q) by LOP3,
+//     minus (128+zp) and times the group scale with packed bf16 arithmetic, which is exactly
+//     bf16(float(q-zp)*float(s)), the value w4a16_dequant_rows produces - and store them as the A operand
+//     into tensor memory (tcgen05.st);
+//   * a second producer thread per CTA brings its half of the activation tile in with tiled TMA loads
+//     (cp.async.bulk.tensor, 128-byte swizzle), which is the K-major B operand as is; both CTAs' loads
+//     complete on the leader's mbarrier;
+//   * one thread of the leader CTA issues tcgen05.mma (256 x N x 16, kind::f16) per 16-k slab for both
+//     CTAs, and one commit per group tells both CTAs that the A columns and the stage are free;
+//   * eight epilogue warps per CTA read the accumulator back with tcgen05.ld into shared memory, hand it back to the
+//     issuer, and store C in 256-byte rows while the next tile's main loop runs;
+//   * few tiles (short prompts, narrow layers): a cluster of 2 S CTAs splits K S ways; the splits' fp32 tiles
+//     are added through distributed shared memory, always in split order (bitwise reproducible).
+//
+// What bounds it: long prompts run at the tensor cores' rate under the power cap (256 x 256 x 16 per 128 cycles; the
+// expansion of a group needs about 500 issue and ALU cycles of the 1024 its MMAs take), short ones at the
+// expansion of the weights. Measured against one CTA per tile of 128 x 256 with eight dequant warps:
+//   34816 x 5120, M = 4096: 1238 -> 890 us (1641 TFLOP/s); 5120 x 17408, M = 4096: 674 -> 475 us (1537)
+//   34816 x 5120, M = 777:   344 -> 202 us;                5120 x 8192, M = 777:   113 -> 82 us
+//   34816 x 5120, M = 77:     76 -> 52 us;                 5120 x 17408, M = 77:  108 -> 31 us
+// and on the way: half groups as the unit of every hand-off 1134 us (the first shape; the issuing thread is the
+// limit), whole groups 1063, two teams of dequant warps and C through shared memory 890.
 #include <cuda.h>
 #include <cstring>
+#include <mutex>
 
 #include "common.cuh"
 
 namespace w4a16 {
 namespace {
 
-constexpr int PW = 8;                       // dequant warps: 4 TMEM lane quadrants x 2 k-halves
-constexpr int kPWarps = PW + 3;             // + weight producer + MMA issuer + activation producer
-constexpr int TN = 256;                     // tokens per tile (N of the MMA)
-constexpr int kPNB = 3;                     // groups of A in flight in tensor memory
-constexpr uint32_t kPTmemCols = 512;        // A: kPNB x 64 columns, D: 256 columns
-constexpr uint32_t kPTmemA = 0, kPTmemD = 256;
-constexpr int kPD = 2;                      // weight ring stages (two groups each)
-constexpr int kPStage = 2 * kTileGroupBytes;
-constexpr int kPXBufs = 2;                  // activation group buffers
-constexpr int kPXBytes = TN * 128 * 2;      // one k group of the token tile: 64 KB
+constexpr int PW = 16;                      // dequant warps: 4 TMEM lane quarters x 2 halves of a k group x 2 groups
+constexpr int EW = 8;                       // epilogue warps: two per lane quarter, each half of the tokens
+constexpr int kWEpi0 = PW, kWWeights = PW + EW, kWIssue = kWWeights + 1, kWActs = kWIssue + 1;
+constexpr int kPWarps = kWActs + 1;
+constexpr int kPRows = 2 * kTileRows;       // output rows of a CTA pair's tile
+constexpr int kPMaxTN = 256;                // tokens of a tile: a multiple of 32 (the pair's MMA needs N % 32 == 0)
+constexpr int kPMaxSplit = 4;               // 2 S <= 8 CTAs: the portable cluster size
+constexpr int kPSteps = 4;                  // activation stages, each one k group of the CTA's TN / 2 tokens
+constexpr int kPDone = 8;                   // ring of "group multiplied" barriers: at least kPSteps and the A slots
+constexpr int kPMaxWD = 16;                 // weight ring stages (one k group each), at most
+constexpr uint32_t kPTmemCols = 512;
 constexpr uint32_t kPSpin = 1u << 20;
 constexpr uint32_t kMagicP = 0x43004300u, kNibMaskP = 0x000F000Fu;
-constexpr int kPBars = 2 * kPD + 2 * kPNB + 2 * kPXBufs + 2;
-// activation buffers come first: 128-byte-swizzled TMA tiles must start on a 1024-byte boundary
-constexpr int kPSmem = kPXBufs * kPXBytes + kPD * kPStage + kPBars * 8 + 16 + 1024;
+constexpr int kPMaxA = 6;                   // A slots, at most
+constexpr int kPBars = 2 * kPMaxWD + kPDone + kPMaxA + kPSteps + 2;
+// Tensor memory: the accumulator's TN columns, the rest are slots of the A operand, 64 columns per k group.
+__host__ __device__ constexpr int a_slots(int tn) { return tn <= 128 ? 6 : 4; }
+static_assert(128 + 6 * 64 <= 512 && 256 + 4 * 64 <= 512 && kPMaxA <= kPDone && kPSteps <= kPDone, "ring depths");
 
 struct PrefillParams {
-  CUtensorMap amap;   // A as [M][K] bf16, box 64 k x 256 tokens, 128-byte swizzle, zero fill
+  CUtensorMap amap;   // A as [M][K] bf16, box 64 k x TN / 2 tokens, 128-byte swizzle, zero fill
   const uint8_t* stream;
-  const uint16_t* A;  // [M][K] bf16
   uint16_t* C;        // [M][ldc] bf16; this launch's rows land in columns [col0, col0 + N)
-  int M, N, K, G, row_tiles, tok_tiles;
+  int M, N, K, G, row_tiles, pairs;  // pairs: row tiles in twos (an odd last one repeats the last tile and stores nothing)
+  int tn, splits, wdepth;            // wdepth is even: a stage is always read by the same dequant warps
+  int full_tt, tiles;                // token tiles of TN tokens; tiles in all (the ragged token tile's come last)
   long long ldc;
+  int wide;                          // C (and every peer's) takes 16-byte stores: base, ldc and col0 are multiples of that
   int col0;
   int* status;
   // column-sharded call: the other ranks' C (peer-mapped) receive the same tile, then the completion flag
@@ -66,10 +87,62 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
   return d;
 }
 
-// Tiled TMA load of a 64 x 256 box (k, token) into shared memory, completion on an mbarrier.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+// ---- CTA pairs and clusters --------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t saddr, uint32_t rank) {
+  uint32_t d;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(saddr), "r"(rank));
+  return d;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Arrival on a barrier of any CTA of the cluster (a mapped address). What it hands over is tensor memory, ordered by
+// the tcgen05 fences around it, so the barrier needs no cluster-scope release (which costs a memory fence).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+  return pred != 0;
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+// D[both CTAs' tmem] (+)= A[both CTAs' tmem] * B[half of the columns from each CTA's shared memory]
+__device__ __forceinline__ void umma_bf16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                                  uint32_t accumulate) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// One arrival on the barrier at this offset in every CTA of `mask` once all MMAs issued so far have completed.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t mask) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+      "h"(mask)
+      : "memory");
+}
+// Tiled TMA load of a 64 x TN / 2 box (k, token) into this CTA's shared memory; completion on the pair leader's mbarrier.
+__device__ __forceinline__ void tma_load_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::
           "r"(dst),
       "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
@@ -80,252 +153,393 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
          (static_cast<uint64_t>(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 
+// A tile: its row pair, first token and the tokens it multiplies (a multiple of 32; the ragged token tile has fewer).
+struct PTile {
+  int pair, tok0, n;
+};
+__device__ __forceinline__ PTile tile_of(const PrefillParams& p, int tile) {
+  const int nfull = p.pairs * p.full_tt;
+  PTile t;
+  if (tile < nfull) {  // token tiles of one row pair are neighbours: its weights stay in L2
+    t.pair = tile / p.full_tt;
+    t.tok0 = (tile - t.pair * p.full_tt) * p.tn;
+    t.n = p.tn;
+  } else {
+    t.pair = tile - nfull;
+    t.tok0 = p.full_tt * p.tn;
+    t.n = (p.M - t.tok0 + 31) & ~31;
+  }
+  return t;
+}
+
 __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_constant__ PrefillParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* xbuf = smem;
-  uint8_t* ring = xbuf + kPXBufs * kPXBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ring + kPD * kPStage);
+  const int xbytes = p.tn * 128;  // one activation stage: two swizzled tiles of TN / 2 tokens x 64 k
+  uint8_t* xbuf = smem;          // 128-byte-swizzled TMA tiles start on 1024-byte boundaries
+  uint8_t* cbuf = xbuf + kPSteps * xbytes;  // [TN tokens][128 rows] bf16: the finished tile on its way out
+  uint8_t* ring = cbuf + p.tn * (kTileRows * 2);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ring + p.wdepth * kTileGroupBytes);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kPBars);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int G = p.G;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const uint32_t rank = cluster_rank(), leader = rank & ~1u;
+  const int half = static_cast<int>(rank & 1u), split = static_cast<int>(rank >> 1);
+  const int WD = p.wdepth, S = p.splits;
+  const int na = a_slots(p.tn);
   const uint32_t ring_a = smem_u32(ring), xbuf_a = smem_u32(xbuf);
-  const uint32_t wfull_a = smem_u32(bars);
-  const uint32_t wempty_a = wfull_a + kPD * 8;
-  const uint32_t afull_a = wempty_a + kPD * 8;       // [kPNB] a group's A operand is in TMEM (8 warps)
-  const uint32_t mdone_a = afull_a + kPNB * 8;       // [kPNB] the MMAs reading that A have completed
-  const uint32_t xfull_a = mdone_a + kPNB * 8;       // [kPXBufs] activation group staged (4 warps)
-  const uint32_t xempty_a = xfull_a + kPXBufs * 8;   // [kPXBufs] the MMAs reading it have completed
-  const uint32_t ddone_a = xempty_a + kPXBufs * 8;   // accumulator of the tile is complete
-  const uint32_t alldone_a = ddone_a + 8;            // the dequant warps are finished with tensor memory
+  const uint32_t wfull_a = smem_u32(bars);               // [WD] weights of a group landed
+  const uint32_t wempty_a = wfull_a + kPMaxWD * 8;       // [WD] read by the 8 dequant warps
+  const uint32_t done_a = wempty_a + kPMaxWD * 8;        // [kPDone] group j % 8 multiplied (both CTAs get the commit)
+  const uint32_t dfull_a = done_a + kPDone * 8;          // accumulator complete (both CTAs)
+  const uint32_t afull_a = dfull_a + 8;                  // [na] leader: a group's A operand written (8 warps of each CTA)
+  const uint32_t xfull_a = afull_a + kPMaxA * 8;         // [kPSteps] leader: both CTAs' activations of a group landed
+  const uint32_t dempty_a = xfull_a + kPSteps * 8;       // leader: accumulator read out (the epilogue warps of both CTAs)
 
   if (tid == 0) {
-    for (int i = 0; i < kPD; ++i) {
+    for (int i = 0; i < kPMaxWD; ++i) {
       mbar_init(wfull_a + i * 8, 1);
-      mbar_init(wempty_a + i * 8, PW);
+      mbar_init(wempty_a + i * 8, 8);
     }
-    for (int i = 0; i < kPNB; ++i) {
-      mbar_init(afull_a + i * 8, PW);
-      mbar_init(mdone_a + i * 8, 1);
-    }
-    for (int i = 0; i < kPXBufs; ++i) {
-      mbar_init(xfull_a + i * 8, 1);
-      mbar_init(xempty_a + i * 8, 1);
-    }
-    mbar_init(ddone_a, 1);
-    mbar_init(alldone_a, PW);
+    for (int i = 0; i < kPDone; ++i) mbar_init(done_a + i * 8, 1);
+    for (int i = 0; i < kPSteps; ++i) mbar_init(xfull_a + i * 8, 1);
+    for (int i = 0; i < kPMaxA; ++i) mbar_init(afull_a + i * 8, 16);
+    mbar_init(dfull_a, 1);
+    mbar_init(dempty_a, 2 * EW);
     fence_mbar_init();
   }
-  if (warp == PW + 1) tmem_alloc(smem_u32(tmem_slot), kPTmemCols);
+  if (warp == kWIssue) tmem_alloc_pair(smem_u32(tmem_slot), kPTmemCols);
   tc_fence_before();
   __syncthreads();
+  cluster_sync();  // the other CTAs' barriers exist from here on
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem_a = tmem + (p.tn <= 128 ? 128 : 256);
 
-  const int ntiles = p.row_tiles * p.tok_tiles;
+  const int cluster = blockIdx.x / (2 * S), nclusters = gridDim.x / (2 * S);
+  const int g0 = p.G * split / S, g1 = p.G * (split + 1) / S;  // this split's k groups (S <= G)
+  bool dead = false;
 
-  // ================================================================ weight producer
-  if (warp == PW) {
+  if (warp == kWWeights) {
+    // ================================================================ weight producer
     if (lane == 0) {
       int st = 0;
       uint32_t ph = 1;
-      bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
-        const int rt = tile / p.tok_tiles;  // token tiles of one row tile are neighbours: weights stay in L2
-        for (int g = 0; g < G; g += 2) {
-          const int ng = (G - g < 2) ? G - g : 2;
+      for (int tile = cluster; !dead && tile < p.tiles; tile += nclusters) {
+        const int rt = min(2 * tile_of(p, tile).pair + half, p.row_tiles - 1);
+        const uint8_t* src = p.stream + (static_cast<size_t>(rt) * p.G + g0) * kTileGroupBytes;
+        for (int g = g0; g < g1; ++g, src += kTileGroupBytes) {
           if (!mbar_wait_bounded_relaxed(wempty_a + st * 8, ph, kPSpin)) {
             atomicExch(p.status, W4A16_ETIMEOUT);
-            ok = false;
+            dead = true;
             break;
           }
-          mbar_expect_tx(wfull_a + st * 8, ng * kTileGroupBytes);
-          bulk_g2s(ring_a + st * kPStage, p.stream + (static_cast<size_t>(rt) * G + g) * kTileGroupBytes,
-                   ng * kTileGroupBytes, wfull_a + st * 8);
-          if (++st == kPD) {
+          mbar_expect_tx(wfull_a + st * 8, kTileGroupBytes);
+          bulk_g2s(ring_a + st * kTileGroupBytes, src, kTileGroupBytes, wfull_a + st * 8);
+          if (++st == WD) {
             st = 0;
             ph ^= 1;
           }
         }
       }
+      if (dead) {  // the copies in flight still have to land
+        for (int i = 0; i < WD; ++i) mbar_wait_bounded_relaxed(wfull_a + i * 8, i < st ? ph ^ 1u : ph, 1u << 10);
+      }
     }
-    return;
-  }
-
-  // ================================================================ MMA issuer
-  if (warp == PW + 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(kTileRows, TN);
-      int b = 0, xb = 0;
-      uint32_t bph = 0, xph = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
-        for (int g = 0; g < G; ++g) {
-          if (!mbar_wait_bounded(xfull_a + xb * 8, xph, kPSpin) ||
-              !mbar_wait_bounded(afull_a + b * 8, bph, kPSpin)) {
-            atomicExch(p.status, W4A16_ETIMEOUT);
-            ok = false;
+  } else if (warp == kWIssue) {
+    // ================================================================ MMA issuer (leader CTA only)
+    // The whole warp walks (so that the operands stay in uniform registers), one elected lane issues.
+    if (half == 0) {
+      const uint16_t both = static_cast<uint16_t>(3u << rank);
+      const uint64_t desc0 = umma_desc_sw128(xbuf_a);
+      const uint32_t x16 = static_cast<uint32_t>(xbytes) >> 4;
+      uint32_t j = 0, aph = 0, dph = 1;
+      int a = 0;
+      for (int tile = cluster; !dead && tile < p.tiles; tile += nclusters, dph ^= 1) {
+        const uint32_t idesc = umma_idesc_bf16(kPRows, tile_of(p, tile).n);
+        if (!mbar_wait_bounded(dempty_a, dph, kPSpin)) dead = true;  // (passes on the first tile)
+        for (int g = g0; !dead && g < g1; ++g, ++j) {
+          const uint32_t st = j & (kPSteps - 1);
+          if (!mbar_wait_bounded(xfull_a + st * 8, (j / kPSteps) & 1u, kPSpin) ||
+              !mbar_wait_bounded(afull_a + a * 8, aph, kPSpin)) {
+            dead = true;
             break;
           }
           tc_fence_after();
-          // B operand of the group: two swizzled tiles of 64 k x 256 tokens (32 KB each); a 16-k slab
-          // is 32 bytes further along the 128-byte rows
-          const uint32_t a_t = tmem + kPTmemA + b * 64;
+          // B operand of the group: two swizzled tiles of 128-byte rows, one per token; a 16-k slab is 32 bytes
+          // further along them
+          const uint64_t b0 = desc0 + st * x16, b1 = b0 + (x16 >> 1);
+          const uint32_t at = tmem_a + a * 64;
+          if (elect_one()) {
 #pragma unroll
-          for (int s = 0; s < 8; ++s)
-            umma_bf16_ts(tmem + kPTmemD, a_t + s * 8,
-                         umma_desc_sw128(xbuf_a + xb * kPXBytes + (s >> 2) * (kPXBytes / 2) + (s & 3) * 32), idesc,
-                         (g | s) != 0);
-          umma_commit(mdone_a + b * 8);
-          umma_commit(xempty_a + xb * 8);
-          if (++b == kPNB) {
-            b = 0;
-            bph ^= 1;
+            for (int s = 0; s < 8; ++s)
+              umma_bf16_ts_pair(tmem, at + s * 8, (s < 4 ? b0 : b1) + 2 * (s & 3), idesc, s > 0 || g > g0);
+            umma_commit_pair(done_a + (j & (kPDone - 1)) * 8, both);
+            if (g == g1 - 1) umma_commit_pair(dfull_a, both);
           }
-          if (++xb == kPXBufs) {
-            xb = 0;
-            xph ^= 1;
+          __syncwarp();
+          if (++a == na) {
+            a = 0;
+            aph ^= 1;
           }
         }
-        umma_commit(ddone_a);  // accumulator complete once everything issued so far has finished
       }
+      if (dead && lane == 0) atomicExch(p.status, W4A16_ETIMEOUT);
     }
-    __syncwarp();
-    // tensor memory goes back only after every dequant warp has read its last accumulator columns
-    mbar_wait_bounded_relaxed(alldone_a, 0, kPSpin);
-    tc_fence_after();
-    tmem_dealloc(tmem, kPTmemCols);
-    return;
-  }
-
-  // ================================================================ activation producer
-  // One thread: two tiled TMA loads per k group (k halves of 64), rows past M are zero-filled.
-  if (warp == PW + 2) {
+  } else if (warp == kWActs) {
+    // ================================================================ activation producer
+    // Two tiled TMA loads per k group (64 k each) into this CTA's half of the token tile; rows past M are zero-filled. The
+    // leader's barrier expects both CTAs' bytes.
     if (lane == 0) {
-      int xb = 0;
-      uint32_t eph = 1;
-      bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
-        const int tok0 = (tile % p.tok_tiles) * TN;
-        for (int g = 0; g < G; ++g) {
-          if (!mbar_wait_bounded_relaxed(xempty_a + xb * 8, eph, kPSpin)) {
+      const uint32_t xfull_l = map_to_rank(xfull_a, leader);
+      uint32_t j = 0;
+      for (int tile = cluster; !dead && tile < p.tiles; tile += nclusters) {
+        const PTile t = tile_of(p, tile);
+        const int y = t.tok0 + half * (t.n >> 1);
+        for (int g = g0; g < g1; ++g, ++j) {
+          const uint32_t st = j & (kPSteps - 1);
+          const uint32_t jd = j - kPSteps;
+          if (j >= kPSteps && !mbar_wait_bounded_relaxed(done_a + (jd & (kPDone - 1)) * 8, (jd / kPDone) & 1u, kPSpin)) {
             atomicExch(p.status, W4A16_ETIMEOUT);
-            ok = false;
+            dead = true;
             break;
           }
-          mbar_expect_tx(xfull_a + xb * 8, kPXBytes);
-          tma_load_2d(xbuf_a + xb * kPXBytes, &p.amap, g * kGroup, tok0, xfull_a + xb * 8);
-          tma_load_2d(xbuf_a + xb * kPXBytes + kPXBytes / 2, &p.amap, g * kGroup + 64, tok0, xfull_a + xb * 8);
-          if (++xb == kPXBufs) {
-            xb = 0;
-            eph ^= 1;
-          }
+          if (half == 0) mbar_expect_tx(xfull_a + st * 8, 2 * xbytes);
+          tma_load_pair(xbuf_a + st * xbytes, &p.amap, g * kGroup, y, xfull_l + st * 8);
+          tma_load_pair(xbuf_a + st * xbytes + (xbytes >> 1), &p.amap, g * kGroup + 64, y, xfull_l + st * 8);
         }
+      }
+      if (dead && half == 0) {
+        for (uint32_t i = j < kPSteps ? 0 : j - kPSteps; i < j; ++i)
+          mbar_wait_bounded_relaxed(xfull_a + (i & (kPSteps - 1)) * 8, (i / kPSteps) & 1u, 1u << 10);
       }
     }
-    return;
-  }
-
-  // ================================================================ dequant warps + epilogue
-  const int q = warp & 3, h = warp >> 2;
-  const int row = q * 32 + lane;
-  const uint32_t tlane = static_cast<uint32_t>(q * 32) << 16;
-  int wst = 0, b = 0;
-  uint32_t wph = 0, eph = 1, dph = 0;  // eph: "A columns free" reads as true on the first lap
-  bool dead = false;
-
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int rt = tile / p.tok_tiles, tt = tile % p.tok_tiles;
-    for (int g = 0; g < G; ++g) {
-      if ((g & 1) == 0) {
-        if (!dead && !mbar_wait_bounded(wfull_a + wst * 8, wph, kPSpin)) {
-          dead = true;
-          atomicExch(p.status, W4A16_ETIMEOUT);
-        }
-      }
-      // the MMAs that read this A buffer three groups ago must have completed
-      if (!dead && !mbar_wait_bounded(mdone_a + b * 8, eph, kPSpin)) {
+  } else if (warp < PW) {
+    // ================================================================ dequant warps
+    // The walk over tiles does not matter here: the groups come in the order of the weight ring.
+    // Two teams of eight warps take alternate groups: one group's waits, shared-memory loads and tensor-memory stores
+    // run beside the other's arithmetic. (Ring depths are even, so a barrier's consecutive phases belong to one team;
+    // a parity wait could not tell them apart otherwise.)
+    const int q = warp & 3, odd = (warp >> 2) & 1, team = warp >> 3;  // odd: takes the second half (64 k) of its groups
+    const int row = q * 32 + lane;
+    const uint32_t a_t = tmem_a + (static_cast<uint32_t>(q * 32) << 16) + odd * 32;
+    const uint32_t afull_l = map_to_rank(afull_a, leader);
+    const int ntiles = cluster < p.tiles ? (p.tiles - 1 - cluster) / nclusters + 1 : 0;
+    const uint32_t ngroups = static_cast<uint32_t>(ntiles) * static_cast<uint32_t>(g1 - g0);
+    const uint32_t off0 = 2 * odd * kChunkBytes + weight_slot(row, 0) * 16, off1 = (2 * odd + 1) * kChunkBytes + weight_slot(row, 1) * 16;
+    int st = team, a = team;  // weight stage and A slot
+    uint32_t wph = 0;
+    for (uint32_t j = team; j < ngroups; j += 2) {
+      if (!mbar_wait_bounded(wfull_a + st * 8, wph, kPSpin)) {
         dead = true;
-        atomicExch(p.status, W4A16_ETIMEOUT);
+        break;
       }
-      const uint8_t* blk = ring + wst * kPStage + (g & 1) * kTileGroupBytes;
+      const uint8_t* blk = ring + st * kTileGroupBytes;
+      const uint4 w0 = *reinterpret_cast<const uint4*>(blk + off0), w1 = *reinterpret_cast<const uint4*>(blk + off1);
       const uint32_t zp = blk[kTgZpOff + row];
-      const uint32_t zpair = __byte_perm(zp, 0x43434343u, 0x4040);  // bf16 pair (128+zp, 128+zp)
       const uint32_t sc = reinterpret_cast<const uint16_t*>(blk + kTgScaleOff)[row];
+      const uint32_t zpair = __byte_perm(zp, 0x43434343u, 0x4040);  // bf16 pair (128+zp, 128+zp)
       const uint32_t spair = sc | (sc << 16);
+      const uint32_t w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+      uint32_t v[2][16];
 #pragma unroll
-      for (int jj = 0; jj < 2; ++jj) {
-        const int j = 2 * h + jj;
-        const uint4 wq = *reinterpret_cast<const uint4*>(blk + j * kChunkBytes + weight_slot(row, j) * 16);
-        const uint32_t w[4] = {wq.x, wq.y, wq.z, wq.w};
-        uint32_t a[16];
+      for (int c = 0; c < 2; ++c)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int pp = 0; pp < 4; ++pp)
-            a[4 * i + pp] =
-                mul_bf16x2(sub_bf16x2(((w[i] >> (4 * pp)) & kNibMaskP) | kMagicP, zpair), spair);
-        }
-        tmem_st16(tmem + tlane + kPTmemA + b * 64 + j * 16, a);
+            v[c][4 * i + pp] = mul_bf16x2(sub_bf16x2(((w[4 * c + i] >> (4 * pp)) & kNibMaskP) | kMagicP, zpair), spair);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(wempty_a + st * 8);
+      // only now the wait for the A slot: the MMAs that read it last, na groups ago, must have completed
+      const uint32_t jd = j - na;
+      if (j >= static_cast<uint32_t>(na) && !mbar_wait_bounded(done_a + (jd & (kPDone - 1)) * 8, (jd / kPDone) & 1u, kPSpin)) {
+        dead = true;
+        break;
       }
+      tc_fence_after();
+      tmem_st16(a_t + a * 64, v[0]);
+      tmem_st16(a_t + a * 64 + 16, v[1]);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(afull_a + b * 8);
-      if (++b == kPNB) {
-        b = 0;
-        eph ^= 1;
-      }
-      if ((g & 1) == 1 || g == G - 1) {
-        if (lane == 0) mbar_arrive(wempty_a + wst * 8);
-        if (++wst == kPD) {
-          wst = 0;
-          wph ^= 1;
-        }
+      if (lane == 0) mbar_arrive_cluster(afull_l + a * 8);
+      if ((a += 2) >= na) a -= na;
+      if ((st += 2) >= WD) {
+        st -= WD;
+        wph ^= 1;
       }
     }
-    // ---- epilogue: the k-half h of a row's warps writes tokens [128 h, 128 h + 128) ----
-    if (!dead && !mbar_wait_bounded(ddone_a, dph, kPSpin)) {
-      dead = true;
-      atomicExch(p.status, W4A16_ETIMEOUT);
-    }
-    dph ^= 1;
-    tc_fence_after();
-    const int r = rt * kTileRows + row;
-#pragma unroll 1
-    for (int cblk = 0; cblk < 8; ++cblk) {
-      float d[16];
-      const int col0 = h * 128 + cblk * 16;
-      tmem_ld<16>(tmem + tlane + kPTmemD + col0, d);
-      tmem_wait_ld();
-      if (r < p.N) {
+    if (dead) atomicExch(p.status, W4A16_ETIMEOUT);
+  } else if (S == 1) {
+    // ================================================================ epilogue warps
+    // The next tile's MMAs wait for the accumulator, so it is read out into shared memory (as bf16) and handed back;
+    // the stores to C, 256 bytes per token, run beside the next tile's main loop.
+    const int q = warp & 3, eh = (warp - kWEpi0) >> 2, et = tid - kWEpi0 * 32;
+    const uint32_t lane_t = tmem + (static_cast<uint32_t>(q * 32) << 16);
+    const uint32_t dempty_l = map_to_rank(dempty_a, leader);
+    uint32_t dph = 0;
+    for (int tile = cluster; tile < p.tiles; tile += nclusters, dph ^= 1) {
+      const PTile t = tile_of(p, tile);
+      if (!mbar_wait_bounded_relaxed(dfull_a, dph, kPSpin)) {
+        atomicExch(p.status, W4A16_ETIMEOUT);
+        break;
+      }
+      tc_fence_after();
+      uint16_t* cs = reinterpret_cast<uint16_t*>(cbuf);
+#pragma unroll 2
+      for (int c = eh * 16; c < t.n; c += EW / 4 * 16) {
+        float v[16];
+        tmem_ld<16>(lane_t + c, v);
+        tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const int tok = tt * TN + col0 + i;
-          if (tok < p.M) {
-            const size_t o = static_cast<size_t>(tok) * p.ldc + p.col0 + r;
-            const uint16_t hb = float_to_bf16_bits(d[i]);
-            p.C[o] = hb;
-            for (int pq = 0; pq < p.npeers; ++pq) p.C_peers[pq][o] = hb;  // fused all-gather over NVLink
+        for (int i = 0; i < 16; ++i) cs[(c + i) * kTileRows + q * 32 + lane] = float_to_bf16_bits(v[i]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(dempty_l);
+      named_bar_sync(1, EW * 32);
+      const int r0 = (2 * t.pair + half) * kTileRows;
+      const int rows = min(kTileRows, p.N - r0), toks = min(t.n, p.M - t.tok0);  // (rows <= 0: an odd last row tile's second half)
+      if (p.wide) {
+        const int rl = (et & 15) * 8;  // eight rows of one token per thread
+        if (rl < rows) {
+          for (int c = et >> 4; c < toks; c += EW * 2) {
+            const uint4 v = *reinterpret_cast<const uint4*>(cs + c * kTileRows + rl);
+            const size_t o = static_cast<size_t>(t.tok0 + c) * p.ldc + p.col0 + r0 + rl;
+            *reinterpret_cast<uint4*>(p.C + o) = v;
+            for (int pq = 0; pq < p.npeers; ++pq) *reinterpret_cast<uint4*>(p.C_peers[pq] + o) = v;  // fused all-gather over NVLink
+          }
+        }
+      } else {
+        for (int i = et; i < toks * kTileRows; i += EW * 32) {
+          const int rl = i & (kTileRows - 1);
+          if (rl < rows) {
+            const size_t o = static_cast<size_t>(t.tok0 + i / kTileRows) * p.ldc + p.col0 + r0 + rl;
+            p.C[o] = cs[i];
+            for (int pq = 0; pq < p.npeers; ++pq) p.C_peers[pq][o] = cs[i];
           }
         }
       }
+      named_bar_sync(1, EW * 32);  // the next tile overwrites the staged one
     }
-    // the next tile's first MMA overwrites the accumulator: all 8 warps must have read it
-    tc_fence_before();
-    named_bar_sync(2, PW * 32);
   }
 
+  if (S > 1) {
+    // ================================================================ split K: one tile per cluster
+    // Every split's fp32 tile goes to its own shared memory (the activation stages: all MMAs have read them, and
+    // [TN tokens][128 rows] floats are exactly their size), then split s adds up and stores the s-th share
+    // of the tokens, reading the others' tiles through the cluster.
+    const PTile t = tile_of(p, cluster);
+    if (warp >= kWEpi0 && warp < kWEpi0 + EW) {
+      const int q = warp & 3;
+      const uint32_t lane_t = tmem + (static_cast<uint32_t>(q * 32) << 16);
+      if (mbar_wait_bounded(dfull_a, 0, kPSpin)) {
+        tc_fence_after();
+        float* tile_s = reinterpret_cast<float*>(xbuf) + q * 32 + lane;
+#pragma unroll 1
+        for (int c = ((warp - kWEpi0) >> 2) * 16; c < t.n; c += EW / 4 * 16) {
+          float v[16];
+          tmem_ld<16>(lane_t + c, v);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) tile_s[(c + i) * kTileRows] = v[i];
+        }
+      } else {
+        atomicExch(p.status, W4A16_ETIMEOUT);
+      }
+    }
+    __syncwarp();
+    cluster_sync();
+    if (warp < PW + EW) {
+      const int q = warp & 3, row = q * 32 + lane;
+      const int r = (2 * t.pair + half) * kTileRows + row;
+      uint32_t src[kPMaxSplit];
+#pragma unroll
+      for (int s = 0; s < kPMaxSplit; ++s)
+        src[s] = map_to_rank(xbuf_a + row * 4, static_cast<uint32_t>(2 * min(s, S - 1) + half));
+      const int c1 = t.n * (split + 1) / S;
+#pragma unroll 4
+      for (int c = t.n * split / S + (warp >> 2); c < c1; c += (PW + EW) / 4) {
+        float part[kPMaxSplit];
+#pragma unroll
+        for (int s = 0; s < kPMaxSplit; ++s)
+          part[s] = s < S ? ld_cluster_f32(src[s] + c * (kTileRows * 4)) : 0.f;
+        float acc = part[0];
+#pragma unroll
+        for (int s = 1; s < kPMaxSplit; ++s)
+          if (s < S) acc += part[s];
+        const int tok = t.tok0 + c;
+        if (r < p.N && tok < p.M) {
+          const size_t o = static_cast<size_t>(tok) * p.ldc + p.col0 + r;
+          const uint16_t hb = float_to_bf16_bits(acc);
+          p.C[o] = hb;
+          for (int pq = 0; pq < p.npeers; ++pq) p.C_peers[pq][o] = hb;
+        }
+      }
+    }
+  }
+
+  // Nobody leaves while the other CTAs of the cluster may still reach its barriers, shared or tensor memory.
   tc_fence_before();
   __syncwarp();
-  if (lane == 0) mbar_arrive(alldone_a);
-  if (p.comm_local) {
-    // every store of this CTA comes from these eight warps: once they are all here, the CTA's share of the
-    // launch's completion signal goes to every rank
-    named_bar_sync(2, PW * 32);
-    if (tid == 0) signal_cta_done(p.comm_local, p.comm_peers, p.comm_n, p.comm_rank);
+  cluster_sync();
+  if (warp == kWIssue) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem, kPTmemCols);
   }
+  // every store of this CTA was issued before the barrier above: its share of the launch's completion signal
+  if (p.comm_local && tid == 0) signal_cta_done(p.comm_local, p.comm_peers, p.comm_n, p.comm_rank);
+}
+
+// ------------------------------------------------------------------ the plan of a launch
+struct PrefillPlan {
+  int tn = 0, splits = 1, full_tt = 0, tiles = 0, clusters = 0, wdepth = 0, smem = 0;
+};
+
+int prefill_smem(int tn, int wdepth) {
+  return 1024 + kPSteps * tn * 128 + tn * kTileRows * 2 + wdepth * kTileGroupBytes + kPBars * 8 + 16;
+}
+
+// Tokens per tile and K splits. A cluster's time for a tile is its k groups times the slower of the tensor cores
+// (4 TN cycles per group for a pair) and the expansion of the weights (kExpand cycles per group), plus
+// what is paid once per tile (pipeline fill, read-out of the accumulator, the exchange of split K). Tiles go to
+// the clusters in turn, dearest first, so cluster 0 has the longest list: its total is what is minimised.
+PrefillPlan plan_prefill(int M, int pairs, int G, const int* clusters_of_split, int smem_optin) {
+  constexpr int kExpand = 420, kFill = 2500, kReduce = 4000;
+  PrefillPlan best;
+  long long best_cost = -1;
+  for (int S = 1; S <= kPMaxSplit && S <= G; ++S) {
+    const int slots = clusters_of_split[S];
+    if (slots < 1) continue;
+    for (int tn = 32; tn <= kPMaxTN; tn += 32) {
+      const int full = M / tn, rest = M - full * tn;
+      if (full == 0 && tn - 32 >= rest) break;  // one token tile: the smallest that holds M
+      const long long nfull = static_cast<long long>(pairs) * full, tiles = nfull + (rest ? pairs : 0);
+      if (S > 1 && tiles > slots) continue;     // split clusters take one tile each
+      const int groups = (G + S - 1) / S;
+      auto cost = [&](int n) {
+        const long long loop = static_cast<long long>(groups) * (4 * n > kExpand ? 4 * n : kExpand);
+        return loop + (S > 1 ? kFill + kReduce : kFill / 2);
+      };
+      const long long cf = cost(tn), cr = cost((rest + 31) & ~31);
+      const long long wf = (nfull + slots - 1) / slots, wa = (tiles + slots - 1) / slots;
+      const long long total = wf * cf + (wa - wf) * cr;
+      if (best_cost < 0 || total < best_cost) {
+        best_cost = total;
+        best.tn = tn;
+        best.splits = S;
+        best.full_tt = full;
+        best.tiles = static_cast<int>(tiles);
+        best.clusters = static_cast<int>(tiles < slots ? tiles : slots);
+      }
+    }
+  }
+  best.wdepth = kPMaxWD;
+  while (best.wdepth > 2 && prefill_smem(best.tn, best.wdepth) > smem_optin) best.wdepth -= 2;
+  best.smem = prefill_smem(best.tn, best.wdepth);
+  return best;
 }
 
 }  // namespace
@@ -356,6 +570,46 @@ int w4a16_workspace_free(w4a16_workspace_t* ws) {
 }
 
 namespace {
+void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* at, int splits, int clusters, int smem) {
+  cfg.gridDim = dim3(2 * splits * clusters);
+  cfg.blockDim = dim3(kPWarps * 32);
+  cfg.dynamicSmemBytes = smem;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2 * splits;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+}
+
+// How many clusters of 2 S CTAs (one CTA per SM) the device runs at once, index S; asked for once per device.
+// The kernel's shared-memory attribute is set on the way. Returns nullptr (and sets the error) on failure.
+const int* cluster_slots(int dev, const DeviceInfo* di) {
+  struct Slots {
+    bool ready = false;
+    int n[kPMaxSplit + 1] = {};
+  };
+  static std::mutex mu;
+  static Slots all[64];
+  std::lock_guard<std::mutex> lk(mu);
+  Slots& s = all[dev & 63];
+  if (!s.ready) {
+    cudaError_t e = cudaFuncSetAttribute(k_prefill, cudaFuncAttributeMaxDynamicSharedMemorySize, di->smem_optin);
+    for (int S = 1; S <= kPMaxSplit && e == cudaSuccess; ++S) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute at[1];
+      cluster_config(cfg, at, S, 1, prefill_smem(kPMaxTN, 2));
+      e = cudaOccupancyMaxActiveClusters(&s.n[S], k_prefill, &cfg);
+    }
+    if (e != cudaSuccess || s.n[1] < 1) {
+      fail(W4A16_ECUDA, "gemm_prefill: the device runs no CTA pair of the kernel (%s)", cudaGetErrorString(e));
+      return nullptr;
+    }
+    s.ready = true;
+  }
+  return s.n;
+}
+
 int launch_prefill(PrefillParams& p, uint16_t* C, const w4a16_weights_t* w, const uint16_t* A, int M, w4a16_workspace_t* ws,
                    void* stream) {
   if (int rc = check_weights(w)) return rc;
@@ -365,16 +619,29 @@ int launch_prefill(PrefillParams& p, uint16_t* C, const w4a16_weights_t* w, cons
   W4_REQUIRE(ws != nullptr, "gemm_prefill: null workspace");
   const DeviceInfo* di = device_info();
   if (!di) return W4A16_ECUDA;
+  int dev = 0;
+  W4_CUDA(cudaGetDevice(&dev));
+  const int* slots = cluster_slots(dev, di);
+  if (!slots) return W4A16_ECUDA;
   p.stream = reinterpret_cast<const uint8_t*>(w->qweight);
-  p.A = A;
   p.C = C;
   p.M = M;
   p.N = w->out_f;
   p.K = w->in_f;
   p.G = w->num_groups;
   p.row_tiles = (w->out_f + kTileRows - 1) / kTileRows;
-  p.tok_tiles = (M + TN - 1) / TN;
+  p.pairs = (p.row_tiles + 1) / 2;
+  const PrefillPlan plan = plan_prefill(M, p.pairs, p.G, slots, di->smem_optin);
+  W4_REQUIRE(plan.tn > 0, "gemm_prefill: no launch shape for M = %d, %d x %d", M, w->out_f, w->in_f);
+  p.tn = plan.tn;
+  p.splits = plan.splits;
+  p.wdepth = plan.wdepth;
+  p.full_tt = plan.full_tt;
+  p.tiles = plan.tiles;
   p.status = di->status;
+  p.wide = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && p.ldc % 8 == 0 && p.col0 % 8 == 0;
+  for (int q = 0; q < p.npeers; ++q)
+    if (reinterpret_cast<uintptr_t>(p.C_peers[q]) & 15) p.wide = 0;
   {
     // driver entry point for the tensor-map encoder (no link-time dependency on libcuda)
     typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -390,24 +657,18 @@ int launch_prefill(PrefillParams& p, uint16_t* C, const w4a16_weights_t* w, cons
     }
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(w->in_f), static_cast<cuuint64_t>(M)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(w->in_f) * 2};
-    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(TN)};
+    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(plan.tn / 2)};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult cr = encode(&p.amap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t*>(A), dims, strides,
                                box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) return fail(W4A16_ECUDA, "gemm_prefill: cuTensorMapEncodeTiled failed (%d)", int(cr));
   }
-  static bool attr_set[64] = {};
-  int dev = 0;
-  W4_CUDA(cudaGetDevice(&dev));
-  if (!attr_set[dev & 63]) {
-    W4_CUDA(cudaFuncSetAttribute(k_prefill, cudaFuncAttributeMaxDynamicSharedMemorySize, kPSmem));
-    attr_set[dev & 63] = true;
-  }
-  const long long ntiles = static_cast<long long>(p.row_tiles) * p.tok_tiles;
-  const int grid = static_cast<int>(ntiles < di->sms ? ntiles : di->sms);
-  k_prefill<<<grid, kPWarps * 32, kPSmem, static_cast<cudaStream_t>(stream)>>>(p);
-  W4_CUDA(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  cluster_config(cfg, at, plan.splits, plan.clusters, plan.smem);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  W4_CUDA(cudaLaunchKernelEx(&cfg, k_prefill, p));
   return W4A16_OK;
 }
 }  // namespace
