@@ -81,12 +81,6 @@ struct PrefillParams {
   int comm_n, comm_rank;
 };
 
-__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
-  uint32_t d;
-  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  return d;
-}
-
 // ---- CTA pairs and clusters --------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
@@ -105,11 +99,6 @@ __device__ __forceinline__ void cluster_sync() {
 // the tcgen05 fences around it, so the barrier needs no cluster-scope release (which costs a memory fence).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool elect_one() {
-  uint32_t pred;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
-  return pred != 0;
 }
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
   float v;

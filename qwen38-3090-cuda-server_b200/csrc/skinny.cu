@@ -253,13 +253,6 @@ __device__ __forceinline__ uint32_t step_word(int slot0, int slot1, int ng, bool
 }
 
 // ---- PTX used only here ------------------------------------------------------------------
-// One lane of the (converged) warp; unlike a test of the lane index this keeps the code around it
-// warp-uniform for the compiler, so tensor-core operands stay in uniform registers.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t pred;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
-  return pred != 0;
-}
 // Bounded wait with a per-launch suspend hint: how long one try_wait may park the thread.
 __device__ __forceinline__ bool wait_h(uint32_t bar, uint32_t parity, uint32_t hint_ns, uint32_t limit) {
   for (uint32_t i = 0; i < limit; ++i)
