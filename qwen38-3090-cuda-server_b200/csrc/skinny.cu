@@ -7,7 +7,7 @@
 // for lm_head, the separate argmax kernels (src/kernels/elementwise.cu:96-194).
 //
 // Shape of the computation (HBM-bound: every weight byte is read exactly once):
-//   * persistent grid, one CTA per SM (24 warps, all 512 tensor-memory columns, about 160 KB of shared
+//   * persistent grid, one CTA per SM (24 or 28 warps, all 512 tensor-memory columns, about 160 KB of shared
 //     memory). The (128-row tile, k group) units of the matrix are dealt out as equal contiguous
 //     ranges, so every CTA streams the same number of bytes whatever N and K are. A row tile whose K
 //     range is shared by several CTAs is finished by the CTA that owns its first units: the others
@@ -44,7 +44,7 @@
 //     (k_digits) into the scratch and every CTA streams the rows of the groups it multiplies through
 //     a second ring of bulk copies (they come from L2), instead of 148 identical conversions of M
 //     tokens and a cache of M x K digit bytes per CTA. 3 M <= 48 rows of B: one launch for every
-//     M <= 16. The converter warps become more fix-up warps (up to three token sets).
+//     M <= 16. The converter warps become more fix-up warps (up to four token sets).
 #include <cfloat>
 #include <climits>
 #include <cstdlib>
@@ -58,8 +58,6 @@ namespace w4a16 {
 namespace {
 
 constexpr int CW = 4;                      // fix-up warps per CTA: 32 rows of the 128-row tile each
-constexpr int kWarps = 24;
-constexpr int kThreads = kWarps * 32;
 constexpr int kWUnpack0 = 4;               // warps 4..11 unpack
 constexpr int kWProducer = 12;
 constexpr int kWMma = 13;                  // MMA issuer of the even steps; owns the tensor-memory allocation
@@ -86,7 +84,11 @@ constexpr int kAColsG = 32;                // 128 int8 along k = 32 columns of 3
 
 
 // Per token-count geometry. N = rows of the B operand the tensor core reads (3 digit rows per token are
-// real). Ring depths are in steps: AD2 for A, DD2 for D and for the ring of "step done" barriers.
+// real). Ring depths are in steps: AD2 for A, DD2 for D.
+// With N = 48 the D ring is two steps deep: a fix-up warp hands a slot back as soon as its sums are in registers, a few
+// hundred cycles after they appear, while an A slot is away for the whole way from unpack to "step done". Against
+// four D and two A steps, 248320 x 5120: M = 9 147 -> 141 us, M = 12 163 -> 158, M = 16 195 -> 194. Sets of five tokens
+// hold a D slot longer and keep the four: M = 15 181 -> 176 us.
 template <int MT, bool ST>
 struct Geo {
   static constexpr bool kStream = ST;  // digit rows streamed from the pre-pass output instead of converted here
@@ -95,13 +97,32 @@ struct Geo {
   // accumulator columns [CB F, CB F + 3 TM), so every set runs the SAME code on its own aligned column block
   // (one copy of the fix-up code per kernel: the instruction footprint of all roles has to stay cache resident).
   //   MT:        1    2    4    6    8    9   12   15   16
-  //   FW x TM: 1x1  2x1  2x2  2x3  2x4  3x3  3x4  3x5  2x8
-  static constexpr int FW = MT <= 1 ? 1 : ((MT == 9 || MT == 12 || MT == 15) ? 3 : 2);
+  //   FW x TM: 1x1  2x1  2x2  2x3  2x4  3x3  4x3  3x5  4x4
+  // A set is a chain of waits, tensor-memory loads and dependent arithmetic per step, so more and smaller sets go
+  // faster until their fixed cost (about 60 instructions per warp and step) takes the issue slots: 248320 x 5120 in us,
+  //   M = 4: 2x2 109, 4x1 125;  M = 8: 2x4 135, 4x2 139;  M = 12: 3x4 161, 4x3 158;  M = 16: 2x8 275, 4x4 194
+  // and 34816 x 5120 before (scalar arithmetic; 3x4 at M = 12, 2x8 at M = 16) and now:
+  //   M = 4 21.6 -> 20.0, M = 6 22.4 -> 21.9, M = 8 26.8 -> 24.2, M = 9 27.1 -> 25.0, M = 12 29.4 -> 28.3, M = 16 36.9 -> 32.4
+  static constexpr int FW = MT <= 1 ? 1 : (MT <= 8 ? 2 : (MT == 9 || MT == 15 ? 3 : 4));
   static constexpr int TM = (MT + FW - 1) / FW;                // tokens per fix-up warp
-  static constexpr int CB = !ST ? 16 : (3 * TM <= 8 ? 8 : (3 * TM <= 16 ? 16 : 24));  // accumulator columns per set
+  static constexpr int CB = !ST ? 16 : (MT <= 2 ? 8 : (3 * TM + 3) / 4 * 4);  // accumulator columns per set
+  static constexpr int TP = TM == 1 ? 1 : (TM + 1) / 2 * 2;    // a set's entries per group in the (sum, 2^-p) table: TP sums, TP scales
+  static constexpr int kPairBytes = FW * TP * 8;               // the table's bytes per group
+  static constexpr int kWarps = FW <= 3 ? 24 : 28;
+  static constexpr int kThreads = kWarps * 32;
+  // The block size the compiler plans for sets the register limit: 80 (24 warps), 72 (28 warps) or, asked for with 1024
+  // threads, 64. The pre-pass's CTAs of the NEXT call want to sit beside this kernel's (4096 registers each): 24 warps
+  // of 80 leave room for one, 28 of 72 for none. Fewer registers pay where the code fits them; 34816, 17408 and 6144
+  // columns in us, default -> 64:
+  //   M = 8  24.3 / 17.2 / 10.5 -> 24.2 / 15.7 / 9.6      M = 16 33.3 / 22.3 / 13.6 -> 32.4 / 21.9 / 12.6
+  //   M = 6  21.9 / 15.1 / 8.6  -> 23.0 / 14.7 / 8.8      M = 9  25.2 / 17.1 / 9.3  -> 26.4 / 16.8 / 9.8
+  //   M = 12 28.5 / 19.1 / 11.8 -> 29.8 / 19.7 / 10.7     M = 15 30.5 / 20.2 / 12.1 -> 31.7 / 20.3 / 12.4
+  static constexpr int kBoundThreads = MT == 8 || MT == 16 ? 1024 : kThreads;
   static constexpr int N = !ST ? 16 : ((FW * CB + 15) / 16) * 16;  // rows of the B operand the tensor core reads
-  static constexpr int AD2 = N == 48 ? 2 : 4;
-  static constexpr int DD2 = N == 16 ? 8 : 4;
+  static constexpr bool kFiveTokens = N == 48 && CB == 16;         // (MT = 15)
+  static constexpr int AD2 = kFiveTokens ? 2 : 4;
+  static constexpr int DD2 = N == 16 ? 8 : (N == 32 || kFiveTokens ? 4 : 2);
+  static constexpr int ND = 8;                           // ring of "step done" barriers
   static constexpr int kAColsS = kStepGroups * kAColsG;  // A columns per step
   static constexpr int kDColsS = kStepGroups * N;        // D columns per step
   static constexpr int kDCol0 = AD2 * kAColsS;           // first D column
@@ -111,9 +132,11 @@ struct Geo {
   // shallow one (4 steps) the wait is on the critical loop and belongs to the issuer, so that the operand is
   // already unpacked when the slot comes free.
   static constexpr bool kIssuerWaitsD = DD2 < 8;
+  // A round of the fix-up warps is one step, except at M = 1, where two steps' loads are in flight together.
+  static constexpr bool kPairRounds = MT == 1;
   static_assert(3 * TM <= CB && FW * CB <= N, "token sets must fit their column blocks");
   static_assert(kDCol0 + DD2 * kDColsS <= kTmemCols, "tensor memory budget");
-  static_assert(AD2 <= DD2 && 2 <= DD2 / 2, "ring depths");
+  static_assert(AD2 <= ND && DD2 <= ND && DD2 % 2 == 0, "ring depths");  // even: a slot belongs to one issuer
   static_assert(AD2 + DD2 <= kSideSteps, "a (scale, zp) slot must have been read before the unpack warps reuse it");
 };
 
@@ -127,7 +150,7 @@ struct SkinnyParams {
   int M, N, K, G, tiles;
   int b_bytes;       // bytes of the B region (M = 1: digit rows of the groups this CTA multiplies; else the digit ring)
   int xs_bytes;      // bytes of the (sum, 2^-p) region (M = 1)
-  const uint8_t* dig;  // pre-pass output: G blocks of db_bytes = [8 chunks of 16 k][3 M digit rows] 16 B, then G x M (sum, 2^-p) pairs
+  const uint8_t* dig;  // pre-pass output: G blocks of db_bytes = [8 chunks of 16 k][N digit rows] 16 B, then per group and token set TP sums of X and TP scales 2^-p
   int db_bytes;
   int bdepth;        // M >= 2: steps in the digit ring (a power of two)
   int bshift;        //         and its log2
@@ -285,26 +308,40 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* d) {
                : "r"(taddr)
                : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* d) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]),
-        "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
-      : "r"(taddr)
-      : "memory");
-}
-// Columns [C0, C0 + CNT) of this thread's lane, relative to `base` (a multiple of CNT's block size; C0 and CNT
-// multiples of 8), as loads of 16 or 8 columns whose start is a multiple of their width; the caller awaits
-// them all at once.
-template <int C0, int CNT>
+// CNT columns of this thread's lane from `base` on (both multiples of 4), as loads whose start is a multiple of their
+// width: base is a multiple of 8 when CNT is, else of 4. The caller awaits them all at once.
+template <int CNT>
 __device__ __forceinline__ void tmem_ld_span(uint32_t base, uint32_t* d) {
   if constexpr (CNT > 0) {
-    // (a 24-column block starts at a multiple of 8 only: three loads of 8)
-    constexpr int W = (C0 % 16 == 0 && CNT == 16) ? 16 : 8;
-    if constexpr (W == 16) tmem_ld16(base + C0, d);
-    else tmem_ld8(base + C0, d);
-    tmem_ld_span<C0 + W, CNT - W>(base, d + W);
+    constexpr int W = CNT % 8 == 0 ? 8 : 4;
+    if constexpr (W == 8) tmem_ld8(base, d);
+    else tmem_ld4(base, d);
+    tmem_ld_span<CNT - W>(base + W, d + W);
   }
+}
+// Two fp32 operations per instruction (each lane of the pair rounds as the scalar instruction does).
+__device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ void unpack_f32x2(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long add_f32x2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long mul_f32x2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
 }
 __device__ __forceinline__ unsigned long long tagged(float v) {
   return (static_cast<unsigned long long>(kPieceTag) << 32) | __float_as_uint(v);
@@ -314,9 +351,13 @@ __device__ __forceinline__ unsigned long long tagged(float v) {
 __device__ __forceinline__ uint32_t fdiv(uint32_t u, unsigned long long m) {
   return static_cast<uint32_t>((static_cast<unsigned long long>(u) * m) >> 40);
 }
-// exact int -> float for |v| < 2^22 without the conversion pipe
+// exact int -> float for |v| < 2^22 without the conversion pipe: the magic constant's low mantissa bits take the integer
+constexpr float kMagicFloat = 12582912.0f;  // 0x4B400000
+__device__ __forceinline__ unsigned long long magic_pair(uint32_t lo, uint32_t hi) {
+  return pack_f32x2(__uint_as_float(0x4B400000u + lo), __uint_as_float(0x4B400000u + hi));
+}
 __device__ __forceinline__ float small_int_to_float(uint32_t v) {
-  return __uint_as_float(0x4B400000u + v) - 12582912.0f;
+  return __uint_as_float(0x4B400000u + v) - kMagicFloat;
 }
 
 // dynamic shared memory:
@@ -337,7 +378,7 @@ constexpr int kMailStride = 40;                    // words per mailbox entry (3
 constexpr int kMailWords = 2 * CW * kMailStride;
 template <int MT, bool ST>
 __host__ __device__ constexpr int bar_count(int depth, int bdepth) {
-  return 2 * depth + Geo<MT, ST>::AD2 + 2 * Geo<MT, ST>::DD2 + 2 + (ST ? 2 * bdepth : 0) + 1 + (tile_end_helper<MT, ST>() ? 2 * CW : 0);
+  return 2 * depth + Geo<MT, ST>::AD2 + Geo<MT, ST>::ND + Geo<MT, ST>::DD2 + 2 + (ST ? 2 * bdepth : 0) + 1 + (tile_end_helper<MT, ST>() ? 2 * CW : 0);
 }
 template <int MT, bool ST>
 __host__ __device__ inline int total_smem(int depth, int stage_bytes, int b_bytes, int xs_bytes, int bdepth) {
@@ -347,14 +388,14 @@ __host__ __device__ inline int total_smem(int depth, int stage_bytes, int b_byte
 
 // One token's 128 values of one k group (this lane: k = 4 lane .. 4 lane + 3, `rv`) -> three int8 digit
 // rows of the B operand at `bslot` (rows row0, row0 + 1, row0 + 2 of every 16-k chunk, chunks `lbo` bytes apart)
-// and (sum of X, 2^-p) at `xs`.
+// and the sum of X at xs[0], 2^-p at xs[xs_step].
 //   X = rint(x * 2^p), p chosen per group so that the largest |X| lies in [2^21, 2^22).
 //   The fp32 magic constant 1.5 * 2^23 makes the FMA deliver X in the low mantissa bits; adding 0x808080
 //   turns the balanced base-256 digits (d0, d1 in [-128,127], |d2| <= 64) into plain bytes, the XOR
 //   with 0x808080 turns those bytes back into signed digits: X = d0 + 2^8 d1 + 2^16 d2.
 // K index j of the operand holds k = 8 (j/8) + perm(j%8) with perm = {0,4,1,5,2,6,3,7}: the order in which
 // the two nibble masks deliver a packed word's weights.
-__device__ __forceinline__ void convert_group(uint2 rv, uint8_t* bslot, int lbo, int row0, float2* xs, int lane) {
+__device__ __forceinline__ void convert_group(uint2 rv, uint8_t* bslot, int lbo, int row0, float* xs, int xs_step, int lane) {
   const uint32_t mx = __vmaxu2(rv.x & 0x7FFF7FFFu, rv.y & 0x7FFF7FFFu);
   const uint32_t am = max(mx & 0xFFFFu, mx >> 16);               // bf16 bits of the lane's largest magnitude
   const uint32_t e = __reduce_max_sync(0xffffffffu, am) >> 7;    // its biased exponent, group-wide
@@ -383,17 +424,20 @@ __device__ __forceinline__ void convert_group(uint2 rv, uint8_t* bslot, int lbo,
   *reinterpret_cast<uint32_t*>(dst) = __byte_perm(P0, Q0, sel);
   *reinterpret_cast<uint32_t*>(dst + 16) = __byte_perm(P1, Q1, sel);
   *reinterpret_cast<uint32_t*>(dst + 32) = __byte_perm(P2, Q2, sel);
-  if (lane == 0) *xs = make_float2(static_cast<float>(tot), inv);
+  if (lane == 0) {
+    xs[0] = static_cast<float>(tot);
+    xs[xs_step] = inv;
+  }
 }
 
 // COMM: the cross-rank flag code (wait before x is read, signal after the last store, the pair exchange of the
 // vocab-sharded head) is compiled into separate instances, so that single-GPU launches run exactly the code
 // they ran without it.
 template <int MT, int WB, bool ST, bool COMM>
-__global__ void __launch_bounds__(kThreads, 1) k_skinny(const SkinnyParams p) {
+__global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const SkinnyParams p) {
   using GE = Geo<MT, ST>;
   constexpr int kBlock = Fmt<WB>::kBlock, kStageBytes = Fmt<WB>::kStage;
-  constexpr int N = GE::N, AD2 = GE::AD2, DD2 = GE::DD2;
+  constexpr int N = GE::N, AD2 = GE::AD2, DD2 = GE::DD2, ND = GE::ND;
   constexpr bool kStream = GE::kStream;
   constexpr int SLOT = kTileRows * MT;  // floats per partial tile
   extern __shared__ __align__(128) uint8_t smem[];
@@ -444,9 +488,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_skinny(const SkinnyParams p) {
   const uint32_t wfull_a = smem_u32(bars);          // [DS]  weights of a step landed (tx bytes)
   const uint32_t wempty_a = wfull_a + DS * 8;       // [DS]  stage free again (4 unpack warps)
   const uint32_t afull_a = wempty_a + DS * 8;       // [AD2] A slot written (4 unpack warps)
-  const uint32_t done_a = afull_a + AD2 * 8;        // [DD2] step t's MMAs have completed (tcgen05.commit): its sums are
+  const uint32_t done_a = afull_a + AD2 * 8;        // [ND]  step t's MMAs have completed (tcgen05.commit): its sums are
                                                     //       in D slot t % DD2, its A slot t % AD2 is free again
-  const uint32_t dempty_a = done_a + DD2 * 8;       // [DD2] D slot read out (4 fix-up warps)
+  const uint32_t dempty_a = done_a + ND * 8;        // [DD2] D slot read out (4 fix-up warps)
   const uint32_t bready_a = dempty_a + DD2 * 8;     // every needed group's digit rows are written
   const uint32_t tmemrdy_a = bready_a + 8;          // tensor memory allocated, base address published
   const uint32_t bfull_a = tmemrdy_a + 8;           // [BD]  M >= 2: digit rows of a step landed (tx bytes)
@@ -458,12 +502,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_skinny(const SkinnyParams p) {
   {
     // barrier i of the block [wfull | wempty | afull | done | dempty | bready | tmemrdy]: arrival counts
     // (+ [bfull | bempty] for M >= 2)
-    const int nb = bar_count<MT, ST>(DS, BD), nb0 = 2 * DS + AD2 + 2 * DD2 + 2;
+    const int nb = bar_count<MT, ST>(DS, BD), nb0 = 2 * DS + AD2 + ND + DD2 + 2;
     const uint32_t nfix = CW * ((M + GE::TM - 1) / GE::TM);                // active fix-up warps
     if (tid < nb) {
       uint32_t cnt = 1;                                                    // wfull, done, tmemrdy, bfull
       if (tid >= DS && tid < 2 * DS + AD2) cnt = 4;                        // wempty, afull: 4 unpack warps
-      else if (tid >= 2 * DS + AD2 + DD2 && tid < 2 * DS + AD2 + 2 * DD2) cnt = nfix;  // dempty
+      else if (tid >= 2 * DS + AD2 + ND && tid < 2 * DS + AD2 + ND + DD2) cnt = nfix;  // dempty
       else if (tid == nb0 - 2) cnt = kStream ? 1 : kTeam;                  // bready
       mbar_init(wfull_a + tid * 8, cnt);
     }
@@ -524,7 +568,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_skinny(const SkinnyParams p) {
         const int i = i0 + j * kTeam;
         if (i < total) {
           const int gj = i, m = 0;
-          convert_group(rv[j], bq + gj * b_slot, b_lbo, m, reinterpret_cast<float2*>(xsinv) + gj * MT + m, lane);
+          convert_group(rv[j], bq + gj * b_slot, b_lbo, m, reinterpret_cast<float*>(xsinv) + 2 * (gj * MT + m), 1, lane);
           // publish the item: B was written through the generic proxy, the tensor core reads it through the
           // async one; the slot counts as ready once all M tokens are in. Slots are numbered in the order the
           // CTA walks its groups, and items are taken in slot order, so the first steps can start after the
@@ -655,7 +699,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_skinny(const SkinnyParams p) {
           umma_s8_ts(d_t + N, a_t + kAColsG + 8, db1 + step16, idesc, 1);
           umma_s8_ts(d_t + N, a_t + kAColsG + 16, db1 + 2 * step16, idesc, 1);
           umma_s8_ts(d_t + N, a_t + kAColsG + 24, db1 + 3 * step16, idesc, 1);
-          umma_commit(done_a + d * 8);
+          umma_commit(done_a + (t & (ND - 1)) * 8);
         }
         __syncwarp();
       }
@@ -697,7 +741,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_skinny(const SkinnyParams p) {
       load_row(base);
       // the A slot's previous step has been multiplied (whether the D slot is free is the issuer's concern: the
       // operand can be unpacked while the fix-up warps are still reading the sums of DD2 steps ago)
-      if ((t >= AD2 && !wait_h(done_a + ((t - AD2) & (DD2 - 1)) * 8, static_cast<uint32_t>((t - AD2) / DD2) & 1u, p.hint,
+      if ((t >= AD2 && !wait_h(done_a + ((t - AD2) & (ND - 1)) * 8, static_cast<uint32_t>((t - AD2) / ND) & 1u, p.hint,
                                kSpinLimit)) ||
           (!GE::kIssuerWaitsD && t >= DD2 &&
            !wait_h(dempty_a + (t & (DD2 - 1)) * 8, static_cast<uint32_t>(t / DD2 - 1) & 1u, p.hint, kSpinLimit))) {
@@ -754,7 +798,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_skinny(const SkinnyParams p) {
   } else if (warp == 14) {
     // ================================================================ digit-row producer (M >= 2)
     // One thread walks the same unit range as the weight producer and brings each step's digit rows (and the
-    // tokens' (sum, 2^-p) pairs behind them) from the pre-pass output into the digit ring: one bulk copy per
+    // tokens' sums and scales behind them) from the pre-pass output into the digit ring: one bulk copy per
     // step, two consecutive groups. The pre-pass is the previous kernel in the stream, so this thread - and
     // only this one - waits for it; the weights are already streaming meanwhile.
     if constexpr (kStream) {
@@ -766,7 +810,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_skinny(const SkinnyParams p) {
         int t = 0;
         bool ok = true;
         const uint32_t db = static_cast<uint32_t>(p.db_bytes);
-        // all (sum, 2^-p) pairs of the call, once: G x M x 8 bytes, read by the fix-up warps to the end
+        // the sums and scales of the whole call, once, read by the fix-up warps to the end
         mbar_expect_tx(bready_a, static_cast<uint32_t>(p.xs_bytes));
         bulk_g2s(xsinv_a, p.dig + static_cast<size_t>(G) * db, static_cast<uint32_t>(p.xs_bytes), bready_a);
         while (ok && it.next(sg)) {
@@ -873,7 +917,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_skinny(const SkinnyParams p) {
     // 3 i .. 3 i + 2 of it
     constexpr int NLD = kStream ? CB : 4;
     const uint32_t* side_r = reinterpret_cast<const uint32_t*>(side) + r;
-    const float2* xs_tab = reinterpret_cast<const float2*>(xsinv);  // (sum, 2^-p): per cache slot (M = 1), else [k group][token]
+    const float2* xs_tab = reinterpret_cast<const float2*>(xsinv);  // M = 1: (sum, 2^-p) per cache slot or (pre-pass) per k group
     if constexpr (kStream) {
       // the pair table of the call arrives once, by bulk copy
       if (!wait_h(bready_a, 0, p.hint, kSpinLimit)) {
@@ -896,16 +940,16 @@ __global__ void __launch_bounds__(kThreads, 1) k_skinny(const SkinnyParams p) {
         seg_tile = reinterpret_cast<const int*>(mslot)[32];
         ++nmail;
       } else {
-      // A round is one or two steps (two unless the first ends its segment): one wait per issuer (a commit
+      // A round is one or (M = 1) two steps (two unless the first ends its segment): one wait per issuer (a commit
       // covers everything its thread issued before), GB groups' tensor-memory loads in flight together.
-      if (!wait_h(done_a + (t & (DD2 - 1)) * 8, static_cast<uint32_t>(t / DD2) & 1u, p.hint, kSpinLimit)) {
+      if (!wait_h(done_a + (t & (ND - 1)) * 8, static_cast<uint32_t>(t / ND) & 1u, p.hint, kSpinLimit)) {
         atomicExch(p.status, W4A16_ETIMEOUT);
         ok = false;
         break;
       }
       const uint2 e0 = table[t & (kTable - 1)];  // written before the step's weights were requested
-      const bool two = !((e0.x >> 17) & 1u) && t + 1 < T;
-      if (two && !wait_h(done_a + ((t + 1) & (DD2 - 1)) * 8, static_cast<uint32_t>((t + 1) / DD2) & 1u, p.hint, kSpinLimit)) {
+      const bool two = GE::kPairRounds && !((e0.x >> 17) & 1u) && t + 1 < T;
+      if (two && !wait_h(done_a + ((t + 1) & (ND - 1)) * 8, static_cast<uint32_t>((t + 1) / ND) & 1u, p.hint, kSpinLimit)) {
         atomicExch(p.status, W4A16_ETIMEOUT);
         ok = false;
         break;
@@ -970,68 +1014,57 @@ __global__ void __launch_bounds__(kThreads, 1) k_skinny(const SkinnyParams p) {
       }
       } else {
         // Per step: both groups' tensor-memory loads in flight together, one wait, and the step's D slot goes
-        // back at once (the issuer of step t + DD2 is waiting for it); then the two groups are added up. (With
-        // 24-column blocks the registers only allow one group at a time.)
-        constexpr int kInFlight = NLD <= 16 ? 2 : 1;
-        uint32_t dv[kInFlight][NLD];
+        // back at once (the issuer of step t + DD2 is waiting for it); then the two groups are added up.
+        uint32_t dv[2][NLD];
         auto add_group = [&](const uint32_t* d, uint32_t szv, int g) {
-          const float2* xs_g = xs_tab + g * M + m0;
+          // the set's sums, then its scales 2^-p
+          const float* xs_g = reinterpret_cast<const float*>(xsinv) + (g * GE::FW + F) * 2 * GE::TP;
           const float s = __uint_as_float(szv & 0xFFFF0000u);
           const float z = __uint_as_float(0x4B000000u | (szv & 0xFFu)) - 8388608.0f;
+          // No test for "token exists" here: the TM chains stay independent straight-line code. A set's
+          // tokens past M add up whatever their columns and the table's unused entries hold, and are
+          // never stored. Tokens go in pairs: packed fp32 instructions round like the scalar ones of the last odd
+          // token (and of the M = 1 kernel), so a row's value does not depend on the call's M.
+          const unsigned long long s2 = pack_f32x2(s, s), nz2 = pack_f32x2(-z, -z);
+          const unsigned long long off2 = pack_f32x2(-kMagicFloat, -kMagicFloat);
+          const unsigned long long k8 = pack_f32x2(256.f, 256.f), k16 = pack_f32x2(65536.f, 65536.f);
 #pragma unroll
-          for (int i = 0; i < TM; ++i) {
-            // No test for "token exists" here: the TM chains stay independent straight-line code. A set's
-            // tokens past M add up whatever their columns and the pair table's next entries hold, and are
-            // never stored.
-            const float2 xv = xs_g[i];  // (sum of X, 2^-p)
+          for (int i = 0; i + 1 < TM; i += 2) {
+            const unsigned long long sum2 = *reinterpret_cast<const unsigned long long*>(xs_g + i);
+            const unsigned long long inv2 = *reinterpret_cast<const unsigned long long*>(xs_g + GE::TP + i);
+            const unsigned long long d0 = add_f32x2(magic_pair(d[3 * i], d[3 * i + 3]), off2);
+            const unsigned long long d1 = add_f32x2(magic_pair(d[3 * i + 1], d[3 * i + 4]), off2);
+            const unsigned long long d2 = add_f32x2(magic_pair(d[3 * i + 2], d[3 * i + 5]), off2);
+            const unsigned long long dot = fma_f32x2(d2, k16, fma_f32x2(d1, k8, d0));
+            const unsigned long long acc = fma_f32x2(mul_f32x2(s2, inv2), fma_f32x2(nz2, sum2, dot), pack_f32x2(fin[i], fin[i + 1]));
+            unpack_f32x2(acc, fin[i], fin[i + 1]);
+          }
+          if constexpr (TM & 1) {
+            constexpr int i = TM - 1;
             const float d0 = small_int_to_float(d[3 * i]);
             const float d1 = small_int_to_float(d[3 * i + 1]);
             const float d2 = small_int_to_float(d[3 * i + 2]);
             const float dot = fmaf(d2, 65536.f, fmaf(d1, 256.f, d0));
-            fin[i] = fmaf(s * xv.y, fmaf(-z, xv.x, dot), fin[i]);
+            fin[i] = fmaf(s * xs_g[GE::TP + i], fmaf(-z, xs_g[i], dot), fin[i]);
           }
         };
-#pragma unroll
-        for (int sI = 0; sI < 2; ++sI) {
-          if (sI == 0 || two) {
-            const int ts = t + sI;
-            const uint32_t ew = sI ? e1.x : e0.x;
-            const int ng = static_cast<int>((ew >> 16) & 1u) + 1;
-            const uint32_t d_t = lane_t + (ts & (DD2 - 1)) * GE::kDColsS;
-            const int g0 = static_cast<int>((ew >> 19) & 0xFFu);  // the step's first k group: row of the pair table
-            const uint32_t* side_s = side_r + ((ts % kSideSteps) * kStepGroups) * kTileRows;
-            auto release = [&]() {
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(dempty_a + (ts & (DD2 - 1)) * 8);
-            };
-            if constexpr (kInFlight == 2) {
-              uint32_t sz[2];
-              tmem_ld_span<0, NLD>(d_t, dv[0]);
-              sz[0] = side_s[0];
-              if (ng == 2) {
-                tmem_ld_span<0, NLD>(d_t + N, dv[1]);
-                sz[1] = side_s[kTileRows];
-              }
-              tmem_wait_ld();
-              release();
-              add_group(dv[0], sz[0], g0);
-              if (ng == 2) add_group(dv[kInFlight - 1], sz[1], g0 + 1);
-            } else {
-              tmem_ld_span<0, NLD>(d_t, dv[0]);
-              const uint32_t sz0 = side_s[0], sz1 = side_s[kTileRows];
-              tmem_wait_ld();
-              if (ng == 1) release();
-              add_group(dv[0], sz0, g0);
-              if (ng == 2) {
-                tmem_ld_span<0, NLD>(d_t + N, dv[0]);
-                tmem_wait_ld();
-                release();
-                add_group(dv[0], sz1, g0 + 1);
-              }
-            }
-          }
+        const int ng = static_cast<int>((e0.x >> 16) & 1u) + 1;
+        const uint32_t d_t = lane_t + (t & (DD2 - 1)) * GE::kDColsS;
+        const int g0 = static_cast<int>((e0.x >> 19) & 0xFFu);  // the step's first k group: row of the table of sums and scales
+        const uint32_t* side_s = side_r + ((t % kSideSteps) * kStepGroups) * kTileRows;
+        uint32_t sz[2];
+        tmem_ld_span<NLD>(d_t, dv[0]);
+        sz[0] = side_s[0];
+        if (ng == 2) {
+          tmem_ld_span<NLD>(d_t + N, dv[1]);
+          sz[1] = side_s[kTileRows];
         }
+        tmem_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(dempty_a + (t & (DD2 - 1)) * 8);
+        add_group(dv[0], sz[0], g0);
+        if (ng == 2) add_group(dv[1], sz[1], g0 + 1);
       }
       const uint2 el = two ? e1 : e0;  // the round's last step
       t += two ? 2 : 1;
@@ -1249,7 +1282,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_skinny(const SkinnyParams p) {
 // (four warps, at most 32 registers) so that they fit beside a resident main-kernel CTA of the previous
 // layer and are ready to run the moment that layer completes.
 __global__ void __launch_bounds__(128, 16) k_digits(const uint16_t* __restrict__ x, uint8_t* __restrict__ dig, int M,
-                                                    int K, int G, int db_bytes, int tm, int cb,
+                                                    int K, int G, int db_bytes, int tm, int cb, int tp, int sets,
                                                     const unsigned* comm_local, int comm_n, int* status,
                                                     const uint16_t* __restrict__ ln_w, float ln_eps,
                                                     uint16_t* __restrict__ xn_out) {
@@ -1288,11 +1321,11 @@ __global__ void __launch_bounds__(128, 16) k_digits(const uint16_t* __restrict__
     rv.y = nrm(rv.y << 16, wq.y << 16) | (nrm(rv.y & 0xFFFF0000u, wq.y & 0xFFFF0000u) << 16);
     if (xn_out) reinterpret_cast<uint2*>(xn_out + static_cast<size_t>(m) * K + g * kGroup)[lane] = rv;
   }
-  float2* pairs = reinterpret_cast<float2*>(dig + static_cast<size_t>(G) * db_bytes);
+  float* pairs = reinterpret_cast<float*>(dig + static_cast<size_t>(G) * db_bytes);
   // token m belongs to set m / tm; its digit rows are rows cb (m / tm) + 3 (m % tm) .. + 2 of every 16-k chunk,
-  // a chunk being db_bytes / 8 bytes (N rows of 16 bytes)
-  const int f = m / tm;
-  convert_group(rv, dig + static_cast<size_t>(g) * db_bytes, db_bytes >> 3, cb * f + 3 * (m - f * tm), pairs + g * M + m, lane);
+  // a chunk being db_bytes / 8 bytes (N rows of 16 bytes); a group's table holds per set tp sums, then tp scales
+  const int f = m / tm, i = m - f * tm;
+  convert_group(rv, dig + static_cast<size_t>(g) * db_bytes, db_bytes >> 3, cb * f + 3 * i, pairs + (g * sets + f) * 2 * tp + i, tp, lane);
 }
 
 // Cross-rank reduction of a K-sharded layer: every rank's fp32 partial [M][N] sits in slot r of this rank's buffer
@@ -1402,7 +1435,7 @@ int launch_cfg(SkinnyParams& p, int grid, cudaStream_t st, int smem_optin) {
       p.bdepth = c[1];
       p.bshift = c[1] == 8 ? 3 : (c[1] == 4 ? 2 : 1);
       p.b_bytes = p.bdepth * kStepGroups * p.db_bytes;
-      p.xs_bytes = (p.G * p.M * 8 + 15) & ~15;
+      p.xs_bytes = (p.G * Geo<MT, ST>::kPairBytes + 15) & ~15;
       smem = total_smem<MT, ST>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, p.bdepth);
       if (smem <= limit) {
         found = true;
@@ -1445,7 +1478,7 @@ int launch_kernel(const SkinnyParams& p, int grid, cudaStream_t st, int smem) {
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(Geo<MT, ST>::kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
@@ -1469,29 +1502,31 @@ bool gemv_cache_fits(int groups, int stage_bytes, int smem_optin) {
 int instance_for(int M) {
   return M <= 2 ? M : (M <= 4 ? 4 : (M <= 6 ? 6 : (M <= 8 ? 8 : (M == 9 ? 9 : (M <= 12 ? 12 : (M <= 15 ? 15 : 16))))));
 }
+struct DigitGeometry {
+  int tm, cb, tp, sets, nrows;
+};
 template <int MT>
-void geometry_of(int& tm, int& cb, int& nrows) {
-  tm = Geo<MT, true>::TM;
-  cb = Geo<MT, true>::CB;
-  nrows = Geo<MT, true>::N;
+DigitGeometry geometry_of() {
+  using GE = Geo<MT, true>;
+  return {GE::TM, GE::CB, GE::TP, GE::FW, GE::N};
 }
-void set_geometry(int M, int& tm, int& cb, int& nrows) {
+DigitGeometry digit_geometry(int M) {
   switch (instance_for(M)) {
-    case 1: geometry_of<1>(tm, cb, nrows); break;
-    case 2: geometry_of<2>(tm, cb, nrows); break;
-    case 4: geometry_of<4>(tm, cb, nrows); break;
-    case 6: geometry_of<6>(tm, cb, nrows); break;
-    case 8: geometry_of<8>(tm, cb, nrows); break;
-    case 9: geometry_of<9>(tm, cb, nrows); break;
-    case 12: geometry_of<12>(tm, cb, nrows); break;
-    case 15: geometry_of<15>(tm, cb, nrows); break;
-    default: geometry_of<16>(tm, cb, nrows); break;
+    case 1: return geometry_of<1>();
+    case 2: return geometry_of<2>();
+    case 4: return geometry_of<4>();
+    case 6: return geometry_of<6>();
+    case 8: return geometry_of<8>();
+    case 9: return geometry_of<9>();
+    case 12: return geometry_of<12>();
+    case 15: return geometry_of<15>();
+    default: return geometry_of<16>();
   }
 }
 // pre-pass output: per k group the B operand's digit rows, [8 chunks of 16 k][at most 48 rows] 16 B; behind all
-// groups' rows the table of (sum, 2^-p) pairs, G x M x 8 bytes (+ 16 so that a bulk copy of the rounded-up size
-// stays inside)
-size_t prepass_bytes(int G, int M) { return static_cast<size_t>(G) * (128 * 48 + 8 * M) + 16; }
+// groups' rows the table of sums and scales, at most 16 tokens x 8 bytes per group (+ 16 so that a bulk copy of the
+// rounded-up size stays inside)
+size_t prepass_bytes(int G) { return static_cast<size_t>(G) * (128 * 48 + 8 * 16) + 16; }
 
 // A validated layer in either weight format, as the launcher sees it.
 struct LayerRef {
@@ -1514,14 +1549,14 @@ int launch_batch_c(SkinnyParams& q, int grid, cudaStream_t st, int smem_optin) {
   switch (instance_for(q.M)) {
     case 1: return q.dig ? launch_cfg<1, WB, true, COMM>(q, grid, st, smem_optin)
                          : launch_cfg<1, WB, false, COMM>(q, grid, st, smem_optin);
-    case 2: return launch_cfg<2, WB, true, COMM>(q, grid, st, smem_optin);    // token sets (1, 1)
-    case 4: return launch_cfg<4, WB, true, COMM>(q, grid, st, smem_optin);    // (2, M - 2)
-    case 6: return launch_cfg<6, WB, true, COMM>(q, grid, st, smem_optin);    // (3, M - 3)
-    case 8: return launch_cfg<8, WB, true, COMM>(q, grid, st, smem_optin);    // (4, M - 4)
-    case 9: return launch_cfg<9, WB, true, COMM>(q, grid, st, smem_optin);    // (3, 3, 3)
-    case 12: return launch_cfg<12, WB, true, COMM>(q, grid, st, smem_optin);  // (4, 4, M - 8)
-    case 15: return launch_cfg<15, WB, true, COMM>(q, grid, st, smem_optin);  // (5, 5, M - 10)
-    default: return launch_cfg<16, WB, true, COMM>(q, grid, st, smem_optin);  // (8, 8)
+    case 2: return launch_cfg<2, WB, true, COMM>(q, grid, st, smem_optin);    // token sets 1, 1
+    case 4: return launch_cfg<4, WB, true, COMM>(q, grid, st, smem_optin);    // 2, M - 2
+    case 6: return launch_cfg<6, WB, true, COMM>(q, grid, st, smem_optin);    // 3, M - 3
+    case 8: return launch_cfg<8, WB, true, COMM>(q, grid, st, smem_optin);    // 4, M - 4
+    case 9: return launch_cfg<9, WB, true, COMM>(q, grid, st, smem_optin);    // 3, 3, 3
+    case 12: return launch_cfg<12, WB, true, COMM>(q, grid, st, smem_optin);  // 3, 3, 3, M - 9
+    case 15: return launch_cfg<15, WB, true, COMM>(q, grid, st, smem_optin);  // 5, 5, M - 10
+    default: return launch_cfg<16, WB, true, COMM>(q, grid, st, smem_optin);  // 4, 4, 4, 4
   }
 }
 template <int WB>
@@ -1582,11 +1617,10 @@ int launch_skinny(SkinnyParams& p, const LayerRef* w, const uint16_t* x, int M, 
     // with this one as usual
     cfg.numAttrs = (config().pdl && !p.ordered) ? 1 : 0;
     p.ordered = 0;
-    int tm = 1, cb = 8, nrows = 16;
-    set_geometry(M, tm, cb, nrows);
-    p.db_bytes = 128 * nrows;
+    const DigitGeometry dg = digit_geometry(M);
+    p.db_bytes = 128 * dg.nrows;
     const unsigned* wait_block = p.comm_wait ? p.comm_local : nullptr;
-    W4_CUDA(cudaLaunchKernelEx(&cfg, k_digits, x, dig, M, p.K, p.G, p.db_bytes, tm, cb, wait_block, p.comm_n, p.status,
+    W4_CUDA(cudaLaunchKernelEx(&cfg, k_digits, x, dig, M, p.K, p.G, p.db_bytes, dg.tm, dg.cb, dg.tp, dg.sets, wait_block, p.comm_n, p.status,
                                p.ln_w, p.ln_eps, p.xn_out));
   }
   if (int rc = w->wbits == 4 ? launch_batch<4>(p, grid, st, di->smem_optin) : launch_batch<8>(p, grid, st, di->smem_optin))
@@ -1767,9 +1801,9 @@ int w4a16_scratch_alloc(w4a16_scratch_t* s, int max_in, int max_out, int min_gro
   // two partial tiles per CTA (head and tail of its unit range), widest tile, 16 tokens, 8-byte (sum, tag) words
   s->partial_elems = static_cast<size_t>(s->max_splits) * 2 * kTileRows * 16 * 2;
   const size_t counters = counter_bytes(max_out);
-  // per-CTA argmax pairs, then (max_m >= 2) the pre-pass output: digit rows of max_m tokens for every k group
+  // per-CTA argmax pairs, then (max_m >= 2) the pre-pass output: digit rows of up to 16 tokens for every k group
   const size_t pairs = pair_bytes(s->max_splits) +
-                       (max_m >= 2 ? prepass_bytes(s->max_groups, max_m > 16 ? 16 : max_m) : 0);
+                       (max_m >= 2 ? prepass_bytes(s->max_groups) : 0);
   void *xf = nullptr, *cn = nullptr, *pa = nullptr;
   cudaError_t e = cudaMalloc(&xf, pairs);
   if (e == cudaSuccess) e = cudaMalloc(&cn, counters);
