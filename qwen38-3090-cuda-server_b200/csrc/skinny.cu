@@ -85,10 +85,8 @@ constexpr int kAColsG = 32;                // 128 int8 along k = 32 columns of 3
 
 // Per token-count geometry. N = rows of the B operand the tensor core reads (3 digit rows per token are
 // real). Ring depths are in steps: AD2 for A, DD2 for D.
-// With N = 48 the D ring is two steps deep: a fix-up warp hands a slot back as soon as its sums are in registers, a few
-// hundred cycles after they appear, while an A slot is away for the whole way from unpack to "step done". Against
-// four D and two A steps, 248320 x 5120: M = 9 147 -> 141 us, M = 12 163 -> 158, M = 16 195 -> 194. Sets of five tokens
-// hold a D slot longer and keep the four: M = 15 181 -> 176 us.
+// (With N = 48, four A and two D steps are no better: the argmax head 163840 x 2560 at M = 16 75.1 us with two and four,
+// 77.5 with four and two; int8 weights 82.1 and 85.2.)
 template <int MT, bool ST>
 struct Geo {
   static constexpr bool kStream = ST;  // digit rows streamed from the pre-pass output instead of converted here
@@ -97,31 +95,31 @@ struct Geo {
   // accumulator columns [CB F, CB F + 3 TM), so every set runs the SAME code on its own aligned column block
   // (one copy of the fix-up code per kernel: the instruction footprint of all roles has to stay cache resident).
   //   MT:        1    2    4    6    8    9   12   15   16
-  //   FW x TM: 1x1  2x1  2x2  2x3  2x4  3x3  4x3  3x5  4x4
+  //   FW x TM: 1x1  2x1  2x2  2x3  2x4  3x3  3x4  3x5  4x4
   // A set is a chain of waits, tensor-memory loads and dependent arithmetic per step, so more and smaller sets go
   // faster until their fixed cost (about 60 instructions per warp and step) takes the issue slots: 248320 x 5120 in us,
-  //   M = 4: 2x2 109, 4x1 125;  M = 8: 2x4 135, 4x2 139;  M = 12: 3x4 161, 4x3 158;  M = 16: 2x8 275, 4x4 194
-  // and 34816 x 5120 before (scalar arithmetic; 3x4 at M = 12, 2x8 at M = 16) and now:
+  //   M = 4: 2x2 109, 4x1 125;  M = 8: 2x4 135, 4x2 139;  M = 12: 3x4 160, 4x3 158 (int8, 163840 x 2560: 75 and 78);
+  //   M = 16: 2x8 275, 4x4 194
+  // and 34816 x 5120 before (scalar arithmetic, a round of two steps per hand-off; 2x8 at M = 16) and now:
   //   M = 4 21.6 -> 20.0, M = 6 22.4 -> 21.9, M = 8 26.8 -> 24.2, M = 9 27.1 -> 25.0, M = 12 29.4 -> 28.3, M = 16 36.9 -> 32.4
-  static constexpr int FW = MT <= 1 ? 1 : (MT <= 8 ? 2 : (MT == 9 || MT == 15 ? 3 : 4));
+  static constexpr int FW = MT <= 1 ? 1 : (MT <= 8 ? 2 : (MT <= 15 ? 3 : 4));
   static constexpr int TM = (MT + FW - 1) / FW;                // tokens per fix-up warp
   static constexpr int CB = !ST ? 16 : (MT <= 2 ? 8 : (3 * TM + 3) / 4 * 4);  // accumulator columns per set
   static constexpr int TP = TM == 1 ? 1 : (TM + 1) / 2 * 2;    // a set's entries per group in the (sum, 2^-p) table: TP sums, TP scales
   static constexpr int kPairBytes = FW * TP * 8;               // the table's bytes per group
   static constexpr int kWarps = FW <= 3 ? 24 : 28;
   static constexpr int kThreads = kWarps * 32;
-  // The block size the compiler plans for sets the register limit: 80 (24 warps), 72 (28 warps) or, asked for with 1024
-  // threads, 64. The pre-pass's CTAs of the NEXT call want to sit beside this kernel's (4096 registers each): 24 warps
-  // of 80 leave room for one, 28 of 72 for none. Fewer registers pay where the code fits them; 34816, 17408 and 6144
+  // The block size the compiler plans for sets the register limit: 80 (24 warps) or, asked for with 1024 threads,
+  // 64. The pre-pass's CTAs of the NEXT call want to sit beside this kernel's (4096 registers each): 24 warps
+  // of 80 leave room for one, 28 of 72 (M = 16) for none. Fewer registers pay where the code fits them; 34816, 17408 and 6144
   // columns in us, default -> 64:
   //   M = 8  24.3 / 17.2 / 10.5 -> 24.2 / 15.7 / 9.6      M = 16 33.3 / 22.3 / 13.6 -> 32.4 / 21.9 / 12.6
   //   M = 6  21.9 / 15.1 / 8.6  -> 23.0 / 14.7 / 8.8      M = 9  25.2 / 17.1 / 9.3  -> 26.4 / 16.8 / 9.8
-  //   M = 12 28.5 / 19.1 / 11.8 -> 29.8 / 19.7 / 10.7     M = 15 30.5 / 20.2 / 12.1 -> 31.7 / 20.3 / 12.4
+  //   M = 15 30.5 / 20.2 / 12.1 -> 31.7 / 20.3 / 12.4
   static constexpr int kBoundThreads = MT == 8 || MT == 16 ? 1024 : kThreads;
   static constexpr int N = !ST ? 16 : ((FW * CB + 15) / 16) * 16;  // rows of the B operand the tensor core reads
-  static constexpr bool kFiveTokens = N == 48 && CB == 16;         // (MT = 15)
-  static constexpr int AD2 = kFiveTokens ? 2 : 4;
-  static constexpr int DD2 = N == 16 ? 8 : (N == 32 || kFiveTokens ? 4 : 2);
+  static constexpr int AD2 = N == 48 ? 2 : 4;
+  static constexpr int DD2 = N == 16 ? 8 : 4;
   static constexpr int ND = 8;                           // ring of "step done" barriers
   static constexpr int kAColsS = kStepGroups * kAColsG;  // A columns per step
   static constexpr int kDColsS = kStepGroups * N;        // D columns per step
@@ -1554,7 +1552,7 @@ int launch_batch_c(SkinnyParams& q, int grid, cudaStream_t st, int smem_optin) {
     case 6: return launch_cfg<6, WB, true, COMM>(q, grid, st, smem_optin);    // 3, M - 3
     case 8: return launch_cfg<8, WB, true, COMM>(q, grid, st, smem_optin);    // 4, M - 4
     case 9: return launch_cfg<9, WB, true, COMM>(q, grid, st, smem_optin);    // 3, 3, 3
-    case 12: return launch_cfg<12, WB, true, COMM>(q, grid, st, smem_optin);  // 3, 3, 3, M - 9
+    case 12: return launch_cfg<12, WB, true, COMM>(q, grid, st, smem_optin);  // 4, 4, M - 8
     case 15: return launch_cfg<15, WB, true, COMM>(q, grid, st, smem_optin);  // 5, 5, M - 10
     default: return launch_cfg<16, WB, true, COMM>(q, grid, st, smem_optin);  // 4, 4, 4, 4
   }
