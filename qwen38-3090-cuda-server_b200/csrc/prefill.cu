@@ -495,6 +495,8 @@ int prefill_smem(int tn, int wdepth) {
 // (4 TN cycles per group for a pair) and the expansion of the weights (kExpand cycles per group), plus
 // what is paid once per tile (pipeline fill, read-out of the accumulator, the exchange of split K). Tiles go to
 // the clusters in turn, dearest first, so cluster 0 has the longest list: its total is what is minimised.
+// (Measured against 256 tokens and no split for every shape: 5120 x 17408 at M = 77, 20 row pairs, takes 96 tokens and
+// three splits, 108 -> 31 us; 8192 x 5120 at M = 77 39 -> 21 us; 5120 x 8192 at M = 777 113 -> 82 us.)
 PrefillPlan plan_prefill(int M, int pairs, int G, const int* clusters_of_split, int smem_optin) {
   constexpr int kExpand = 420, kFill = 2500, kReduce = 4000;
   PrefillPlan best;
