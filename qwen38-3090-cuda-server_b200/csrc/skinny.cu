@@ -1503,9 +1503,25 @@ int instance_for(int M) {
 struct DigitGeometry {
   int tm, cb, tp, sets, nrows;
 };
+// What an instance's pre-pass writes per k group: the B operand's digit rows ([8 chunks of 16 k][N rows] 16 B), and
+// behind all groups' rows the table of sums and scales. A scratch serves every instance, so it holds the widest of each
+// (N = 48 rows; the table of three sets of five tokens, padded to six: 144 bytes, more than sixteen tokens' 128).
+template <int MT>
+constexpr int digit_bytes() {
+  return 128 * Geo<MT, true>::N;
+}
+template <int... MT>
+constexpr int widest_group() {
+  int digits = 0, pairs = 0;
+  ((digits = digit_bytes<MT>() > digits ? digit_bytes<MT>() : digits), ...);
+  ((pairs = Geo<MT, true>::kPairBytes > pairs ? Geo<MT, true>::kPairBytes : pairs), ...);
+  return digits + pairs;
+}
+constexpr int kPrepassGroupBytes = widest_group<1, 2, 4, 6, 8, 9, 12, 15, 16>();
 template <int MT>
 DigitGeometry geometry_of() {
   using GE = Geo<MT, true>;
+  static_assert(digit_bytes<MT>() + GE::kPairBytes <= kPrepassGroupBytes, "the scratch must hold every instance's pre-pass output");
   return {GE::TM, GE::CB, GE::TP, GE::FW, GE::N};
 }
 DigitGeometry digit_geometry(int M) {
@@ -1521,10 +1537,8 @@ DigitGeometry digit_geometry(int M) {
     default: return geometry_of<16>();
   }
 }
-// pre-pass output: per k group the B operand's digit rows, [8 chunks of 16 k][at most 48 rows] 16 B; behind all
-// groups' rows the table of sums and scales, at most 16 tokens x 8 bytes per group (+ 16 so that a bulk copy of the
-// rounded-up size stays inside)
-size_t prepass_bytes(int G) { return static_cast<size_t>(G) * (128 * 48 + 8 * 16) + 16; }
+// The pre-pass output's bytes for G k groups (+ 16: the table's bulk copy is rounded up to 16 bytes).
+size_t prepass_bytes(int G) { return static_cast<size_t>(G) * kPrepassGroupBytes + 16; }
 
 // A validated layer in either weight format, as the launcher sees it.
 struct LayerRef {
@@ -1799,7 +1813,7 @@ int w4a16_scratch_alloc(w4a16_scratch_t* s, int max_in, int max_out, int min_gro
   // two partial tiles per CTA (head and tail of its unit range), widest tile, 16 tokens, 8-byte (sum, tag) words
   s->partial_elems = static_cast<size_t>(s->max_splits) * 2 * kTileRows * 16 * 2;
   const size_t counters = counter_bytes(max_out);
-  // per-CTA argmax pairs, then (max_m >= 2) the pre-pass output: digit rows of up to 16 tokens for every k group
+  // per-CTA argmax pairs, then (max_m >= 2) the pre-pass output: digit rows and the table of sums and scales, whatever M <= 16
   const size_t pairs = pair_bytes(s->max_splits) +
                        (max_m >= 2 ? prepass_bytes(s->max_groups) : 0);
   void *xf = nullptr, *cn = nullptr, *pa = nullptr;
