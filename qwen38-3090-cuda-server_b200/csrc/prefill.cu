@@ -100,6 +100,11 @@ __device__ __forceinline__ void cluster_sync() {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// A whole warp's answer to a bounded wait. Lanes poll on their own, so when the limit runs out some may have seen the phase
+// complete and others not; what follows a wait is warp-collective (tensor-memory access, the elected issue, barriers), so
+// they have to agree. A warp that gave up sets the status word, does no more work and still reaches every barrier
+// that other warps wait at.
+__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok); }
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
@@ -247,11 +252,11 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
       int a = 0;
       for (int tile = cluster; !dead && tile < p.tiles; tile += nclusters, dph ^= 1) {
         const uint32_t idesc = umma_idesc_bf16(kPRows, tile_of(p, tile).n);
-        if (!mbar_wait_bounded(dempty_a, dph, kPSpin)) dead = true;  // (passes on the first tile)
+        if (!warp_agrees(mbar_wait_bounded(dempty_a, dph, kPSpin))) dead = true;  // (passes on the first tile)
         for (int g = g0; !dead && g < g1; ++g, ++j) {
           const uint32_t st = j & (kPSteps - 1);
-          if (!mbar_wait_bounded(xfull_a + st * 8, (j / kPSteps) & 1u, kPSpin) ||
-              !mbar_wait_bounded(afull_a + a * 8, aph, kPSpin)) {
+          if (!warp_agrees(mbar_wait_bounded(xfull_a + st * 8, (j / kPSteps) & 1u, kPSpin) &&
+                           mbar_wait_bounded(afull_a + a * 8, aph, kPSpin))) {
             dead = true;
             break;
           }
@@ -320,10 +325,7 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
     int st = team, a = team;  // weight stage and A slot
     uint32_t wph = 0;
     for (uint32_t j = team; j < ngroups; j += 2) {
-      if (!mbar_wait_bounded(wfull_a + st * 8, wph, kPSpin)) {
-        dead = true;
-        break;
-      }
+      const bool landed = mbar_wait_bounded(wfull_a + st * 8, wph, kPSpin);
       const uint8_t* blk = ring + st * kTileGroupBytes;
       const uint4 w0 = *reinterpret_cast<const uint4*>(blk + off0), w1 = *reinterpret_cast<const uint4*>(blk + off1);
       const uint32_t zp = blk[kTgZpOff + row];
@@ -339,11 +341,16 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
 #pragma unroll
           for (int pp = 0; pp < 4; ++pp)
             v[c][4 * i + pp] = mul_bf16x2(sub_bf16x2(((w[4 * c + i] >> (4 * pp)) & kNibMaskP) | kMagicP, zpair), spair);
-      __syncwarp();
+      // (the vote is also what tells lane 0 that the whole warp has read the stage)
+      if (!warp_agrees(landed)) {
+        dead = true;
+        break;
+      }
       if (lane == 0) mbar_arrive(wempty_a + st * 8);
       // only now the wait for the A slot: the MMAs that read it last, na groups ago, must have completed
       const uint32_t jd = j - na;
-      if (j >= static_cast<uint32_t>(na) && !mbar_wait_bounded(done_a + (jd & (kPDone - 1)) * 8, (jd / kPDone) & 1u, kPSpin)) {
+      if (!warp_agrees(j < static_cast<uint32_t>(na) ||
+                       mbar_wait_bounded(done_a + (jd & (kPDone - 1)) * 8, (jd / kPDone) & 1u, kPSpin))) {
         dead = true;
         break;
       }
@@ -360,7 +367,7 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
         wph ^= 1;
       }
     }
-    if (dead) atomicExch(p.status, W4A16_ETIMEOUT);
+    if (dead && lane == 0) atomicExch(p.status, W4A16_ETIMEOUT);
   } else if (S == 1) {
     // ================================================================ epilogue warps
     // The next tile's MMAs wait for the accumulator, so it is read out into shared memory (as bf16) and handed back;
@@ -371,26 +378,29 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
     uint32_t dph = 0;
     for (int tile = cluster; tile < p.tiles; tile += nclusters, dph ^= 1) {
       const PTile t = tile_of(p, tile);
-      if (!mbar_wait_bounded_relaxed(dfull_a, dph, kPSpin)) {
-        atomicExch(p.status, W4A16_ETIMEOUT);
-        break;
-      }
-      tc_fence_after();
       uint16_t* cs = reinterpret_cast<uint16_t*>(cbuf);
-#pragma unroll 2
-      for (int c = eh * 16; c < t.n; c += EW / 4 * 16) {
-        float v[16];
-        tmem_ld<16>(lane_t + c, v);
-        tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 16; ++i) cs[(c + i) * kTileRows + q * 32 + lane] = float_to_bf16_bits(v[i]);
+      if (!dead && !warp_agrees(mbar_wait_bounded_relaxed(dfull_a, dph, kPSpin))) {
+        dead = true;
+        if (lane == 0) atomicExch(p.status, W4A16_ETIMEOUT);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(dempty_l);
-      named_bar_sync(1, EW * 32);
+      if (!dead) {
+        tc_fence_after();
+#pragma unroll 2
+        for (int c = eh * 16; c < t.n; c += EW / 4 * 16) {
+          float v[16];
+          tmem_ld<16>(lane_t + c, v);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 16; ++i) cs[(c + i) * kTileRows + q * 32 + lane] = float_to_bf16_bits(v[i]);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(dempty_l);
+      }
+      named_bar_sync(1, EW * 32);  // every epilogue warp comes here for every tile, dead or not
       const int r0 = (2 * t.pair + half) * kTileRows;
-      const int rows = min(kTileRows, p.N - r0), toks = min(t.n, p.M - t.tok0);  // (rows <= 0: an odd last row tile's second half)
+      const int rows = min(kTileRows, p.N - r0);                     // (<= 0: an odd last row tile's second half)
+      const int toks = dead ? 0 : min(t.n, p.M - t.tok0);
       if (p.wide) {
         const int rl = (et & 15) * 8;  // eight rows of one token per thread
         if (rl < rows) {
@@ -424,7 +434,7 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
     if (warp >= kWEpi0 && warp < kWEpi0 + EW) {
       const int q = warp & 3;
       const uint32_t lane_t = tmem + (static_cast<uint32_t>(q * 32) << 16);
-      if (mbar_wait_bounded(dfull_a, 0, kPSpin)) {
+      if (warp_agrees(mbar_wait_bounded(dfull_a, 0, kPSpin))) {
         tc_fence_after();
         float* tile_s = reinterpret_cast<float*>(xbuf) + q * 32 + lane;
 #pragma unroll 1
@@ -435,7 +445,7 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
 #pragma unroll
           for (int i = 0; i < 16; ++i) tile_s[(c + i) * kTileRows] = v[i];
         }
-      } else {
+      } else if (lane == 0) {
         atomicExch(p.status, W4A16_ETIMEOUT);
       }
     }
