@@ -154,6 +154,11 @@ __device__ __forceinline__ bool mbar_wait_bounded_relaxed(uint32_t bar, uint32_t
   }
   return false;
 }
+// A whole warp's answer to a bounded wait. Lanes poll on their own, so when the limit runs out some may have seen the phase
+// complete and others not; what follows a wait is warp-collective (tensor-memory access, the elected issue, barriers), so
+// they have to agree. A warp that gave up sets the status word, does no more work and still reaches every barrier
+// that other warps wait at.
+__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok); }
 // 1-D bulk async copy global -> this CTA's shared memory, completion on an mbarrier.
 // dst, src 16-byte aligned; bytes a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes,

@@ -100,11 +100,6 @@ __device__ __forceinline__ void cluster_sync() {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// A whole warp's answer to a bounded wait. Lanes poll on their own, so when the limit runs out some may have seen the phase
-// complete and others not; what follows a wait is warp-collective (tensor-memory access, the elected issue, barriers), so
-// they have to agree. A warp that gave up sets the status word, does no more work and still reaches every barrier
-// that other warps wait at.
-__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok); }
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");

@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
   constexpr uint32_t tmem = 0;
   const bool uses_tmem = warp < kWProducer || warp == kWMma || warp == kWMma2 || warp >= kWConv0;
   if (uses_tmem) {
-    if (!wait_h(tmemrdy_a, 0, p.hint, kSpinLimit) || *reinterpret_cast<volatile uint32_t*>(tmem_slot) != 0u) {
+    if (!warp_agrees(wait_h(tmemrdy_a, 0, p.hint, kSpinLimit)) || *reinterpret_cast<volatile uint32_t*>(tmem_slot) != 0u) {
       atomicExch(p.status, W4A16_ETIMEOUT);
       team_ok = false;
     }
@@ -654,16 +654,16 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
         const int a = t & (AD2 - 1), d = t & (DD2 - 1);
         // A written (its writers also saw the step's weights and table entry landed), and the D slot this
         // step fills has been read out by every fix-up warp
-        if (!wait_h(afull_a + a * 8, static_cast<uint32_t>(t / AD2) & 1u, p.hint, kSpinLimit) ||
-            (GE::kIssuerWaitsD && t >= DD2 &&
-             !wait_h(dempty_a + d * 8, static_cast<uint32_t>(t / DD2 - 1) & 1u, p.hint, kSpinLimit))) {
+        if (!warp_agrees(wait_h(afull_a + a * 8, static_cast<uint32_t>(t / AD2) & 1u, p.hint, kSpinLimit) &&
+                         (!GE::kIssuerWaitsD || t < DD2 ||
+                          wait_h(dempty_a + d * 8, static_cast<uint32_t>(t / DD2 - 1) & 1u, p.hint, kSpinLimit)))) {
           atomicExch(p.status, W4A16_ETIMEOUT);
           break;
         }
         const uint32_t e = table[t & (kTable - 1)].x;
         if constexpr (kStream) {
           // the step's digit rows have landed in their ring slot (bulk copy: async proxy, as the MMA reads them)
-          if (!wait_h(bfull_a + (t & (BD - 1)) * 8, static_cast<uint32_t>(t >> BS) & 1u, p.hint, kSpinLimit)) {
+          if (!warp_agrees(wait_h(bfull_a + (t & (BD - 1)) * 8, static_cast<uint32_t>(t >> BS) & 1u, p.hint, kSpinLimit))) {
             atomicExch(p.status, W4A16_ETIMEOUT);
             break;
           }
@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
             if (++spins > kSpinLimit) break;
             __nanosleep(40);
           }
-          if (spins > kSpinLimit) {
+          if (!warp_agrees(spins <= kSpinLimit)) {
             atomicExch(p.status, W4A16_ETIMEOUT);
             break;
           }
@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
     bool ok = team_ok;
     for (int t = pair; ok && t < T; t += 2) {
       const int a = t & (AD2 - 1);
-      if (!wait_h(wfull_a + st * 8, wph, p.hint, kSpinLimit)) {
+      if (!warp_agrees(wait_h(wfull_a + st * 8, wph, p.hint, kSpinLimit))) {
         atomicExch(p.status, W4A16_ETIMEOUT);
         break;
       }
@@ -739,10 +739,10 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
       load_row(base);
       // the A slot's previous step has been multiplied (whether the D slot is free is the issuer's concern: the
       // operand can be unpacked while the fix-up warps are still reading the sums of DD2 steps ago)
-      if ((t >= AD2 && !wait_h(done_a + ((t - AD2) & (ND - 1)) * 8, static_cast<uint32_t>((t - AD2) / ND) & 1u, p.hint,
-                               kSpinLimit)) ||
-          (!GE::kIssuerWaitsD && t >= DD2 &&
-           !wait_h(dempty_a + (t & (DD2 - 1)) * 8, static_cast<uint32_t>(t / DD2 - 1) & 1u, p.hint, kSpinLimit))) {
+      if (!warp_agrees((t < AD2 || wait_h(done_a + ((t - AD2) & (ND - 1)) * 8, static_cast<uint32_t>((t - AD2) / ND) & 1u,
+                                          p.hint, kSpinLimit)) &&
+                       (GE::kIssuerWaitsD || t < DD2 ||
+                        wait_h(dempty_a + (t & (DD2 - 1)) * 8, static_cast<uint32_t>(t / DD2 - 1) & 1u, p.hint, kSpinLimit)))) {
         atomicExch(p.status, W4A16_ETIMEOUT);
         break;
       }
@@ -918,7 +918,7 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
     const float2* xs_tab = reinterpret_cast<const float2*>(xsinv);  // M = 1: (sum, 2^-p) per cache slot or (pre-pass) per k group
     if constexpr (kStream) {
       // the pair table of the call arrives once, by bulk copy
-      if (!wait_h(bready_a, 0, p.hint, kSpinLimit)) {
+      if (!warp_agrees(wait_h(bready_a, 0, p.hint, kSpinLimit))) {
         atomicExch(p.status, W4A16_ETIMEOUT);
         ok = false;
       }
@@ -930,7 +930,7 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
       int seg_tile = 0;
       if (helper) {
         const float* mslot = mail + (nmail * CW + q) * kMailStride;
-        if (!wait_h(mailfull_a + (nmail * CW + q) * 8, 0, p.hint, 4 * kSpinLimit)) {
+        if (!warp_agrees(wait_h(mailfull_a + (nmail * CW + q) * 8, 0, p.hint, 4 * kSpinLimit))) {
           atomicExch(p.status, W4A16_ETIMEOUT);
           break;
         }
@@ -940,14 +940,14 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
       } else {
       // A round is one or (M = 1) two steps (two unless the first ends its segment): one wait per issuer (a commit
       // covers everything its thread issued before), GB groups' tensor-memory loads in flight together.
-      if (!wait_h(done_a + (t & (ND - 1)) * 8, static_cast<uint32_t>(t / ND) & 1u, p.hint, kSpinLimit)) {
+      if (!warp_agrees(wait_h(done_a + (t & (ND - 1)) * 8, static_cast<uint32_t>(t / ND) & 1u, p.hint, kSpinLimit))) {
         atomicExch(p.status, W4A16_ETIMEOUT);
         ok = false;
         break;
       }
       const uint2 e0 = table[t & (kTable - 1)];  // written before the step's weights were requested
       const bool two = GE::kPairRounds && !((e0.x >> 17) & 1u) && t + 1 < T;
-      if (two && !wait_h(done_a + ((t + 1) & (ND - 1)) * 8, static_cast<uint32_t>((t + 1) / ND) & 1u, p.hint, kSpinLimit)) {
+      if (two && !warp_agrees(wait_h(done_a + ((t + 1) & (ND - 1)) * 8, static_cast<uint32_t>((t + 1) / ND) & 1u, p.hint, kSpinLimit))) {
         atomicExch(p.status, W4A16_ETIMEOUT);
         ok = false;
         break;
