@@ -225,6 +225,12 @@ int w4a16_workspace_free(w4a16_workspace_t* ws);
  * any M >= 1, bf16 in/out, fp32 accumulate, dequantisation fused into the tensor-core tiles. */
 int w4a16_gemm_prefill(uint16_t* C, const w4a16_weights_t* w, const uint16_t* A, int M,
                        w4a16_workspace_t* ws, void* stream);
+/* The launch shape w4a16_gemm_prefill takes on the current device for M tokens through an out_f x in_f
+ * layer: tokens per tile, and the number of consecutive pieces K is summed in (1..4; the pieces' fp32 sums
+ * are added in order). It follows from the sizes and the device alone. Every result is reproducible, and a
+ * row has the same bits in any two calls with the same k_splits; with different ones it may differ by the
+ * order of the fp32 sum. No counterpart in the reference. */
+int w4a16_prefill_plan(int M, int out_f, int in_f, int* tokens_per_tile, int* k_splits);
 
 /* Column (output-row) sharding over the GPUs of one node. No reference
  * counterpart (the reference is single-GPU; README.md:123). Rank r of nranks owns

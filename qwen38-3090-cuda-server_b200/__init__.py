@@ -106,6 +106,7 @@ _SIGNATURES = {
     "w4a16_workspace_free": (C.c_int, [C.POINTER(Workspace)]),
     "w4a16_gemm_prefill": (C.c_int, [C.c_void_p, C.POINTER(Weights), C.c_void_p, C.c_int,
                                      C.POINTER(Workspace), C.c_void_p]),
+    "w4a16_prefill_plan": (C.c_int, [C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "w4a16_gemm_skinny_gather": (C.c_int, [C.POINTER(C.c_void_p), C.POINTER(Comm), C.c_int, C.c_int, C.c_int,
                                            C.POINTER(Weights), C.c_void_p, C.c_int, C.POINTER(Scratch), C.c_void_p]),
     "w4a16_gemm_skinny_partial": (C.c_int, [C.POINTER(C.c_void_p), C.POINTER(Comm), C.POINTER(Weights), C.c_void_p,
@@ -263,6 +264,13 @@ def gemm_workspace_free(ws: Workspace):
 
 def gemm_w4a16(Cout, w: Weights, A, M: int, ws: Workspace, stream=None):
     check(lib().w4a16_gemm_prefill(_ptr(Cout), C.byref(w), _ptr(A), M, C.byref(ws), _stream(stream)))
+
+
+def prefill_plan(M: int, out_f: int, in_f: int):
+    """(tokens per tile, K splits) of gemm_w4a16 for M tokens through an out_f x in_f layer on the current device."""
+    tokens, splits = C.c_int(), C.c_int()
+    check(lib().w4a16_prefill_plan(M, out_f, in_f, C.byref(tokens), C.byref(splits)))
+    return tokens.value, splits.value
 
 
 def shard_rows(out_f: int, nranks: int, rank: int):

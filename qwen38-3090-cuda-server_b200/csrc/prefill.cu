@@ -606,6 +606,17 @@ const int* cluster_slots(int dev, const DeviceInfo* di) {
   return s.n;
 }
 
+// The current device's plan for M tokens through a layer of `row_tiles` row tiles and G k groups.
+int current_plan(PrefillPlan& plan, int M, int row_tiles, int G) {
+  const DeviceInfo* di = device_info();
+  if (!di) return W4A16_ECUDA;
+  const int* slots = cluster_slots(di->device, di);
+  if (!slots) return W4A16_ECUDA;
+  plan = plan_prefill(M, (row_tiles + 1) / 2, G, slots, di->smem_optin);
+  W4_REQUIRE(plan.tn > 0, "gemm_prefill: no launch shape for M = %d, %d row tiles x %d k groups", M, row_tiles, G);
+  return W4A16_OK;
+}
+
 int launch_prefill(PrefillParams& p, uint16_t* C, const w4a16_weights_t* w, const uint16_t* A, int M, w4a16_workspace_t* ws,
                    void* stream) {
   if (int rc = check_weights(w)) return rc;
@@ -615,10 +626,6 @@ int launch_prefill(PrefillParams& p, uint16_t* C, const w4a16_weights_t* w, cons
   W4_REQUIRE(ws != nullptr, "gemm_prefill: null workspace");
   const DeviceInfo* di = device_info();
   if (!di) return W4A16_ECUDA;
-  int dev = 0;
-  W4_CUDA(cudaGetDevice(&dev));
-  const int* slots = cluster_slots(dev, di);
-  if (!slots) return W4A16_ECUDA;
   p.stream = reinterpret_cast<const uint8_t*>(w->qweight);
   p.C = C;
   p.M = M;
@@ -627,8 +634,8 @@ int launch_prefill(PrefillParams& p, uint16_t* C, const w4a16_weights_t* w, cons
   p.G = w->num_groups;
   p.row_tiles = (w->out_f + kTileRows - 1) / kTileRows;
   p.pairs = (p.row_tiles + 1) / 2;
-  const PrefillPlan plan = plan_prefill(M, p.pairs, p.G, slots, di->smem_optin);
-  W4_REQUIRE(plan.tn > 0, "gemm_prefill: no launch shape for M = %d, %d x %d", M, w->out_f, w->in_f);
+  PrefillPlan plan;
+  if (int rc = current_plan(plan, M, p.row_tiles, p.G)) return rc;
   p.tn = plan.tn;
   p.splits = plan.splits;
   p.wdepth = plan.wdepth;
@@ -674,6 +681,17 @@ int w4a16_gemm_prefill(uint16_t* C, const w4a16_weights_t* w, const uint16_t* A,
   PrefillParams p = {};
   p.ldc = w ? w->out_f : 0;
   return launch_prefill(p, C, w, A, M, ws, stream);
+}
+
+int w4a16_prefill_plan(int M, int out_f, int in_f, int* tokens_per_tile, int* k_splits) {
+  W4_REQUIRE(tokens_per_tile != nullptr && k_splits != nullptr, "prefill_plan: null output");
+  W4_REQUIRE(M >= 1 && out_f > 0 && out_f % kRowGranule == 0 && in_f > 0 && in_f % kGroup == 0,
+             "prefill_plan: M = %d, %d x %d", M, out_f, in_f);
+  PrefillPlan plan;
+  if (int rc = current_plan(plan, M, (out_f + kTileRows - 1) / kTileRows, in_f / kGroup)) return rc;
+  *tokens_per_tile = plan.tn;
+  *k_splits = plan.splits;
+  return W4A16_OK;
 }
 
 int w4a16_gemm_prefill_sharded(uint16_t* const* C_peers, const w4a16_comm_t* comm, int out_f_total, int row_begin,

@@ -51,8 +51,48 @@ def test_row_and_token_edges(N, M):
 
 @pytest.mark.parametrize("K", [128, 256, 640, 2176])
 @pytest.mark.parametrize("M", [17, 96, 193, 300])
-def test_k_groups_and_splits(K, M):
+def test_k_groups_in_one_piece(K, M):
+    assert pkg.prefill_plan(M, 512, K)[1] == 1
     _check(512, K, M)
+
+
+# Layers of few tiles and many k groups, which take 2, 3 or 4 splits: odd numbers of row tiles and a last one of 16 rows,
+# ragged token tiles, several of them, k groups that do not divide, outputs that do not take 16-byte stores.
+SPLIT = [(16, 4096, 33, 0), (272, 4096, 1, 0), (272, 5120, 300, 1), (400, 17408, 77, 0), (1040, 4224, 130, 4),
+         (5120, 4096, 77, 0), (5120, 17408, 17, 0), (5120, 17408, 200, 1), (8192, 4224, 77, 0), (8192, 5120, 100, 0)]
+
+
+@pytest.mark.parametrize("N,K,M,skew", SPLIT)
+def test_split_k(N, K, M, skew):
+    assert pkg.prefill_plan(M, N, K)[1] > 1
+    _check(N, K, M, skew)
+
+
+def test_split_cases_cover_every_count():
+    assert {pkg.prefill_plan(M, N, K)[1] for N, K, M, _ in SPLIT} == {2, 3, 4}
+
+
+@pytest.mark.parametrize("K", [512, 4096])
+def test_a_row_depends_on_the_splits_only(K):
+    """Calls with the same number of splits give a row the same bits, whatever M and the tile."""
+    N = 400
+    w, _ = _layer(N, K, seed=7)
+    x = torch.randn((1300, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(7)).to(torch.bfloat16)
+    ws = pkg.gemm_workspace_alloc(4096)
+    first, tokens = {}, {}
+    for M in (1, 33, 77, 130, 300, 520, 1000, 1300):
+        tn, splits = pkg.prefill_plan(M, N, K)
+        c = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+        pkg.gemm_w4a16(c, w, x[:M], M, ws)
+        seen = first.setdefault(splits, c)
+        tokens.setdefault(splits, set()).add(tn)
+        n = min(M, seen.shape[0])
+        assert torch.equal(c[:n].view(torch.int16), seen[:n].view(torch.int16)), (M, tn, splits)
+        if M > seen.shape[0]:
+            first[splits] = c
+    assert pkg.device_status() == 0 and any(len(t) > 1 for t in tokens.values())
+    pkg.gemm_workspace_free(ws)
+    pkg.awq_free(w)
 
 
 @pytest.mark.parametrize("N,K,M", [(5120, 1024, 777), (19072, 256, 520), (4736, 512, 2100)])
