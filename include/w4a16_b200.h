@@ -229,7 +229,8 @@ int w4a16_gemm_prefill(uint16_t* C, const w4a16_weights_t* w, const uint16_t* A,
  * layer: tokens per tile, and the number of consecutive pieces K is summed in (1..4; the pieces' fp32 sums
  * are added in order). It follows from the sizes and the device alone. Every result is reproducible, and a
  * row has the same bits in any two calls with the same k_splits; with different ones it may differ by the
- * order of the fp32 sum. No counterpart in the reference. */
+ * order of the fp32 sum. A sharded call takes the k_splits of the whole layer (out_f_total), so it gives the
+ * bits of the unsharded one. No counterpart in the reference. */
 int w4a16_prefill_plan(int M, int out_f, int in_f, int* tokens_per_tile, int* k_splits);
 
 /* Column (output-row) sharding over the GPUs of one node. No reference

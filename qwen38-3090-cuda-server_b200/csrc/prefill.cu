@@ -502,13 +502,14 @@ int prefill_smem(int tn, int wdepth) {
 // the clusters in turn, dearest first, so cluster 0 has the longest list: its total is what is minimised.
 // (Measured against 256 tokens and no split for every shape: 5120 x 17408 at M = 77, 20 row pairs, takes 96 tokens and
 // three splits, 108 -> 31 us; 8192 x 5120 at M = 77 39 -> 21 us; 5120 x 8192 at M = 777 113 -> 82 us.)
-PrefillPlan plan_prefill(int M, int pairs, int G, const int* clusters_of_split, int smem_optin) {
+// `only` > 0 asks for that number of splits.
+PrefillPlan plan_prefill(int M, int pairs, int G, const int* clusters_of_split, int smem_optin, int only) {
   constexpr int kExpand = 420, kFill = 2500, kReduce = 4000;
   PrefillPlan best;
   long long best_cost = -1;
   for (int S = 1; S <= kPMaxSplit && S <= G; ++S) {
     const int slots = clusters_of_split[S];
-    if (slots < 1) continue;
+    if (slots < 1 || (only > 0 && S != only)) continue;
     for (int tn = 32; tn <= kPMaxTN; tn += 32) {
       const int full = M / tn, rest = M - full * tn;
       if (full == 0 && tn - 32 >= rest) break;  // one token tile: the smallest that holds M
@@ -606,13 +607,17 @@ const int* cluster_slots(int dev, const DeviceInfo* di) {
   return s.n;
 }
 
-// The current device's plan for M tokens through a layer of `row_tiles` row tiles and G k groups.
-int current_plan(PrefillPlan& plan, int M, int row_tiles, int G) {
+// The current device's plan for M tokens through `row_tiles` row tiles and G k groups of a layer of `layer_tiles` row
+// tiles. A shard is split as the whole layer would be, so that a row has the same bits sharded and unsharded; as its
+// tiles are fewer, they always fit the clusters that the layer's would. (What the shard's own choice would save is left.)
+int current_plan(PrefillPlan& plan, int M, int row_tiles, int layer_tiles, int G) {
   const DeviceInfo* di = device_info();
   if (!di) return W4A16_ECUDA;
   const int* slots = cluster_slots(di->device, di);
   if (!slots) return W4A16_ECUDA;
-  plan = plan_prefill(M, (row_tiles + 1) / 2, G, slots, di->smem_optin);
+  plan = plan_prefill(M, (layer_tiles + 1) / 2, G, slots, di->smem_optin, 0);
+  if (row_tiles < layer_tiles && plan.tn > 0)
+    plan = plan_prefill(M, (row_tiles + 1) / 2, G, slots, di->smem_optin, plan.splits);
   W4_REQUIRE(plan.tn > 0, "gemm_prefill: no launch shape for M = %d, %d row tiles x %d k groups", M, row_tiles, G);
   return W4A16_OK;
 }
@@ -635,7 +640,8 @@ int launch_prefill(PrefillParams& p, uint16_t* C, const w4a16_weights_t* w, cons
   p.row_tiles = (w->out_f + kTileRows - 1) / kTileRows;
   p.pairs = (p.row_tiles + 1) / 2;
   PrefillPlan plan;
-  if (int rc = current_plan(plan, M, p.row_tiles, p.G)) return rc;
+  const int layer_tiles = static_cast<int>((p.ldc + kTileRows - 1) / kTileRows);
+  if (int rc = current_plan(plan, M, p.row_tiles, layer_tiles, p.G)) return rc;
   p.tn = plan.tn;
   p.splits = plan.splits;
   p.wdepth = plan.wdepth;
@@ -688,7 +694,8 @@ int w4a16_prefill_plan(int M, int out_f, int in_f, int* tokens_per_tile, int* k_
   W4_REQUIRE(M >= 1 && out_f > 0 && out_f % kRowGranule == 0 && in_f > 0 && in_f % kGroup == 0,
              "prefill_plan: M = %d, %d x %d", M, out_f, in_f);
   PrefillPlan plan;
-  if (int rc = current_plan(plan, M, (out_f + kTileRows - 1) / kTileRows, in_f / kGroup)) return rc;
+  const int row_tiles = (out_f + kTileRows - 1) / kTileRows;
+  if (int rc = current_plan(plan, M, row_tiles, row_tiles, in_f / kGroup)) return rc;
   *tokens_per_tile = plan.tn;
   *k_splits = plan.splits;
   return W4A16_OK;

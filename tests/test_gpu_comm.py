@@ -196,6 +196,35 @@ def test_sharded_prefill_two_emulated_ranks(pkg, synth, sharding):
         pkg.awq_free(w)
 
 
+@pytest.mark.parametrize("N,K,M,splits,own", [(4096, 4096, 300, 1, 2), (8192, 4224, 77, 2, 3), (5120, 4096, 50, 3, 4)])
+def test_sharded_prefill_is_split_as_the_whole_layer(pkg, synth, sharding, N, K, M, splits, own):
+    """Shapes whose half layer alone would sum K in other pieces than the layer: the sharded call gives the unsharded
+    bits, split tiles are stored into every rank's C and the launch's flag is complete."""
+    R = 2
+    assert (pkg.prefill_plan(M, N, K)[1], pkg.prefill_plan(M, N // R, K)[1]) == (splits, own)
+    _, full, parts = _shards(pkg, synth, sharding, N, K, R, seed=97)
+    x = dev_bf16(synth.make_activations(M, K, seed=97))
+    ws = pkg.gemm_workspace_alloc(4096)
+    cs = [torch.zeros((M, N), dtype=torch.bfloat16, device="cuda") for _ in range(R)]
+    flags, ptrs = _blocks(R)
+    torch.cuda.synchronize()
+    comms = [pkg.make_comm(ptrs, r) for r in range(R)]
+    for r in range(R):
+        pkg.gemm_w4a16_sharded([c.data_ptr() for c in cs], comms[r], N, parts[r][1], parts[r][0], x, M, ws)
+    want = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    pkg.gemm_w4a16(want, full, x, M, ws)
+    torch.cuda.synchronize()
+    assert pkg.device_status() == 0
+    f = flags.cpu().numpy()
+    assert (f[:, :R] == 65536).all() and (f[:, 16] == 1).all()
+    for c in cs:
+        assert torch.equal(c.view(torch.int16), want.view(torch.int16))
+    pkg.gemm_workspace_free(ws)
+    pkg.awq_free(full)
+    for w, _ in parts:
+        pkg.awq_free(w)
+
+
 @pytest.mark.parametrize("M", [1, 8])
 def test_gather_free_mlp_two_emulated_ranks(pkg, oracle, synth, sharding, M):
     """gate|up row-sharded with the SwiGLU epilogue (no exchange) -> K-sharded down -> fp32 partials into every
