@@ -227,7 +227,7 @@ int w4a16_gemm_prefill(uint16_t* C, const w4a16_weights_t* w, const uint16_t* A,
                        w4a16_workspace_t* ws, void* stream);
 /* The launch shape w4a16_gemm_prefill takes on the current device for M tokens through an out_f x in_f
  * layer: tokens per tile, and the number of consecutive pieces K is summed in (1..4; the pieces' fp32 sums
- * are added in order). It follows from the sizes and the device alone. Every result is reproducible, and a
+ * are added in order). It follows from the sizes alone, the same on every B200. Every result is reproducible, and a
  * row has the same bits in any two calls with the same k_splits; with different ones it may differ by the
  * order of the fp32 sum. A sharded call takes the k_splits of the whole layer (out_f_total), so it gives the
  * bits of the unsharded one. No counterpart in the reference. */

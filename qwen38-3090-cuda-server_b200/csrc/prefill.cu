@@ -502,14 +502,17 @@ int prefill_smem(int tn, int wdepth) {
 // the clusters in turn, dearest first, so cluster 0 has the longest list: its total is what is minimised.
 // (Measured against 256 tokens and no split for every shape: 5120 x 17408 at M = 77, 20 row pairs, takes 96 tokens and
 // three splits, 108 -> 31 us; 8192 x 5120 at M = 77 39 -> 21 us; 5120 x 8192 at M = 777 113 -> 82 us.)
-// `only` > 0 asks for that number of splits.
-PrefillPlan plan_prefill(int M, int pairs, int G, const int* clusters_of_split, int smem_optin, int only) {
+// `only` > 0 asks for that number of splits. The choice goes by what a B200 of 148 SMs runs (index S: clusters of 2 S CTAs
+// at once, as cudaOccupancyMaxActiveClusters answers on two of them), not by what this device's GPCs happen to fit, so that a
+// row has the same bits on every GPU; the device only rules out clusters it cannot run at all and sizes the grid.
+PrefillPlan plan_prefill(int M, int pairs, int G, const int* device_clusters, int smem_optin, int only) {
+  constexpr int kClusters[kPMaxSplit + 1] = {0, 74, 33, 22, 15};
   constexpr int kExpand = 420, kFill = 2500, kReduce = 4000;
   PrefillPlan best;
   long long best_cost = -1;
   for (int S = 1; S <= kPMaxSplit && S <= G; ++S) {
-    const int slots = clusters_of_split[S];
-    if (slots < 1 || (only > 0 && S != only)) continue;
+    const int slots = kClusters[S];
+    if (device_clusters[S] < 1 || (only > 0 && S != only)) continue;
     for (int tn = 32; tn <= kPMaxTN; tn += 32) {
       const int full = M / tn, rest = M - full * tn;
       if (full == 0 && tn - 32 >= rest) break;  // one token tile: the smallest that holds M
@@ -529,7 +532,7 @@ PrefillPlan plan_prefill(int M, int pairs, int G, const int* clusters_of_split, 
         best.splits = S;
         best.full_tt = full;
         best.tiles = static_cast<int>(tiles);
-        best.clusters = static_cast<int>(tiles < slots ? tiles : slots);
+        best.clusters = static_cast<int>(S > 1 || tiles < device_clusters[S] ? tiles : device_clusters[S]);
       }
     }
   }

@@ -72,6 +72,14 @@ def test_split_cases_cover_every_count():
     assert {pkg.prefill_plan(M, N, K)[1] for N, K, M, _ in SPLIT} == {2, 3, 4}
 
 
+def test_the_plan_is_fixed():
+    """The number of splits decides a row's bits, so it must not follow the device: 33, 22 and 15 clusters of four, six
+    and eight CTAs are what the plan goes by (the first two shapes are one row pair beyond 33 clusters and just within)."""
+    want = [(64, 8704, 5120, 32, 1), (64, 8448, 5120, 64, 2), (300, 2048, 4096, 96, 2), (130, 1040, 4224, 64, 4),
+            (77, 5120, 17408, 96, 3), (777, 5120, 8192, 128, 1), (4096, 34816, 5120, 256, 1)]
+    assert [pkg.prefill_plan(M, N, K) for M, N, K, _, _ in want] == [w[3:] for w in want]
+
+
 @pytest.mark.parametrize("K", [512, 4096])
 def test_a_row_depends_on_the_splits_only(K):
     """Calls with the same number of splits give a row the same bits, whatever M and the tile."""
