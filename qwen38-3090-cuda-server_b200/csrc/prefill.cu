@@ -26,14 +26,17 @@
 //   * few tiles (short prompts, narrow layers): a cluster of 2 S CTAs splits K S ways; the splits' fp32 tiles
 //     are added through distributed shared memory, always in split order (bitwise reproducible).
 //
-// What bounds it: long prompts run at the tensor cores' rate under the power cap (256 x 256 x 16 per 128 cycles; the
-// expansion of a group needs about 500 issue and ALU cycles of the 1024 its MMAs take), short ones at the
-// expansion of the weights. Measured against one CTA per tile of 128 x 256 with eight dequant warps:
-//   34816 x 5120, M = 4096: 1238 -> 890 us (1641 TFLOP/s); 5120 x 17408, M = 4096: 674 -> 475 us (1537)
-//   34816 x 5120, M = 777:   344 -> 202 us;                5120 x 8192, M = 777:   113 -> 82 us
-//   34816 x 5120, M = 77:     76 -> 52 us;                 5120 x 17408, M = 77:  108 -> 31 us
-// and on the way: half groups as the unit of every hand-off 1134 us (the first shape; the issuing thread is the
-// limit), whole groups 1063, two teams of dequant warps and C through shared memory 890.
+// What bounds it: long prompts run at the tensor cores' rate under the power cap (256 x 256 x 16 per 128 cycles: 1024
+// cycles per k group; tensor pipe 87.5 % active over a 4096-token launch), short ones at the expansion of the weights: a
+// CTA and k group is about 2400 warp instructions, 600 cycles if every issue slot were taken, and about 850 as it runs (0.62
+// of the slots, ALU pipe 54 to 68 % active), where HBM would allow 386.
+// In us, weights cold, against one CTA per tile of 128 x 256 with eight dequant warps:
+//   34816 x 5120, M = 4096: 1264 -> 922 (1583 TFLOP/s); 5120 x 17408, M = 4096: 698 -> 488 (1497)
+//   34816 x 5120, M = 777:   300 -> 202;                5120 x 8192, M = 777:   110 -> 57
+//   34816 x 5120, M = 77:     73 -> 37;                 5120 x 17408, M = 77:   105 -> 25;     8192 x 5120, M = 77: 45 -> 20
+// and on the way, 34816 x 5120 at M = 4096 on one device: half groups as the unit of every hand-off 1134 (the first shape; the
+// issuing thread is the limit), whole groups 1063, two teams of dequant warps and C through shared memory 890. A warp's vote on
+// its waits took another 9 % off short prompts (34816 x 5120 at M = 77: 40.8 -> 37.1) by keeping the loops warp-uniform.
 #include <cuda.h>
 #include <cstring>
 #include <mutex>
@@ -500,8 +503,12 @@ int prefill_smem(int tn, int wdepth) {
 // (4 TN cycles per group for a pair) and the expansion of the weights (kExpand cycles per group), plus
 // what is paid once per tile (pipeline fill, read-out of the accumulator, the exchange of split K). Tiles go to
 // the clusters in turn, dearest first, so cluster 0 has the longest list: its total is what is minimised.
-// (Measured against 256 tokens and no split for every shape: 5120 x 17408 at M = 77, 20 row pairs, takes 96 tokens and
-// three splits, 108 -> 31 us; 8192 x 5120 at M = 77 39 -> 21 us; 5120 x 8192 at M = 777 113 -> 82 us.)
+// The constants rank the shapes, they do not predict times: a group of a short prompt takes twice kExpand (see above).
+// Against every other (TN, S), on 20 shapes of 1024..34816 rows, 4096..17408 columns and 24..1500 tokens: the choice was the
+// fastest on 18. 5120 x 17408 at M = 24: 32 tokens and three splits 23.6 us, two 31.5, four 36.8, one 55.1; 6144 x 5120 at
+// M = 100: two splits 17.7, one 22.0; 34816 x 5120 at M = 520: 192 tokens 137, 224 148, 160 152, 128 176. Where kExpand misleads
+// it, tiles come out too narrow: 34816 x 5120 at M = 1024 128 tokens 284 us, 224 277; 12288 x 4096 at M = 200 96 tokens 32.1
+// us, 224 25.2.
 // `only` > 0 asks for that number of splits. The choice goes by what a B200 of 148 SMs runs (index S: clusters of 2 S CTAs
 // at once, as cudaOccupancyMaxActiveClusters answers on two of them), not by what this device's GPCs happen to fit, so that a
 // row has the same bits on every GPU; the device only rules out clusters it cannot run at all and sizes the grid.

@@ -85,8 +85,8 @@ constexpr int kAColsG = 32;                // 128 int8 along k = 32 columns of 3
 
 // Per token-count geometry. N = rows of the B operand the tensor core reads (3 digit rows per token are
 // real). Ring depths are in steps: AD2 for A, DD2 for D.
-// (With N = 48, four A and two D steps are no better: the argmax head 163840 x 2560 at M = 16 75.1 us with two and four,
-// 77.5 with four and two; int8 weights 82.1 and 85.2.)
+// (With N = 48, four A and two D steps are no better: when this was compared, the argmax head 163840 x 2560 at M = 16 took
+// 75.1 us with two and four, 77.5 with four and two, with int8 weights 82.1 and 85.2; now 63.0 and 72.7.)
 template <int MT, bool ST>
 struct Geo {
   static constexpr bool kStream = ST;  // digit rows streamed from the pre-pass output instead of converted here
@@ -98,10 +98,13 @@ struct Geo {
   //   FW x TM: 1x1  2x1  2x2  2x3  2x4  3x3  3x4  3x5  4x4
   // A set is a chain of waits, tensor-memory loads and dependent arithmetic per step, so more and smaller sets go
   // faster until their fixed cost (about 60 instructions per warp and step) takes the issue slots: 248320 x 5120 in us,
+  // both sides of each pair in the same build (before the waits were voted on per warp),
   //   M = 4: 2x2 109, 4x1 125;  M = 8: 2x4 135, 4x2 139;  M = 12: 3x4 160, 4x3 158 (int8, 163840 x 2560: 75 and 78);
   //   M = 16: 2x8 275, 4x4 194
-  // and 34816 x 5120 before (scalar arithmetic, a round of two steps per hand-off; 2x8 at M = 16) and now:
-  //   M = 4 21.6 -> 20.0, M = 6 22.4 -> 21.9, M = 8 26.8 -> 24.2, M = 9 27.1 -> 25.0, M = 12 29.4 -> 28.3, M = 16 36.9 -> 32.4
+  // and with the votes 103.6, 124.0, 148.9 and 167.5. 34816 x 5120 with scalar arithmetic, rounds of two steps per hand-off and
+  // 2x8 at M = 16, then with packed arithmetic, rounds of a step and 4x4, then with the votes:
+  //   M = 4 20.8, 19.6, 19.1     M = 6 22.2, 21.4, 20.8     M = 8 26.1, 24.1, 22.4     M = 9 26.8, 25.1, 24.0
+  //   M = 12 29.5, 27.8, 26.6    M = 15 29.8, 29.7, 28.2    M = 16 36.3, 31.5, 28.6
   static constexpr int FW = MT <= 1 ? 1 : (MT <= 8 ? 2 : (MT <= 15 ? 3 : 4));
   static constexpr int TM = (MT + FW - 1) / FW;                // tokens per fix-up warp
   static constexpr int CB = !ST ? 16 : (MT <= 2 ? 8 : (3 * TM + 3) / 4 * 4);  // accumulator columns per set
@@ -109,13 +112,16 @@ struct Geo {
   static constexpr int kPairBytes = FW * TP * 8;               // the table's bytes per group
   static constexpr int kWarps = FW <= 3 ? 24 : 28;
   static constexpr int kThreads = kWarps * 32;
-  // The block size the compiler plans for sets the register limit: 80 (24 warps) or, asked for with 1024 threads,
-  // 64. The pre-pass's CTAs of the NEXT call want to sit beside this kernel's (4096 registers each): 24 warps
-  // of 80 leave room for one, 28 of 72 (M = 16) for none. Fewer registers pay where the code fits them; 34816, 17408 and 6144
-  // columns in us, default -> 64:
-  //   M = 8  24.3 / 17.2 / 10.5 -> 24.2 / 15.7 / 9.6      M = 16 33.3 / 22.3 / 13.6 -> 32.4 / 21.9 / 12.6
-  //   M = 6  21.9 / 15.1 / 8.6  -> 23.0 / 14.7 / 8.8      M = 9  25.2 / 17.1 / 9.3  -> 26.4 / 16.8 / 9.8
-  //   M = 15 30.5 / 20.2 / 12.1 -> 31.7 / 20.3 / 12.4
+  // The block size the compiler plans for sets the register limit: 80 (24 warps), 72 (28 warps) or, asked for with 1024
+  // threads, 64. The pre-pass's CTAs of the NEXT call want to sit beside this kernel's (4096 registers each): 24 warps
+  // of 80 leave room for one, 28 of 72 (M = 16) for none. 64 is taken where it was faster, or on the narrow layers
+  // faster and on the wide one no slower by more than 2 %; neither M = 8 nor M = 16 spills at 64. 34816, 17408 and 6144 columns
+  // (in_f 5120) in us, 80 or 72 -> 64:
+  //   M = 8  22.4 / 14.3 / 10.1 -> 22.7 / 14.0 / 9.2      M = 16 30.5 / 19.1 / 12.7 -> 28.9 / 17.1 / 11.1
+  //   M = 4  19.3 / 12.6 / 9.3  -> 19.6 / 12.8 / 9.3      M = 6  21.0 / 13.3 / 8.4  -> 21.3 / 13.4 / 8.6
+  //   M = 9  24.3 / 15.0 / 9.4  -> 24.4 / 14.9 / 9.5      M = 12 26.6 / 16.5 / 11.4 -> 26.8 / 16.0 / 10.8
+  //   M = 15 28.5 / 17.0 / 10.2 -> 29.8 / 18.1 / 11.4
+  // (M = 12 would do by the same measure; it keeps 80.)
   static constexpr int kBoundThreads = MT == 8 || MT == 16 ? 1024 : kThreads;
   static constexpr int N = !ST ? 16 : ((FW * CB + 15) / 16) * 16;  // rows of the B operand the tensor core reads
   static constexpr int AD2 = N == 48 ? 2 : 4;
@@ -147,7 +153,7 @@ struct SkinnyParams {
   int y_col0;     // first column of this launch's rows inside y
   int M, N, K, G, tiles;
   int b_bytes;       // bytes of the B region (M = 1: digit rows of the groups this CTA multiplies; else the digit ring)
-  int xs_bytes;      // bytes of the (sum, 2^-p) region (M = 1)
+  int xs_bytes;      // bytes of the table of sums and scales 2^-p (M = 1: of the groups this CTA multiplies; else of all k groups)
   const uint8_t* dig;  // pre-pass output: G blocks of db_bytes = [8 chunks of 16 k][N digit rows] 16 B, then per group and token set TP sums of X and TP scales 2^-p
   int db_bytes;
   int bdepth;        // M >= 2: steps in the digit ring (a power of two)
@@ -1274,9 +1280,9 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
 }
 
 // Pre-pass of the M >= 2 calls: one warp per (k group, token) turns the token's 128 bf16 values of the
-// group into three digit rows of the B operand and its (sum, 2^-p) pair, laid out per group exactly as
-// the main kernel's digit ring wants them ([8 chunks of 16 k][3 M rows] 16 B), the pairs as one [G][M] table
-// behind all groups' rows. Small CTAs
+// group into three digit rows of the B operand, their sum and the scale 2^-p, laid out as the main kernel of this M
+// reads them: per group [8 chunks of 16 k][N rows] 16 B (N = 16, 32 or 48, a token set's rows in its own column block of `cb`;
+// db_bytes in all), and behind all groups' rows, per group and token set, `tp` sums and then `tp` scales. Small CTAs
 // (four warps, at most 32 registers) so that they fit beside a resident main-kernel CTA of the previous
 // layer and are ready to run the moment that layer completes.
 __global__ void __launch_bounds__(128, 16) k_digits(const uint16_t* __restrict__ x, uint8_t* __restrict__ dig, int M,
