@@ -45,6 +45,7 @@ const DeviceInfo* device_info();
 // pending it costs one relaxed atomic load.
 void note_weight_write(cudaStream_t st);
 bool take_weight_write(cudaStream_t st);
+bool pdl_enabled();  // programmatic dependent launch (default on; W4A16_PDL=0 turns it off)
 
 // Validates a weight container (non-null 16-byte aligned buffers, supported shape).
 int check_weights(const w4a16_weights_t* w);

@@ -37,6 +37,8 @@
 // and on the way, 34816 x 5120 at M = 4096 on one device: half groups as the unit of every hand-off 1134 (the first shape; the
 // issuing thread is the limit), whole groups 1063, two teams of dequant warps and C through shared memory 890. A warp's vote on
 // its waits took another 9 % off short prompts (34816 x 5120 at M = 77: 40.8 -> 37.1) by keeping the loops warp-uniform.
+// Programmatic dependent launch (the next launch sets up, streams and expands its first weights as this one's CTAs leave) took
+// the four layers of a block from 104.8 to 96.5 us at M = 77 (5120 -> 8192, 6144 -> 5120, MLP) and from 562.5 to 546.7 at M = 777.
 #include <cuda.h>
 #include <cstring>
 #include <mutex>
@@ -205,6 +207,9 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
   tc_fence_before();
   __syncthreads();
   cluster_sync();  // the other CTAs' barriers exist from here on
+  // The next launch's CTAs may take over each SM as this one's leave it: set-up, first weights and their expansion then run
+  // under the rest of this launch. Its activations and everything behind them wait for this launch's end (griddepcontrol.wait).
+  pdl_launch_dependents();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t tmem_a = tmem + (p.tn <= 128 ? 128 : 256);
@@ -285,6 +290,7 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
     // leader's barrier expects both CTAs' bytes.
     if (lane == 0) {
       const uint32_t xfull_l = map_to_rank(xfull_a, leader);
+      pdl_wait();  // the previous kernel produced the activations (the weights never depend on it)
       uint32_t j = 0;
       for (int tile = cluster; !dead && tile < p.tiles; tile += nclusters) {
         const PTile t = tile_of(p, tile);
@@ -684,8 +690,14 @@ int launch_prefill(PrefillParams& p, uint16_t* C, const w4a16_weights_t* w, cons
     if (cr != CUDA_SUCCESS) return fail(W4A16_ECUDA, "gemm_prefill: cuTensorMapEncodeTiled failed (%d)", int(cr));
   }
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   cluster_config(cfg, at, plan.splits, plan.clusters, plan.smem);
+  if (!take_weight_write(static_cast<cudaStream_t>(stream)) && pdl_enabled()) {
+    // (behind a weight write the launch is fully ordered: the weights are read before the wait)
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
+  }
   cfg.stream = static_cast<cudaStream_t>(stream);
   W4_CUDA(cudaLaunchKernelEx(&cfg, k_prefill, p));
   return W4A16_OK;

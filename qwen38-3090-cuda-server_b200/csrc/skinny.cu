@@ -1647,6 +1647,7 @@ int launch_skinny(SkinnyParams& p, const LayerRef* w, const uint16_t* x, int M, 
 }
 
 }  // namespace
+bool pdl_enabled() { return config().pdl != 0; }
 }  // namespace w4a16
 
 using namespace w4a16;
