@@ -38,13 +38,14 @@
 //                  (+4)        reduction, output / fused argmax; for M >= 3 a second warp per lane
 //                              quarter takes half of the tokens
 //       converters  9 warps    M = 1 only; after griddepcontrol.wait: bf16 x -> digit rows of the B operand,
-//                  (+fix-up)   once per CTA, for exactly the k groups it multiplies; issuers start on a
-//                              group as soon as its rows are in
+//                  (+fix-up)   once per CTA, for exactly the k groups it multiplies (with a fused RMSNorm
+//                              they normalise it first); issuers start on a group as soon as its rows are in
 //   * M >= 2 (verify blocks): the digit rows are made ONCE per call by a small pre-pass kernel
 //     (k_digits) into the scratch and every CTA streams the rows of the groups it multiplies through
 //     a second ring of bulk copies (they come from L2), instead of 148 identical conversions of M
 //     tokens and a cache of M x K digit bytes per CTA. 3 M <= 48 rows of B: one launch for every
 //     M <= 16. The converter warps become more fix-up warps (up to four token sets).
+#include <algorithm>
 #include <cfloat>
 #include <climits>
 #include <cstdlib>
@@ -78,6 +79,8 @@ constexpr int kTable = 64;                 // step table entries (ring)
 constexpr uint32_t kSpinLimit = 1u << 20;  // polls before a wait gives up
 constexpr uint32_t kPieceTag = 0x7A6B5C4Du;  // upper half of a published (sum, tag) word of a split tile's piece
 constexpr int kFixBar = 1;                 // named barrier of the fix-up warps
+constexpr int kConvBar = 2;                // named barrier of the converting warps
+constexpr int kConvBatch = 4;              // M = 1: k groups a warp converts with their loads in flight together
 constexpr int kTmemCols = 512;             // all of tensor memory; the next launch's CTA, resident beside this one,
                                            // gets it when this CTA exits (it cannot multiply before that anyway)
 constexpr int kAColsG = 32;                // 128 int8 along k = 32 columns of 32 bits per group
@@ -87,10 +90,9 @@ constexpr int kAColsG = 32;                // 128 int8 along k = 32 columns of 3
 // real). Ring depths are in steps: AD2 for A, DD2 for D.
 // (With N = 48, four A and two D steps are no better: when this was compared, the argmax head 163840 x 2560 at M = 16 took
 // 75.1 us with two and four, 77.5 with four and two, with int8 weights 82.1 and 85.2; now 63.0 and 72.7.)
-template <int MT, bool ST>
+template <int MT>
 struct Geo {
-  static constexpr bool kStream = ST;  // digit rows streamed from the pre-pass output instead of converted here
-  static_assert(ST || MT == 1, "only the M = 1 kernel converts activations itself");
+  static constexpr bool kStream = MT > 1;  // digit rows streamed from the pre-pass output (M = 1: converted here)
   // Token sets: the fix-up warps of one lane quarter split the tokens into FW sets of TM tokens; set F owns the
   // accumulator columns [CB F, CB F + 3 TM), so every set runs the SAME code on its own aligned column block
   // (one copy of the fix-up code per kernel: the instruction footprint of all roles has to stay cache resident).
@@ -107,7 +109,7 @@ struct Geo {
   //   M = 12 29.5, 27.8, 26.6    M = 15 29.8, 29.7, 28.2    M = 16 36.3, 31.5, 28.6
   static constexpr int FW = MT <= 1 ? 1 : (MT <= 8 ? 2 : (MT <= 15 ? 3 : 4));
   static constexpr int TM = (MT + FW - 1) / FW;                // tokens per fix-up warp
-  static constexpr int CB = !ST ? 16 : (MT <= 2 ? 8 : (3 * TM + 3) / 4 * 4);  // accumulator columns per set
+  static constexpr int CB = !kStream ? 16 : (MT <= 2 ? 8 : (3 * TM + 3) / 4 * 4);  // accumulator columns per set
   static constexpr int TP = TM == 1 ? 1 : (TM + 1) / 2 * 2;    // a set's entries per group in the (sum, 2^-p) table: TP sums, TP scales
   static constexpr int kPairBytes = FW * TP * 8;               // the table's bytes per group
   static constexpr int kWarps = FW <= 3 ? 24 : 28;
@@ -123,7 +125,7 @@ struct Geo {
   //   M = 15 28.5 / 17.0 / 10.2 -> 29.8 / 18.1 / 11.4
   // (M = 12 would do by the same measure; it keeps 80.)
   static constexpr int kBoundThreads = MT == 8 || MT == 16 ? 1024 : kThreads;
-  static constexpr int N = !ST ? 16 : ((FW * CB + 15) / 16) * 16;  // rows of the B operand the tensor core reads
+  static constexpr int N = !kStream ? 16 : ((FW * CB + 15) / 16) * 16;  // rows of the B operand the tensor core reads
   static constexpr int AD2 = N == 48 ? 2 : 4;
   static constexpr int DD2 = N == 16 ? 8 : 4;
   static constexpr int ND = 8;                           // ring of "step done" barriers
@@ -171,7 +173,7 @@ struct SkinnyParams {
   int* status;
   int npeers;  // extra destinations for y (fused all-gather / partial sums for a cross-rank reduction), 0 = none
   void* y_peers[8];  // bf16, or fp32 when y_f32
-  const uint16_t* ln_w;  // RMSNorm fused into the pre-pass: x is normalised with these bf16 weights first (null: off)
+  const uint16_t* ln_w;  // RMSNorm fused into the conversion of x: x is normalised with these bf16 weights first (null: off)
   float ln_eps;
   uint16_t* xn_out;      // optional [M][K] copy of the normalised activations
   int epilogue;      // kEpiNone, kEpiSwiglu (rows interleaved gate, up, gate, up ...: y[m][row / 2] = silu(gate) * up)
@@ -366,7 +368,7 @@ __device__ __forceinline__ float small_int_to_float(uint32_t v) {
 
 // dynamic shared memory:
 //   [weight ring: depth x 17152][B region: b_bytes][(scale,zp) ring: kSide x 128 x 4][(sum, 2^-p): xs_bytes]
-//   [step table: kTable x 8][ready counters: 256 x 4][mbarriers][tmem base, flag]
+//   [step table: kTable x 8][ready flags: 256 x 4][M = 1: sums of squares 256 x 4, mailbox][mbarriers][tmem base, flag]
 // The B operand of one k group is eight 16-k chunks, 48 M bytes apart, each holding the 3 M digit rows in
 // use as consecutive 16-byte rows (an 8-row core matrix every 128 bytes). The rows the tensor core reads
 // beyond them are the next chunk's bytes: they only produce accumulator columns nobody reads, and the
@@ -376,18 +378,18 @@ __device__ __forceinline__ float small_int_to_float(uint32_t v) {
 // the CTA's walk follows, the waiting for the other CTAs' pieces (a global-memory round trip of 1 to 2 us under
 // load, which a fix-up warp in the middle of the stream cannot make up for) goes to the helper warp of its lane
 // quarter: a mailbox entry of 32 sums and the tile number (two entries per quarter; one is used).
-template <int MT, bool ST>
-__host__ __device__ constexpr bool tile_end_helper() { return MT == 1 && !ST; }
+template <int MT>
+__host__ __device__ constexpr bool tile_end_helper() { return MT == 1; }
 constexpr int kMailStride = 40;                    // words per mailbox entry (32 sums, the tile, padding)
 constexpr int kMailWords = 2 * CW * kMailStride;
-template <int MT, bool ST>
+template <int MT>
 __host__ __device__ constexpr int bar_count(int depth, int bdepth) {
-  return 2 * depth + Geo<MT, ST>::AD2 + Geo<MT, ST>::ND + Geo<MT, ST>::DD2 + 2 + (ST ? 2 * bdepth : 0) + 1 + (tile_end_helper<MT, ST>() ? 2 * CW : 0);
+  return 2 * depth + Geo<MT>::AD2 + Geo<MT>::ND + Geo<MT>::DD2 + 2 + (Geo<MT>::kStream ? 2 * bdepth : 0) + 1 + (tile_end_helper<MT>() ? 2 * CW : 0);
 }
-template <int MT, bool ST>
+template <int MT>
 __host__ __device__ inline int total_smem(int depth, int stage_bytes, int b_bytes, int xs_bytes, int bdepth) {
   return depth * stage_bytes + b_bytes + kSide * kTileRows * 4 + xs_bytes + kTable * 8 + 256 * 4 +
-         (tile_end_helper<MT, ST>() ? kMailWords * 4 : 0) + bar_count<MT, ST>(depth, bdepth) * 8 + 16;
+         (tile_end_helper<MT>() ? (kMailWords + 256) * 4 : 0) + bar_count<MT>(depth, bdepth) * 8 + 16;
 }
 
 // One token's 128 values of one k group (this lane: k = 4 lane .. 4 lane + 3, `rv`) -> three int8 digit
@@ -434,12 +436,39 @@ __device__ __forceinline__ void convert_group(uint2 rv, uint8_t* bslot, int lbo,
   }
 }
 
+// ---- RMSNorm in front of a layer: xn = bf16(x * inv * (1 + w)), inv = rsqrt(mean(x^2) + eps) over the token's row ----
+// One group's sum of squares (this lane: four of its 128 values), on every lane.
+__device__ __forceinline__ float group_sumsq(uint2 q) {
+  const float a0 = __uint_as_float(q.x << 16), a1 = __uint_as_float(q.x & 0xFFFF0000u);
+  const float a2 = __uint_as_float(q.y << 16), a3 = __uint_as_float(q.y & 0xFFFF0000u);
+  float ss = (a0 * a0 + a1 * a1) + (a2 * a2 + a3 * a3);
+#pragma unroll
+  for (int off = 16; off; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+  return ss;
+}
+// The row's, from its groups': always added up in this order, so that a token's normalised values do not depend on
+// which warps or CTAs summed the groups.
+__device__ __forceinline__ float row_sumsq(const float* sumsq, int G, int lane) {
+  float ss = 0.f;
+  for (int g = lane; g < G; g += 32) ss += sumsq[g];
+#pragma unroll
+  for (int off = 16; off; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+  return ss;
+}
+__device__ __forceinline__ uint2 normalise(uint2 q, uint2 w, float inv) {
+  auto nrm = [&](uint32_t xb, uint32_t wb) {  // both bf16 bit patterns in the high half
+    return static_cast<uint32_t>(float_to_bf16_bits(__uint_as_float(xb) * inv * (1.0f + __uint_as_float(wb))));
+  };
+  return make_uint2(nrm(q.x << 16, w.x << 16) | (nrm(q.x & 0xFFFF0000u, w.x & 0xFFFF0000u) << 16),
+                    nrm(q.y << 16, w.y << 16) | (nrm(q.y & 0xFFFF0000u, w.y & 0xFFFF0000u) << 16));
+}
+
 // COMM: the cross-rank flag code (wait before x is read, signal after the last store, the pair exchange of the
 // vocab-sharded head) is compiled into separate instances, so that single-GPU launches run exactly the code
 // they ran without it.
-template <int MT, int WB, bool ST, bool COMM>
-__global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const SkinnyParams p) {
-  using GE = Geo<MT, ST>;
+template <int MT, int WB, bool COMM>
+__global__ void __launch_bounds__(Geo<MT>::kBoundThreads, 1) k_skinny(const SkinnyParams p) {
+  using GE = Geo<MT>;
   constexpr int kBlock = Fmt<WB>::kBlock, kStageBytes = Fmt<WB>::kStage;
   constexpr int N = GE::N, AD2 = GE::AD2, DD2 = GE::DD2, ND = GE::ND;
   constexpr bool kStream = GE::kStream;
@@ -452,12 +481,13 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
   uint8_t* side = bq + p.b_bytes;
   uint8_t* xsinv = side + kSide * kTileRows * 4;
   uint2* table = reinterpret_cast<uint2*>(xsinv + p.xs_bytes);
-  uint32_t* ready = reinterpret_cast<uint32_t*>(table + kTable);  // [slot]: tokens whose digit rows are written
+  uint32_t* ready = reinterpret_cast<uint32_t*>(table + kTable);  // M = 1, [slot]: the group's digit rows are written
   float* mail = reinterpret_cast<float*>(ready + 256);  // [2 entries][lane quarter][kMailStride] (helper instances only)
-  constexpr bool kHelper = tile_end_helper<MT, ST>();
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ready + 256 + (kHelper ? kMailWords : 0));
+  constexpr bool kHelper = tile_end_helper<MT>();
+  float* sumsq = mail + kMailWords;                       // M = 1 with the RMSNorm: [k group] sum of squares
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ready + 256 + (kHelper ? kMailWords + 256 : 0));
   const int BD = p.bdepth, BS = p.bshift;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + bar_count<MT, ST>(DS, BD));
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + bar_count<MT>(DS, BD));
   int* sflag = reinterpret_cast<int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, lane = tid & 31;
@@ -473,7 +503,7 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
   // bytes between the digit rows of consecutive groups (cache slots for M = 1, ring slots otherwise), and
   // between the 16-k chunks of one group
   const int b_slot = kStream ? p.db_bytes : 384 * M, b_lbo = kStream ? 16 * N : 48 * M;
-  const bool tail_last = !(tile_end_helper<MT, ST>() && !p.argmax);  // see SegIter
+  const bool tail_last = !(tile_end_helper<MT>() && !p.argmax);  // see SegIter
   int T;       // steps of this CTA
   int nsplit;  // 1 if the helper warps get a segment of this CTA: the piece at the end of its range (the first
                // piece of that tile, so this CTA adds the tile up) with whole tiles still to come after it
@@ -506,7 +536,7 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
   {
     // barrier i of the block [wfull | wempty | afull | done | dempty | bready | tmemrdy]: arrival counts
     // (+ [bfull | bempty] for M >= 2)
-    const int nb = bar_count<MT, ST>(DS, BD), nb0 = 2 * DS + AD2 + ND + DD2 + 2;
+    const int nb = bar_count<MT>(DS, BD), nb0 = 2 * DS + AD2 + ND + DD2 + 2;
     const uint32_t nfix = CW * ((M + GE::TM - 1) / GE::TM);                // active fix-up warps
     if (tid < nb) {
       uint32_t cnt = 1;                                                    // wfull, done, tmemrdy, bfull
@@ -551,39 +581,63 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
         atomicExch(p.status, W4A16_ETIMEOUT);
       }
     }
+    // Item i is k group (g_first + i) % G, the order in which the CTA walks its groups, so the first steps can start after
+    // the first batch; with the fused RMSNorm it is k group i (every CTA sums the whole row).
     const int ti = warp < CW ? warp : (warp == 14 ? CW : warp - kWConv0 + CW + 1);
     const int cnt = (u1 - u0 < G) ? u1 - u0 : G;
-    const int total = cnt * M;  // (group, token) items; item i belongs to warp i % kTeam
-    constexpr int kBatch = 4;
-    for (int i0 = ti; i0 < total; i0 += kBatch * kTeam) {
-      uint2 rv[kBatch];
+    const bool norm = p.ln_w != nullptr;
+    const int total = norm ? G : cnt;  // items; item i belongs to warp i % kTeam
+    const uint2* x2 = reinterpret_cast<const uint2*>(p.x) + lane;
+    auto group_of = [&](int i) { return norm ? i : (g_first + i < G ? g_first + i : g_first + i - G); };
+    uint2 rv[kConvBatch];
+    auto load = [&](int i0) {
 #pragma unroll
-      for (int j = 0; j < kBatch; ++j) {
+      for (int j = 0; j < kConvBatch; ++j)
+        if (i0 + j * kTeam < total) rv[j] = __ldcg(x2 + group_of(i0 + j * kTeam) * (kGroup / 4));
+    };
+    load(ti);
+    float inv = 0.f;
+    if (norm) {
+      // RMSNorm fused in (replaces the separate kernel in front of the linear layer): every CTA sums the row, 10 KB of
+      // loads that its conversion makes anyway. As a pre-pass kernel whose warps each walked the row, a block of
+      // 34816 x 5120 and 5120 x 17408 took 35.9 us; now 31.7.
+      for (int i0 = ti; i0 < total; i0 += kConvBatch * kTeam) {
+        if (i0 != ti) load(i0);
+#pragma unroll
+        for (int j = 0; j < kConvBatch; ++j)
+          if (i0 + j * kTeam < total) {
+            const float ss = group_sumsq(rv[j]);
+            if (lane == 0) sumsq[i0 + j * kTeam] = ss;
+          }
+      }
+      named_bar_sync(kConvBar, kTeam * 32);
+      inv = rsqrtf(row_sumsq(sumsq, G, lane) / static_cast<float>(p.K) + p.ln_eps);
+      if (total > kConvBatch * kTeam) load(ti);
+    }
+    for (int i0 = ti; i0 < total; i0 += kConvBatch * kTeam) {
+      if (i0 != ti) load(i0);
+#pragma unroll
+      for (int j = 0; j < kConvBatch; ++j) {
         const int i = i0 + j * kTeam;
         if (i < total) {
-          const int gj = i, m = 0;
-          int g = g_first + gj;
-          if (g >= G) g -= G;
-          rv[j] = __ldcg(reinterpret_cast<const uint2*>(p.x + static_cast<size_t>(m) * p.K + g * kGroup) + lane);
+          const int g = group_of(i), slot = norm ? cache_slot(g) : i;
+          if (norm) {
+            rv[j] = normalise(rv[j], __ldg(reinterpret_cast<const uint2*>(p.ln_w + g * kGroup) + lane), inv);
+            if (p.xn_out && g % gridDim.x == blockIdx.x) reinterpret_cast<uint2*>(p.xn_out + g * kGroup)[lane] = rv[j];
+          }
+          if (slot < cnt)
+            convert_group(rv[j], bq + slot * b_slot, b_lbo, 0, reinterpret_cast<float*>(xsinv) + 2 * slot, 1, lane);
         }
       }
-#pragma unroll
-      for (int j = 0; j < kBatch; ++j) {
-        const int i = i0 + j * kTeam;
-        if (i < total) {
-          const int gj = i, m = 0;
-          convert_group(rv[j], bq + gj * b_slot, b_lbo, m, reinterpret_cast<float*>(xsinv) + 2 * (gj * MT + m), 1, lane);
-          // publish the item: B was written through the generic proxy, the tensor core reads it through the
-          // async one; the slot counts as ready once all M tokens are in. Slots are numbered in the order the
-          // CTA walks its groups, and items are taken in slot order, so the first steps can start after the
-          // first round.
-          fence_proxy_async();
-          __syncwarp();
-          if (lane == 0) {
-            __threadfence_block();
-            atomicAdd(ready + gj, 1u);
-          }
-        }
+      // publish the batch, one fence for all of it: B was written through the generic proxy, the tensor core reads it
+      // through the async one
+      fence_proxy_async();
+      __syncwarp();
+      const int i = i0 + lane * kTeam;
+      if (lane < kConvBatch && i < total) {
+        const int slot = norm ? cache_slot(i) : i;
+        __threadfence_block();
+        if (slot < cnt) *reinterpret_cast<volatile uint32_t*>(ready + slot) = 1u;
       }
     }
     __syncwarp();
@@ -921,7 +975,7 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
     // 3 i .. 3 i + 2 of it
     constexpr int NLD = kStream ? CB : 4;
     const uint32_t* side_r = reinterpret_cast<const uint32_t*>(side) + r;
-    const float2* xs_tab = reinterpret_cast<const float2*>(xsinv);  // M = 1: (sum, 2^-p) per cache slot or (pre-pass) per k group
+    const float2* xs_tab = reinterpret_cast<const float2*>(xsinv);  // M = 1: (sum, 2^-p) per cache slot
     if constexpr (kStream) {
       // the pair table of the call arrives once, by bulk copy
       if (!warp_agrees(wait_h(bready_a, 0, p.hint, kSpinLimit))) {
@@ -970,7 +1024,7 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
       const int ng0 = static_cast<int>((e0.x >> 16) & 1u) + 1;
       const int rg = two ? ng0 + static_cast<int>((e1.x >> 16) & 1u) + 1 : ng0;  // groups of the round (ng0 == 2 if two)
       // group k of the round: step t + (k >> 1), position k & 1
-      if constexpr (!kStream || MT == 1) {
+      if constexpr (!kStream) {
 #pragma unroll
       for (int k0 = 0; k0 < 4; k0 += GB) {
         if (k0 < rg) {
@@ -1004,8 +1058,8 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
               const float s = __uint_as_float(sz[j] & 0xFFFF0000u);
               const float z = __uint_as_float(0x4B000000u | (sz[j] & 0xFFu)) - 8388608.0f;
               {
-                // (sum of X, 2^-p): by cache slot, or (pre-pass) by k group
-                const float2 xv = xs_tab[kStream ? ((ew >> 19) & 0xFFu) + (k & 1) : slot];
+                // (sum of X, 2^-p) by cache slot
+                const float2 xv = xs_tab[slot];
                 const float d0 = small_int_to_float(dv[j][0]);
                 const float d1 = small_int_to_float(dv[j][1]);
                 const float d2 = small_int_to_float(dv[j][2]);
@@ -1284,7 +1338,9 @@ __global__ void __launch_bounds__(Geo<MT, ST>::kBoundThreads, 1) k_skinny(const 
 // reads them: per group [8 chunks of 16 k][N rows] 16 B (N = 16, 32 or 48, a token set's rows in its own column block of `cb`;
 // db_bytes in all), and behind all groups' rows, per group and token set, `tp` sums and then `tp` scales. Small CTAs
 // (four warps, at most 32 registers) so that they fit beside a resident main-kernel CTA of the previous
-// layer and are ready to run the moment that layer completes.
+// layer and are ready to run the moment that layer completes. (A CTA per SM whose warps take several items, four loads in flight:
+// the passes at M = 9 and 16 were 1 and 3 % slower.) With the RMSNorm a CTA is four groups of one token.
+template <bool NORM>
 __global__ void __launch_bounds__(128, 16) k_digits(const uint16_t* __restrict__ x, uint8_t* __restrict__ dig, int M,
                                                     int K, int G, int db_bytes, int tm, int cb, int tp, int sets,
                                                     const unsigned* comm_local, int comm_n, int* status,
@@ -1298,31 +1354,42 @@ __global__ void __launch_bounds__(128, 16) k_digits(const uint16_t* __restrict__
       atomicExch(status, W4A16_ETIMEOUT);
     __syncthreads();
   }
-  const int item = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (item >= G * M) return;
-  const int g = item / M, m = item - g * M;
-  uint2 rv = __ldcg(reinterpret_cast<const uint2*>(x + static_cast<size_t>(m) * K + g * kGroup) + lane);
-  if (ln_w) {
-    // RMSNorm fused in (replaces the separate kernel in front of the linear layer): the token's
-    // inv = rsqrt(mean(x^2) + eps) over the whole row - every warp of the token recomputes it from L2 - then
-    // xn = bf16(x * inv * (1 + w)), rounded to bf16 as the unfused path stores it, and the digits are taken of xn.
-    const uint2* row = reinterpret_cast<const uint2*>(x + static_cast<size_t>(m) * K);
-    float ss = 0.f;
-    for (int j = lane; j < K / 4; j += 32) {
-      const uint2 q = __ldcg(row + j);
-      const float a0 = __uint_as_float(q.x << 16), a1 = __uint_as_float(q.x & 0xFFFF0000u);
-      const float a2 = __uint_as_float(q.y << 16), a3 = __uint_as_float(q.y & 0xFFFF0000u);
-      ss += (a0 * a0 + a1 * a1) + (a2 * a2 + a3 * a3);
-    }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int g, m;
+  if constexpr (NORM) {
+    const int per = (G + 3) >> 2;
+    m = blockIdx.x / per;
+    g = 4 * (blockIdx.x - m * per) + warp;
+  } else {
+    const int item = blockIdx.x * 4 + warp;
+    if (item >= G * M) return;
+    g = item / M;
+    m = item - g * M;
+  }
+  const uint2* row = reinterpret_cast<const uint2*>(x + static_cast<size_t>(m) * K) + lane;
+  uint2 rv = !NORM || g < G ? __ldcg(row + g * (kGroup / 4)) : make_uint2(0u, 0u);
+  if constexpr (NORM) {
+    // RMSNorm fused in (replaces the separate kernel in front of the linear layer), rounded to bf16 as the unfused path
+    // stores it; the digits are taken of xn. Every CTA sums the token's whole row, a quarter of it per warp, six loads in
+    // flight; a warp alone, one load after the other, held up the layer behind it.
+    constexpr int kBatch = 6;
+    __shared__ float sumsq[256];
+    for (int g0 = warp; g0 < G; g0 += 4 * kBatch) {
+      uint2 q[kBatch];
 #pragma unroll
-    for (int off = 16; off; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-    const float inv = rsqrtf(ss / static_cast<float>(K) + ln_eps);
-    const uint2 wq = __ldg(reinterpret_cast<const uint2*>(ln_w + g * kGroup) + lane);
-    auto nrm = [&](uint32_t xb, uint32_t wb) {  // both bf16 bit patterns in the high half
-      return static_cast<uint32_t>(float_to_bf16_bits(__uint_as_float(xb) * inv * (1.0f + __uint_as_float(wb))));
-    };
-    rv.x = nrm(rv.x << 16, wq.x << 16) | (nrm(rv.x & 0xFFFF0000u, wq.x & 0xFFFF0000u) << 16);
-    rv.y = nrm(rv.y << 16, wq.y << 16) | (nrm(rv.y & 0xFFFF0000u, wq.y & 0xFFFF0000u) << 16);
+      for (int j = 0; j < kBatch; ++j)
+        if (g0 + 4 * j < G) q[j] = __ldcg(row + (g0 + 4 * j) * (kGroup / 4));
+#pragma unroll
+      for (int j = 0; j < kBatch; ++j)
+        if (g0 + 4 * j < G) {
+          const float ss = group_sumsq(q[j]);
+          if (lane == 0) sumsq[g0 + 4 * j] = ss;
+        }
+    }
+    __syncthreads();
+    if (g >= G) return;
+    const float inv = rsqrtf(row_sumsq(sumsq, G, lane) / static_cast<float>(K) + ln_eps);
+    rv = normalise(rv, __ldg(reinterpret_cast<const uint2*>(ln_w + g * kGroup) + lane), inv);
     if (xn_out) reinterpret_cast<uint2*>(xn_out + static_cast<size_t>(m) * K + g * kGroup)[lane] = rv;
   }
   float* pairs = reinterpret_cast<float*>(dig + static_cast<size_t>(G) * db_bytes);
@@ -1374,13 +1441,11 @@ struct Config {
   int depth;     // weight ring stages (two blocks, 17152 B, each); even
   int pdl;
   int hint;      // suspend-time hint of the in-kernel mbarrier waits, ns
-  int gemv_prepass;  // M = 1 through the pre-pass + digit ring as well (experiment; default off)
 };
 
 const Config& config() {
   static Config c = [] {
-    Config k{6, 1, 2000, 0};
-    if (const char* e = getenv("W4A16_GEMV_PREPASS")) k.gemv_prepass = atoi(e) != 0;
+    Config k{6, 1, 2000};
     if (const char* e = getenv("W4A16_DEPTH")) k.depth = atoi(e);
     if (const char* e = getenv("W4A16_PDL")) k.pdl = atoi(e) != 0;
     if (const char* e = getenv("W4A16_HINT")) k.hint = atoi(e);
@@ -1419,13 +1484,13 @@ int cache_groups_for(int tiles, int G, int grid) {
   return per_cta < G ? per_cta : G;
 }
 
-template <int MT, int WB, bool ST, bool COMM>
+template <int MT, int WB, bool COMM>
 int launch_kernel(const SkinnyParams& p, int grid, cudaStream_t st, int smem);
 
-template <int MT, int WB, bool ST, bool COMM>
+template <int MT, int WB, bool COMM>
 int launch_cfg(SkinnyParams& p, int grid, cudaStream_t st, int smem_optin) {
   constexpr int kStageBytes = Fmt<WB>::kStage;
-  constexpr bool kStream = ST;
+  constexpr bool kStream = Geo<MT>::kStream;
   const int groups = cache_groups_for(p.tiles, p.G, grid);
   const int limit = smem_optin;
   if constexpr (kStream) {
@@ -1439,8 +1504,8 @@ int launch_cfg(SkinnyParams& p, int grid, cudaStream_t st, int smem_optin) {
       p.bdepth = c[1];
       p.bshift = c[1] == 8 ? 3 : (c[1] == 4 ? 2 : 1);
       p.b_bytes = p.bdepth * kStepGroups * p.db_bytes;
-      p.xs_bytes = (p.G * Geo<MT, ST>::kPairBytes + 15) & ~15;
-      smem = total_smem<MT, ST>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, p.bdepth);
+      p.xs_bytes = (p.G * Geo<MT>::kPairBytes + 15) & ~15;
+      smem = total_smem<MT>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, p.bdepth);
       if (smem <= limit) {
         found = true;
         break;
@@ -1449,7 +1514,7 @@ int launch_cfg(SkinnyParams& p, int grid, cudaStream_t st, int smem_optin) {
     if (!found)
       return fail(W4A16_EINVAL, "decode kernel needs %d bytes of shared memory for M = %d; the device offers %d", smem,
                   p.M, smem_optin);
-    return launch_kernel<MT, WB, ST, COMM>(p, grid, st, smem);
+    return launch_kernel<MT, WB, COMM>(p, grid, st, smem);
   }
   p.b_bytes = groups * 384 * p.M + 256;
   p.xs_bytes = groups * MT * 8;
@@ -1460,29 +1525,29 @@ int launch_cfg(SkinnyParams& p, int grid, cudaStream_t st, int smem_optin) {
   // uses would belong to different warps, and a warp that runs ahead could take "the other warp's copy has
   // not landed yet" for "my copy has landed".
   p.depth = config().depth;
-  int smem = total_smem<MT, ST>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
+  int smem = total_smem<MT>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
   while (smem > limit && p.depth > 2) {
     p.depth -= 2;
-    smem = total_smem<MT, ST>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
+    smem = total_smem<MT>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
   }
   if (smem > smem_optin)
     return fail(W4A16_EINVAL, "decode kernel needs %d bytes of shared memory for in_f = %d, M = %d; the device offers %d",
                 smem, p.K, p.M, smem_optin);
-  return launch_kernel<MT, WB, ST, COMM>(p, grid, st, smem);
+  return launch_kernel<MT, WB, COMM>(p, grid, st, smem);
 }
 
-template <int MT, int WB, bool ST, bool COMM>
+template <int MT, int WB, bool COMM>
 int launch_kernel(const SkinnyParams& p, int grid, cudaStream_t st, int smem) {
   static int attr_set[64] = {};
   int dev = 0;
   W4_CUDA(cudaGetDevice(&dev));
   if (attr_set[dev & 63] < smem) {
-    W4_CUDA(cudaFuncSetAttribute(k_skinny<MT, WB, ST, COMM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    W4_CUDA(cudaFuncSetAttribute(k_skinny<MT, WB, COMM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr_set[dev & 63] = smem;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(Geo<MT, ST>::kThreads);
+  cfg.blockDim = dim3(Geo<MT>::kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
@@ -1490,14 +1555,14 @@ int launch_kernel(const SkinnyParams& p, int grid, cudaStream_t st, int smem) {
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = (config().pdl && !p.ordered) ? 1 : 0;
-  W4_CUDA(cudaLaunchKernelEx(&cfg, k_skinny<MT, WB, ST, COMM>, p));
+  W4_CUDA(cudaLaunchKernelEx(&cfg, k_skinny<MT, WB, COMM>, p));
   return W4A16_OK;
 }
 
 // M = 1: the digit rows of `groups` k groups (384 B + one pair per group) must fit beside a two-stage
 // weight ring.
 bool gemv_cache_fits(int groups, int stage_bytes, int smem_optin) {
-  const int fixed = 2 * stage_bytes + kSide * kTileRows * 4 + kTable * 8 + 256 * 4 + kMailWords * 4 + 64 * 8 + 16 + 256;
+  const int fixed = 2 * stage_bytes + kSide * kTileRows * 4 + kTable * 8 + 256 * 4 + (kMailWords + 256) * 4 + 64 * 8 + 16 + 256;
   return groups * (384 + 8) <= smem_optin - fixed;
 }
 
@@ -1514,25 +1579,24 @@ struct DigitGeometry {
 // (N = 48 rows; the table of three sets of five tokens, padded to six: 144 bytes, more than sixteen tokens' 128).
 template <int MT>
 constexpr int digit_bytes() {
-  return 128 * Geo<MT, true>::N;
+  return 128 * Geo<MT>::N;
 }
 template <int... MT>
 constexpr int widest_group() {
   int digits = 0, pairs = 0;
   ((digits = digit_bytes<MT>() > digits ? digit_bytes<MT>() : digits), ...);
-  ((pairs = Geo<MT, true>::kPairBytes > pairs ? Geo<MT, true>::kPairBytes : pairs), ...);
+  ((pairs = Geo<MT>::kPairBytes > pairs ? Geo<MT>::kPairBytes : pairs), ...);
   return digits + pairs;
 }
-constexpr int kPrepassGroupBytes = widest_group<1, 2, 4, 6, 8, 9, 12, 15, 16>();
+constexpr int kPrepassGroupBytes = widest_group<2, 4, 6, 8, 9, 12, 15, 16>();
 template <int MT>
 DigitGeometry geometry_of() {
-  using GE = Geo<MT, true>;
+  using GE = Geo<MT>;
   static_assert(digit_bytes<MT>() + GE::kPairBytes <= kPrepassGroupBytes, "the scratch must hold every instance's pre-pass output");
   return {GE::TM, GE::CB, GE::TP, GE::FW, GE::N};
 }
 DigitGeometry digit_geometry(int M) {
   switch (instance_for(M)) {
-    case 1: return geometry_of<1>();
     case 2: return geometry_of<2>();
     case 4: return geometry_of<4>();
     case 6: return geometry_of<6>();
@@ -1564,17 +1628,16 @@ int layer_of(LayerRef& L, const w4a16_w8_weights_t* w) {
 
 template <int WB, bool COMM>
 int launch_batch_c(SkinnyParams& q, int grid, cudaStream_t st, int smem_optin) {
-  switch (instance_for(q.M)) {
-    case 1: return q.dig ? launch_cfg<1, WB, true, COMM>(q, grid, st, smem_optin)
-                         : launch_cfg<1, WB, false, COMM>(q, grid, st, smem_optin);
-    case 2: return launch_cfg<2, WB, true, COMM>(q, grid, st, smem_optin);    // token sets 1, 1
-    case 4: return launch_cfg<4, WB, true, COMM>(q, grid, st, smem_optin);    // 2, M - 2
-    case 6: return launch_cfg<6, WB, true, COMM>(q, grid, st, smem_optin);    // 3, M - 3
-    case 8: return launch_cfg<8, WB, true, COMM>(q, grid, st, smem_optin);    // 4, M - 4
-    case 9: return launch_cfg<9, WB, true, COMM>(q, grid, st, smem_optin);    // 3, 3, 3
-    case 12: return launch_cfg<12, WB, true, COMM>(q, grid, st, smem_optin);  // 4, 4, M - 8
-    case 15: return launch_cfg<15, WB, true, COMM>(q, grid, st, smem_optin);  // 5, 5, M - 10
-    default: return launch_cfg<16, WB, true, COMM>(q, grid, st, smem_optin);  // 4, 4, 4, 4
+  switch (instance_for(q.dig ? std::max(q.M, 2) : q.M)) {
+    case 1: return launch_cfg<1, WB, COMM>(q, grid, st, smem_optin);
+    case 2: return launch_cfg<2, WB, COMM>(q, grid, st, smem_optin);    // token sets 1, 1
+    case 4: return launch_cfg<4, WB, COMM>(q, grid, st, smem_optin);    // 2, M - 2
+    case 6: return launch_cfg<6, WB, COMM>(q, grid, st, smem_optin);    // 3, M - 3
+    case 8: return launch_cfg<8, WB, COMM>(q, grid, st, smem_optin);    // 4, M - 4
+    case 9: return launch_cfg<9, WB, COMM>(q, grid, st, smem_optin);    // 3, 3, 3
+    case 12: return launch_cfg<12, WB, COMM>(q, grid, st, smem_optin);  // 4, 4, M - 8
+    case 15: return launch_cfg<15, WB, COMM>(q, grid, st, smem_optin);  // 5, 5, M - 10
+    default: return launch_cfg<16, WB, COMM>(q, grid, st, smem_optin);  // 4, 4, 4, 4
   }
 }
 template <int WB>
@@ -1611,20 +1674,24 @@ int launch_skinny(SkinnyParams& p, const LayerRef* w, const uint16_t* x, int M, 
   if (int rc = w4a16_scratch_check(s, w->out_f, M)) return rc;
   p.M = M;
   p.x = x;
-  const bool prepass = M >= 2 || p.ln_w != nullptr || (config().gemv_prepass && s->max_m >= 2 && p.G <= s->max_groups);
+  if ((M >= 2 || p.ln_w != nullptr) && (M > (s->max_m >= 2 ? s->max_m : 0) || p.G > s->max_groups))
+    return fail(W4A16_ESCRATCH, "scratch: sized for max_m = %d and in_f <= %d, got M = %d, in_f = %d", s->max_m,
+                s->max_groups * kGroup, M, w->in_f);
+  // M = 1 converts (and normalises) x inside the decode kernel, while other CTAs may already be storing y. A normalised call whose
+  // y overlaps x (the residual added in place) takes the pre-pass, which has read all of x by then, and the two-token instance.
+  const char *xb = reinterpret_cast<const char*>(x), *yb = static_cast<const char*>(p.y);
+  const bool in_place = p.ln_w != nullptr && yb != nullptr && yb < xb + 2LL * M * p.K && xb < yb + 2LL * M * p.ldy;
+  const bool prepass = M >= 2 || in_place;
   if (!prepass) {
     if (!gemv_cache_fits(cache_groups_for(p.tiles, p.G, grid), w->wbits == 4 ? Fmt<4>::kStage : Fmt<8>::kStage,
                          di->smem_optin))
       return fail(W4A16_EINVAL, "in_f = %d is too wide for the decode kernel's activation cache", w->in_f);
   } else {
     // the pre-pass: digit rows of all M tokens, once per call, into the scratch (behind the argmax pairs)
-    if (M > (s->max_m >= 2 ? s->max_m : 0) || p.G > s->max_groups)
-      return fail(W4A16_ESCRATCH, "scratch: sized for max_m = %d and in_f <= %d, got M = %d, in_f = %d", s->max_m,
-                  s->max_groups * kGroup, M, w->in_f);
     uint8_t* dig = reinterpret_cast<uint8_t*>(s->xf) + pair_bytes(s->max_splits);
     p.dig = dig;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((p.G * M + 3) / 4);
+    cfg.gridDim = dim3(p.ln_w ? M * ((p.G + 3) / 4) : (p.G * M + 3) / 4);
     cfg.blockDim = dim3(128);
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -1635,10 +1702,10 @@ int launch_skinny(SkinnyParams& p, const LayerRef* w, const uint16_t* x, int M, 
     // with this one as usual
     cfg.numAttrs = (config().pdl && !p.ordered) ? 1 : 0;
     p.ordered = 0;
-    const DigitGeometry dg = digit_geometry(M);
+    const DigitGeometry dg = digit_geometry(std::max(M, 2));
     p.db_bytes = 128 * dg.nrows;
     const unsigned* wait_block = p.comm_wait ? p.comm_local : nullptr;
-    W4_CUDA(cudaLaunchKernelEx(&cfg, k_digits, x, dig, M, p.K, p.G, p.db_bytes, dg.tm, dg.cb, dg.tp, dg.sets, wait_block, p.comm_n, p.status,
+    W4_CUDA(cudaLaunchKernelEx(&cfg, p.ln_w ? k_digits<true> : k_digits<false>, x, dig, M, p.K, p.G, p.db_bytes, dg.tm, dg.cb, dg.tp, dg.sets, wait_block, p.comm_n, p.status,
                                p.ln_w, p.ln_eps, p.xn_out));
   }
   if (int rc = w->wbits == 4 ? launch_batch<4>(p, grid, st, di->smem_optin) : launch_batch<8>(p, grid, st, di->smem_optin))
