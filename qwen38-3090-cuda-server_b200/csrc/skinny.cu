@@ -115,17 +115,25 @@ struct Geo {
   static constexpr int kPairBytes = FW * TP * 8;               // the table's bytes per group
   static constexpr int kWarps = FW <= 3 ? 24 : 28;
   static constexpr int kThreads = kWarps * 32;
-  // The block size the compiler plans for sets the register limit: 80 (24 warps), 72 (28 warps) or, asked for with 1024
-  // threads, 64. The pre-pass's CTAs of the NEXT call want to sit beside this kernel's (4096 registers each): 24 warps
-  // of 80 leave room for one, 28 of 72 (M = 16) for none. 64 is taken where it was faster, or on the narrow layers
-  // faster and on the wide one no slower by more than 2 %; neither M = 8 nor M = 16 spills at 64. 34816, 17408 and 6144 columns
-  // (in_f 5120) in us, 80 or 72 -> 64:
-  //   M = 8  22.4 / 14.3 / 10.1 -> 22.7 / 14.0 / 9.2      M = 16 30.5 / 19.1 / 12.7 -> 28.9 / 17.1 / 11.1
-  //   M = 4  19.3 / 12.6 / 9.3  -> 19.6 / 12.8 / 9.3      M = 6  21.0 / 13.3 / 8.4  -> 21.3 / 13.4 / 8.6
-  //   M = 9  24.3 / 15.0 / 9.4  -> 24.4 / 14.9 / 9.5      M = 12 26.6 / 16.5 / 11.4 -> 26.8 / 16.0 / 10.8
-  //   M = 15 28.5 / 17.0 / 10.2 -> 29.8 / 18.1 / 11.4
-  // (M = 12 would do by the same measure; it keeps 80.)
-  static constexpr int kBoundThreads = MT == 8 || MT == 16 ? 1024 : kThreads;
+  // The block size the compiler plans for sets the register limit: 80 (24 warps), 72 (asked for with 896 threads) or 64 (with
+  // 1024). The pre-pass's CTAs of the NEXT call want to sit beside this kernel's (4096 registers each): 24 warps
+  // of 80 leave room for one, of 72 for two, of 64 for four. Taken is what was fastest over the layers (M = 15 spills 36 bytes at
+  // 64 and gains all the same). 34816 x 5120 / 5120 x 17408 / 16384 x 5120 / 5120 x 6144 in us:
+  //           80 registers                72                          64
+  //   M = 4   19.1 / 14.2 / 11.8 /  9.7   19.3 / 14.4 / 11.9 /  9.6   19.5 / 14.5 / 12.0 /  9.5
+  //   M = 6   20.5 / 14.2 / 12.2 /  8.2   20.7 / 13.6 / 12.3 /  8.4   20.6 / 13.6 / 12.3 /  8.3
+  //   M = 9   23.3 / 16.2 / 13.7 /  9.3   23.6 / 15.3 / 13.9 /  9.7   24.2 / 15.7 / 14.3 /  9.8
+  //   M = 12  25.6 / 18.3 / 15.3 / 11.5   26.6 / 18.2 / 15.8 / 11.7   26.3 / 17.2 / 15.1 / 11.1
+  //   M = 15  28.2 / 19.6 / 16.5 / 12.2   28.0 / 19.1 / 16.2 / 11.6   27.5 / 17.1 / 15.5 / 10.3
+  // and earlier M = 8 80 -> 64 22.4 / 14.3 / - / 10.1 -> 22.7 / 14.0 / - / 9.2, M = 16 72 -> 64 30.5 / 19.1 / - / 12.7 -> 28.9 / 17.1 / - / 11.1
+  // (those with 17408 x 5120 in the second place).
+  static constexpr int kBoundThreads = MT == 8 || MT == 12 || MT >= 15 ? 1024 : (MT == 6 ? 896 : kThreads);
+  // int32 -> fp32 of the sums by the conversion instruction (exact below 2^24, the same floats) instead of an integer add of a magic
+  // constant and a packed subtraction: fewer instructions, on a slower pipe. 34816 x 5120 / 5120 x 17408 / 16384 x 5120 / 5120 x 6144 in us, magic -> conversion:
+  //   M = 6 (72 registers) 20.7 / 13.6 / 12.3 / 8.4 -> 20.1 / 13.2 / 12.0 / 8.2    M = 8 22.2 / 14.6 / 13.1 / 9.4 -> 21.2 / 14.1 / 12.6 / 9.1
+  //   M = 9  23.3 / 16.2 / 13.7 / 9.3 -> 24.2 / 17.1 / 14.6 / 10.1                 M = 12 25.6 / 18.3 / 15.3 / 11.5 -> 26.0 / 19.4 / 15.8 / 12.1
+  //   M = 16 28.5 / 19.3 / 16.0 / 11.3 -> 27.5 / 19.3 / 16.0 / 11.5                M = 4 the same
+  static constexpr bool kConvert = MT == 6 || MT == 8 || MT == 16;
   static constexpr int N = !kStream ? 16 : ((FW * CB + 15) / 16) * 16;  // rows of the B operand the tensor core reads
   static constexpr int AD2 = N == 48 ? 2 : 4;
   static constexpr int DD2 = N == 16 ? 8 : 4;
@@ -1091,9 +1099,13 @@ __global__ void __launch_bounds__(Geo<MT>::kBoundThreads, 1) k_skinny(const Skin
           for (int i = 0; i + 1 < TM; i += 2) {
             const unsigned long long sum2 = *reinterpret_cast<const unsigned long long*>(xs_g + i);
             const unsigned long long inv2 = *reinterpret_cast<const unsigned long long*>(xs_g + GE::TP + i);
-            const unsigned long long d0 = add_f32x2(magic_pair(d[3 * i], d[3 * i + 3]), off2);
-            const unsigned long long d1 = add_f32x2(magic_pair(d[3 * i + 1], d[3 * i + 4]), off2);
-            const unsigned long long d2 = add_f32x2(magic_pair(d[3 * i + 2], d[3 * i + 5]), off2);
+            auto to_float = [&](uint32_t lo, uint32_t hi) {
+              return GE::kConvert ? pack_f32x2(__int2float_rn(static_cast<int>(lo)), __int2float_rn(static_cast<int>(hi)))
+                                  : add_f32x2(magic_pair(lo, hi), off2);
+            };
+            const unsigned long long d0 = to_float(d[3 * i], d[3 * i + 3]);
+            const unsigned long long d1 = to_float(d[3 * i + 1], d[3 * i + 4]);
+            const unsigned long long d2 = to_float(d[3 * i + 2], d[3 * i + 5]);
             const unsigned long long dot = fma_f32x2(d2, k16, fma_f32x2(d1, k8, d0));
             const unsigned long long acc = fma_f32x2(mul_f32x2(s2, inv2), fma_f32x2(nz2, sum2, dot), pack_f32x2(fin[i], fin[i + 1]));
             unpack_f32x2(acc, fin[i], fin[i + 1]);
