@@ -81,6 +81,7 @@ constexpr uint32_t kSpinLimit = 1u << 20;  // polls before a wait gives up
 constexpr uint32_t kPieceTag = 0x7A6B5C4Du;  // upper half of a published (sum, tag) word of a split tile's piece
 constexpr int kFixBar = 1;                 // named barrier of the fix-up warps
 constexpr int kConvBar = 2;                // named barrier of the converting warps
+constexpr int kChainBytes = 32 * 4;        // M = 1 with the RMSNorm: a k group's terms of the sum of squares
 constexpr int kConvBatch = 4;              // M = 1: k groups a warp converts with their loads in flight together
 constexpr int kTmemCols = 512;             // all of tensor memory; the next launch's CTA, resident beside this one,
                                            // gets it when this CTA exits (it cannot multiply before that anyway)
@@ -377,7 +378,7 @@ __device__ __forceinline__ float small_int_to_float(uint32_t v) {
 
 // dynamic shared memory:
 //   [weight ring: depth x 17152][B region: b_bytes][(scale,zp) ring: kSide x 128 x 4][(sum, 2^-p): xs_bytes]
-//   [step table: kTable x 8][ready flags: 256 x 4][M = 1: sums of squares 256 x 4, mailbox][mbarriers][tmem base, flag]
+//   [step table: kTable x 8][ready flags: 256 x 4][M = 1: mailbox, the norm's scale 4 x 4][mbarriers][tmem base, flag]
 // The B operand of one k group is eight 16-k chunks, 48 M bytes apart, each holding the 3 M digit rows in
 // use as consecutive 16-byte rows (an 8-row core matrix every 128 bytes). The rows the tensor core reads
 // beyond them are the next chunk's bytes: they only produce accumulator columns nobody reads, and the
@@ -398,7 +399,7 @@ __host__ __device__ constexpr int bar_count(int depth, int bdepth) {
 template <int MT>
 __host__ __device__ inline int total_smem(int depth, int stage_bytes, int b_bytes, int xs_bytes, int bdepth) {
   return depth * stage_bytes + b_bytes + kSide * kTileRows * 4 + xs_bytes + kTable * 8 + 256 * 4 +
-         (tile_end_helper<MT>() ? (kMailWords + 256) * 4 : 0) + bar_count<MT>(depth, bdepth) * 8 + 16;
+         (tile_end_helper<MT>() ? (kMailWords + 4) * 4 : 0) + bar_count<MT>(depth, bdepth) * 8 + 16;
 }
 
 // One token's 128 values of one k group (this lane: k = 4 lane .. 4 lane + 3, `rv`) -> three int8 digit
@@ -446,23 +447,18 @@ __device__ __forceinline__ void convert_group(uint2 rv, uint8_t* bslot, int lbo,
 }
 
 // ---- RMSNorm in front of a layer: xn = bf16(x * inv * (1 + w)), inv = rsqrt(mean(x^2) + eps) over the token's row ----
-// One group's sum of squares (this lane: four of its 128 values), on every lane.
-__device__ __forceinline__ float group_sumsq(uint2 q) {
+// The row's sum of squares is added up in ONE order, so that a token's normalised values do not depend on which warps or
+// CTAs add, nor on M: chain l (0..31) runs over the groups in ascending order and takes elements 4 l .. 4 l + 3 of each as
+// (a0^2 + a1^2) + (a2^2 + a3^2); the 32 chains are then added as an xor tree (16, 8, 4, 2, 1).
+__device__ __forceinline__ float sumsq4(uint2 q) {
   const float a0 = __uint_as_float(q.x << 16), a1 = __uint_as_float(q.x & 0xFFFF0000u);
   const float a2 = __uint_as_float(q.y << 16), a3 = __uint_as_float(q.y & 0xFFFF0000u);
-  float ss = (a0 * a0 + a1 * a1) + (a2 * a2 + a3 * a3);
-#pragma unroll
-  for (int off = 16; off; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-  return ss;
+  return (a0 * a0 + a1 * a1) + (a2 * a2 + a3 * a3);
 }
-// The row's, from its groups': always added up in this order, so that a token's normalised values do not depend on
-// which warps or CTAs summed the groups.
-__device__ __forceinline__ float row_sumsq(const float* sumsq, int G, int lane) {
-  float ss = 0.f;
-  for (int g = lane; g < G; g += 32) ss += sumsq[g];
+__device__ __forceinline__ float row_inv(float chain, int K, float eps) {  // this lane's chain; the result on every lane
 #pragma unroll
-  for (int off = 16; off; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-  return ss;
+  for (int off = 16; off; off >>= 1) chain += __shfl_xor_sync(0xffffffffu, chain, off);
+  return rsqrtf(chain / static_cast<float>(K) + eps);
 }
 __device__ __forceinline__ uint2 normalise(uint2 q, uint2 w, float inv) {
   auto nrm = [&](uint32_t xb, uint32_t wb) {  // both bf16 bit patterns in the high half
@@ -493,8 +489,8 @@ __global__ void __launch_bounds__(Geo<MT>::kBoundThreads, 1) k_skinny(const Skin
   uint32_t* ready = reinterpret_cast<uint32_t*>(table + kTable);  // M = 1, [slot]: the group's digit rows are written
   float* mail = reinterpret_cast<float*>(ready + 256);  // [2 entries][lane quarter][kMailStride] (helper instances only)
   constexpr bool kHelper = tile_end_helper<MT>();
-  float* sumsq = mail + kMailWords;                       // M = 1 with the RMSNorm: [k group] sum of squares
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ready + 256 + (kHelper ? kMailWords + 256 : 0));
+  float* row_scale = mail + kMailWords;                   // M = 1 with the RMSNorm: the row's inv
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ready + 256 + (kHelper ? kMailWords + 4 : 0));
   const int BD = p.bdepth, BS = p.bshift;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + bar_count<MT>(DS, BD));
   int* sflag = reinterpret_cast<int*>(tmem_slot + 1);
@@ -594,33 +590,42 @@ __global__ void __launch_bounds__(Geo<MT>::kBoundThreads, 1) k_skinny(const Skin
     // the first batch; with the fused RMSNorm it is k group i (every CTA sums the whole row).
     const int ti = warp < CW ? warp : (warp == 14 ? CW : warp - kWConv0 + CW + 1);
     const int cnt = (u1 - u0 < G) ? u1 - u0 : G;
-    const bool norm = p.ln_w != nullptr;
+    const bool norm = WB == 4 && p.ln_w != nullptr;
     const int total = norm ? G : cnt;  // items; item i belongs to warp i % kTeam
     const uint2* x2 = reinterpret_cast<const uint2*>(p.x) + lane;
     auto group_of = [&](int i) { return norm ? i : (g_first + i < G ? g_first + i : g_first + i - G); };
-    uint2 rv[kConvBatch];
+    uint2 rv[kConvBatch], wv[kConvBatch];
     auto load = [&](int i0) {
 #pragma unroll
       for (int j = 0; j < kConvBatch; ++j)
-        if (i0 + j * kTeam < total) rv[j] = __ldcg(x2 + group_of(i0 + j * kTeam) * (kGroup / 4));
+        if (i0 + j * kTeam < total) {
+          rv[j] = __ldcg(x2 + group_of(i0 + j * kTeam) * (kGroup / 4));
+          if (norm) wv[j] = __ldg(reinterpret_cast<const uint2*>(p.ln_w) + lane + (i0 + j * kTeam) * (kGroup / 4));
+        }
     };
     load(ti);
     float inv = 0.f;
     if (norm) {
-      // RMSNorm fused in (replaces the separate kernel in front of the linear layer): every CTA sums the row, 10 KB of
-      // loads that its conversion makes anyway. As a pre-pass kernel whose warps each walked the row, a block of
-      // 34816 x 5120 and 5120 x 17408 took 35.9 us; now 31.7.
+      // RMSNorm fused in (replaces the separate kernel in front of the linear layer): every CTA sums the whole row. All
+      // converting warps square, one adds the chains up; the terms lie where the digit rows will (b_bytes has the room).
+      // As a pre-pass kernel whose warps each walked the row, a block of 34816 x 5120 and 5120 x 17408 took 35.9 us; now 30.8.
+      float* terms = reinterpret_cast<float*>(bq) + lane;  // [k group][chain]
       for (int i0 = ti; i0 < total; i0 += kConvBatch * kTeam) {
         if (i0 != ti) load(i0);
 #pragma unroll
         for (int j = 0; j < kConvBatch; ++j)
-          if (i0 + j * kTeam < total) {
-            const float ss = group_sumsq(rv[j]);
-            if (lane == 0) sumsq[i0 + j * kTeam] = ss;
-          }
+          if (i0 + j * kTeam < total) terms[(i0 + j * kTeam) * 32] = sumsq4(rv[j]);
       }
       named_bar_sync(kConvBar, kTeam * 32);
-      inv = rsqrtf(row_sumsq(sumsq, G, lane) / static_cast<float>(p.K) + p.ln_eps);
+      if (ti == 0) {
+        float chain = 0.f;
+#pragma unroll 8
+        for (int g = 0; g < G; ++g) chain += terms[g * 32];
+        inv = row_inv(chain, p.K, p.ln_eps);
+        if (lane == 0) *row_scale = inv;
+      }
+      named_bar_sync(kConvBar, kTeam * 32);
+      inv = *row_scale;
       if (total > kConvBatch * kTeam) load(ti);
     }
     for (int i0 = ti; i0 < total; i0 += kConvBatch * kTeam) {
@@ -631,7 +636,7 @@ __global__ void __launch_bounds__(Geo<MT>::kBoundThreads, 1) k_skinny(const Skin
         if (i < total) {
           const int g = group_of(i), slot = norm ? cache_slot(g) : i;
           if (norm) {
-            rv[j] = normalise(rv[j], __ldg(reinterpret_cast<const uint2*>(p.ln_w + g * kGroup) + lane), inv);
+            rv[j] = normalise(rv[j], wv[j], inv);
             if (p.xn_out && g % gridDim.x == blockIdx.x) reinterpret_cast<uint2*>(p.xn_out + g * kGroup)[lane] = rv[j];
           }
           if (slot < cnt)
@@ -1383,25 +1388,32 @@ __global__ void __launch_bounds__(128, 16) k_digits(const uint16_t* __restrict__
   uint2 rv = !NORM || g < G ? __ldcg(row + g * (kGroup / 4)) : make_uint2(0u, 0u);
   if constexpr (NORM) {
     // RMSNorm fused in (replaces the separate kernel in front of the linear layer), rounded to bf16 as the unfused path
-    // stores it; the digits are taken of xn. Every CTA sums the token's whole row, a quarter of it per warp, six loads in
+    // stores it; the digits are taken of xn. Every CTA sums the token's whole row, eight chains per warp, six loads in
     // flight; a warp alone, one load after the other, held up the layer behind it.
-    constexpr int kBatch = 6;
-    __shared__ float sumsq[256];
-    for (int g0 = warp; g0 < G; g0 += 4 * kBatch) {
+    // A warp loads four groups' terms of its chains at a time; a chain's next terms come by shuffle.
+    constexpr int kBatch = 6, kPer = 8, kPhases = 32 / kPer;
+    __shared__ float chains[32];
+    const int c = lane % kPer, ph = lane / kPer;
+    float chain = 0.f;
+    for (int g0 = 0; g0 < G; g0 += kPhases * kBatch) {
       uint2 q[kBatch];
 #pragma unroll
-      for (int j = 0; j < kBatch; ++j)
-        if (g0 + 4 * j < G) q[j] = __ldcg(row + (g0 + 4 * j) * (kGroup / 4));
+      for (int j = 0; j < kBatch; ++j) {
+        const int gj = g0 + j * kPhases + ph;
+        q[j] = gj < G ? __ldcg(row - lane + gj * (kGroup / 4) + kPer * warp + c) : make_uint2(0u, 0u);
+      }
 #pragma unroll
       for (int j = 0; j < kBatch; ++j)
-        if (g0 + 4 * j < G) {
-          const float ss = group_sumsq(q[j]);
-          if (lane == 0) sumsq[g0 + 4 * j] = ss;
+        if (g0 + j * kPhases < G) {
+          const float v = sumsq4(q[j]);
+#pragma unroll
+          for (int s = 0; s < kPhases; ++s) chain += __shfl_sync(0xffffffffu, v, s * kPer + c);  // (+ 0 past the last group)
         }
     }
+    if (lane < kPer) chains[kPer * warp + lane] = chain;
     __syncthreads();
     if (g >= G) return;
-    const float inv = rsqrtf(row_sumsq(sumsq, G, lane) / static_cast<float>(K) + ln_eps);
+    const float inv = row_inv(chains[lane], K, ln_eps);
     rv = normalise(rv, __ldg(reinterpret_cast<const uint2*>(ln_w + g * kGroup) + lane), inv);
     if (xn_out) reinterpret_cast<uint2*>(xn_out + static_cast<size_t>(m) * K + g * kGroup)[lane] = rv;
   }
@@ -1530,6 +1542,7 @@ int launch_cfg(SkinnyParams& p, int grid, cudaStream_t st, int smem_optin) {
     return launch_kernel<MT, WB, COMM>(p, grid, st, smem);
   }
   p.b_bytes = groups * 384 * p.M + 256;
+  if (p.ln_w) p.b_bytes = std::max(p.b_bytes, p.G * kChainBytes);
   p.xs_bytes = groups * MT * 8;
   p.bdepth = 0;
   p.bshift = 0;
@@ -1575,7 +1588,7 @@ int launch_kernel(const SkinnyParams& p, int grid, cudaStream_t st, int smem) {
 // M = 1: the digit rows of `groups` k groups (384 B + one pair per group) must fit beside a two-stage
 // weight ring.
 bool gemv_cache_fits(int groups, int stage_bytes, int smem_optin) {
-  const int fixed = 2 * stage_bytes + kSide * kTileRows * 4 + kTable * 8 + 256 * 4 + (kMailWords + 256) * 4 + 64 * 8 + 16 + 256;
+  const int fixed = 2 * stage_bytes + kSide * kTileRows * 4 + kTable * 8 + 256 * 4 + (kMailWords + 4) * 4 + 64 * 8 + 16 + 256;
   return groups * (384 + 8) <= smem_optin - fixed;
 }
 

@@ -1,5 +1,6 @@
-"""The fused RMSNorm at M = 1 (inside the decode kernel) against the pre-pass of M >= 2: the row's sum of squares is added up in
-one order everywhere, so a token's normalised activations and its outputs have the same bits alone and in a block."""
+"""The fused RMSNorm at M = 1 (inside the decode kernel) and in the pre-pass of M >= 2: the row's sum of squares is added up in
+one order everywhere, 32 chains over the k groups and then a tree, so a token's normalised activations and its outputs have the
+same bits alone and in a block, and the bits of that order."""
 import numpy as np
 import pytest
 
@@ -39,6 +40,55 @@ def test_normalised_row_alone_and_in_a_block(pkg, oracle, synth, N, K):
     diff = (xn3.view(torch.int16).int() - want.view(torch.int16).int()).abs()
     assert int(diff.max()) <= 1 and float((diff != 0).float().mean()) < 0.01
     assert np.isfinite(host_bits(y3).astype(np.float32)).all() and pkg.device_status() == 0
+    pkg.gemv_scratch_free(scratch)
+    pkg.awq_free(w)
+
+
+def _chains(x):
+    """Sum of squares per row: chain l takes elements 4 l .. 4 l + 3 of every group, groups ascending; then the xor tree."""
+    q = (x.float() ** 2).view(x.shape[0], -1, 32, 4)
+    v = (q[..., 0] + q[..., 1]) + (q[..., 2] + q[..., 3])
+    ss = torch.zeros_like(v[:, 0])
+    for g in range(v.shape[1]):
+        ss = ss + v[:, g]
+    lanes = torch.arange(32, device=x.device)
+    for off in (16, 8, 4, 2, 1):
+        ss = ss + ss[:, lanes ^ off]
+    return ss[:, :1]
+
+
+def _by_groups(x):
+    return (x.float() ** 2).view(x.shape[0], -1, 128).sum(dim=2).sum(dim=1, keepdim=True)
+
+
+# one group; groups that fill the chains' rounds of loads and that do not; all 256 groups
+@pytest.mark.parametrize("K", [128, 640, 5120, 7040, 17408, 32768])
+@pytest.mark.parametrize("M", [1, 3, 16])
+def test_order_of_the_sum_of_squares(pkg, synth, M, K):
+    N, eps = 256, 1e-6
+    w = pkg.weights_from_numpy(*synth.make_weights(N, K, seed=3))
+    scratch = pkg.gemv_scratch_alloc(K, N, 128, 16)
+    gen = torch.Generator(device="cuda").manual_seed(K + M)
+    ln = torch.randn(K, device="cuda", generator=gen).to(torch.bfloat16)
+    smooth = torch.randn((M, K), device="cuda", generator=gen).to(torch.bfloat16)
+    # every chain reaches 2^24 in the first group, and the ones that follow are lost one by one (a sum of several is not)
+    steep = torch.full((M, K), 0.5, device="cuda", dtype=torch.bfloat16)
+    steep[:, :128] = 0.0
+    steep[:, :128:4] = 4096.0
+    n, e = torch.tensor(float(K), device="cuda"), torch.tensor(eps, device="cuda", dtype=torch.float32)
+
+    def norm(x, ss):
+        return (x.float() * torch.rsqrt(ss / n + e) * (1.0 + ln.float())).to(torch.bfloat16).view(torch.int16)
+
+    for x in (smooth, steep):
+        y = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+        xn = torch.zeros((M, K), dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        pkg.linear_fused(y, w, x, M, scratch, ln_weight=ln, ln_eps=eps, xn_out=xn)
+        assert torch.equal(xn.view(torch.int16), norm(x, _chains(x)))
+    if K >= 17408:  # where the order shows in bf16
+        assert not torch.equal(norm(steep, _chains(steep)), norm(steep, _by_groups(steep)))
+    assert pkg.device_status() == 0
     pkg.gemv_scratch_free(scratch)
     pkg.awq_free(w)
 
