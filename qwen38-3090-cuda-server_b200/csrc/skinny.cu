@@ -378,7 +378,7 @@ __device__ __forceinline__ float small_int_to_float(uint32_t v) {
 
 // dynamic shared memory:
 //   [weight ring: depth x 17152][B region: b_bytes][(scale,zp) ring: kSide x 128 x 4][(sum, 2^-p): xs_bytes]
-//   [step table: kTable x 8][ready flags: 256 x 4][M = 1: mailbox, the norm's scale 4 x 4][mbarriers][tmem base, flag]
+//   [step table: kTable x 8][ready flags: 256 x 4][M = 1: mailbox; with the norm: its scale, 16 B][mbarriers][tmem base, flag]
 // The B operand of one k group is eight 16-k chunks, 48 M bytes apart, each holding the 3 M digit rows in
 // use as consecutive 16-byte rows (an 8-row core matrix every 128 bytes). The rows the tensor core reads
 // beyond them are the next chunk's bytes: they only produce accumulator columns nobody reads, and the
@@ -396,10 +396,10 @@ template <int MT>
 __host__ __device__ constexpr int bar_count(int depth, int bdepth) {
   return 2 * depth + Geo<MT>::AD2 + Geo<MT>::ND + Geo<MT>::DD2 + 2 + (Geo<MT>::kStream ? 2 * bdepth : 0) + 1 + (tile_end_helper<MT>() ? 2 * CW : 0);
 }
-template <int MT>
+template <int MT, bool NORM = false>
 __host__ __device__ inline int total_smem(int depth, int stage_bytes, int b_bytes, int xs_bytes, int bdepth) {
   return depth * stage_bytes + b_bytes + kSide * kTileRows * 4 + xs_bytes + kTable * 8 + 256 * 4 +
-         (tile_end_helper<MT>() ? (kMailWords + 4) * 4 : 0) + bar_count<MT>(depth, bdepth) * 8 + 16;
+         (tile_end_helper<MT>() ? kMailWords * 4 : 0) + (NORM ? 16 : 0) + bar_count<MT>(depth, bdepth) * 8 + 16;
 }
 
 // One token's 128 values of one k group (this lane: k = 4 lane .. 4 lane + 3, `rv`) -> three int8 digit
@@ -470,8 +470,9 @@ __device__ __forceinline__ uint2 normalise(uint2 q, uint2 w, float inv) {
 
 // COMM: the cross-rank flag code (wait before x is read, signal after the last store, the pair exchange of the
 // vocab-sharded head) is compiled into separate instances, so that single-GPU launches run exactly the code
-// they ran without it.
-template <int MT, int WB, bool COMM>
+// they ran without it. NORM (M = 1, int4): so is the RMSNorm of x, whose code as a branch of the plain kernel cost the
+// small GEMVs 5 to 14 %: 4096 x 1024 4.02 us without, 4.2 to 4.45 with it, 2048 x 2048 4.6 and 4.9 to 5.3.
+template <int MT, int WB, bool COMM, bool NORM = false>
 __global__ void __launch_bounds__(Geo<MT>::kBoundThreads, 1) k_skinny(const SkinnyParams p) {
   using GE = Geo<MT>;
   constexpr int kBlock = Fmt<WB>::kBlock, kStageBytes = Fmt<WB>::kStage;
@@ -490,7 +491,7 @@ __global__ void __launch_bounds__(Geo<MT>::kBoundThreads, 1) k_skinny(const Skin
   float* mail = reinterpret_cast<float*>(ready + 256);  // [2 entries][lane quarter][kMailStride] (helper instances only)
   constexpr bool kHelper = tile_end_helper<MT>();
   float* row_scale = mail + kMailWords;                   // M = 1 with the RMSNorm: the row's inv
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ready + 256 + (kHelper ? kMailWords + 4 : 0));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ready + 256 + (kHelper ? kMailWords : 0) + (NORM ? 4 : 0));
   const int BD = p.bdepth, BS = p.bshift;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + bar_count<MT>(DS, BD));
   int* sflag = reinterpret_cast<int*>(tmem_slot + 1);
@@ -586,72 +587,90 @@ __global__ void __launch_bounds__(Geo<MT>::kBoundThreads, 1) k_skinny(const Skin
         atomicExch(p.status, W4A16_ETIMEOUT);
       }
     }
-    // Item i is k group (g_first + i) % G, the order in which the CTA walks its groups, so the first steps can start after
-    // the first batch; with the fused RMSNorm it is k group i (every CTA sums the whole row).
     const int ti = warp < CW ? warp : (warp == 14 ? CW : warp - kWConv0 + CW + 1);
     const int cnt = (u1 - u0 < G) ? u1 - u0 : G;
-    const bool norm = WB == 4 && p.ln_w != nullptr;
-    const int total = norm ? G : cnt;  // items; item i belongs to warp i % kTeam
     const uint2* x2 = reinterpret_cast<const uint2*>(p.x) + lane;
-    auto group_of = [&](int i) { return norm ? i : (g_first + i < G ? g_first + i : g_first + i - G); };
-    uint2 rv[kConvBatch], wv[kConvBatch];
-    auto load = [&](int i0) {
-#pragma unroll
-      for (int j = 0; j < kConvBatch; ++j)
-        if (i0 + j * kTeam < total) {
-          rv[j] = __ldcg(x2 + group_of(i0 + j * kTeam) * (kGroup / 4));
-          if (norm) wv[j] = __ldg(reinterpret_cast<const uint2*>(p.ln_w) + lane + (i0 + j * kTeam) * (kGroup / 4));
-        }
+    uint2 rv[kConvBatch];
+    // Publishes slots, one per lane (-1: none): B was written through the generic proxy, the tensor core reads it through the
+    // async one.
+    auto publish = [&](int slot) {
+      fence_proxy_async();
+      __syncwarp();
+      if (slot >= 0) {
+        __threadfence_block();
+        *reinterpret_cast<volatile uint32_t*>(ready + slot) = 1u;
+      }
     };
-    load(ti);
-    float inv = 0.f;
-    if (norm) {
-      // RMSNorm fused in (replaces the separate kernel in front of the linear layer): every CTA sums the whole row. All
-      // converting warps square, one adds the chains up; the terms lie where the digit rows will (b_bytes has the room).
-      // As a pre-pass kernel whose warps each walked the row, a block of 34816 x 5120 and 5120 x 17408 took 35.9 us; now 30.8.
+    if constexpr (!NORM) {
+      // Item i is k group (g_first + i) % G in slot i, the order in which the CTA walks its groups, so the first steps can
+      // start after the first round; it belongs to warp i % kTeam.
+      for (int i0 = ti; i0 < cnt; i0 += kConvBatch * kTeam) {
+#pragma unroll
+        for (int j = 0; j < kConvBatch; ++j) {
+          const int i = i0 + j * kTeam;
+          if (i < cnt) {
+            int g = g_first + i;
+            if (g >= G) g -= G;
+            rv[j] = __ldcg(x2 + g * (kGroup / 4));
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < kConvBatch; ++j) {
+          const int i = i0 + j * kTeam;
+          if (i < cnt) {
+            convert_group(rv[j], bq + i * b_slot, b_lbo, 0, reinterpret_cast<float*>(xsinv) + 2 * i, 1, lane);
+            publish(lane == 0 ? i : -1);
+          }
+        }
+      }
+    } else {
+      // RMSNorm fused in (replaces the separate kernel in front of the linear layer): every CTA sums the whole row, and item i
+      // is k group i. All converting warps square, one adds the chains up; the terms lie where the digit rows will
+      // (b_bytes has the room). As a pre-pass kernel whose warps each walked the row, a block of 34816 x 5120 and
+      // 5120 x 17408 took 35.9 us; now 31.3.
+      uint2 wv[kConvBatch];
+      auto load = [&](int i0) {
+#pragma unroll
+        for (int j = 0; j < kConvBatch; ++j)
+          if (i0 + j * kTeam < G) {
+            rv[j] = __ldcg(x2 + (i0 + j * kTeam) * (kGroup / 4));
+            wv[j] = __ldg(reinterpret_cast<const uint2*>(p.ln_w) + lane + (i0 + j * kTeam) * (kGroup / 4));
+          }
+      };
+      load(ti);
       float* terms = reinterpret_cast<float*>(bq) + lane;  // [k group][chain]
-      for (int i0 = ti; i0 < total; i0 += kConvBatch * kTeam) {
+      for (int i0 = ti; i0 < G; i0 += kConvBatch * kTeam) {
         if (i0 != ti) load(i0);
 #pragma unroll
         for (int j = 0; j < kConvBatch; ++j)
-          if (i0 + j * kTeam < total) terms[(i0 + j * kTeam) * 32] = sumsq4(rv[j]);
+          if (i0 + j * kTeam < G) terms[(i0 + j * kTeam) * 32] = sumsq4(rv[j]);
       }
       named_bar_sync(kConvBar, kTeam * 32);
       if (ti == 0) {
         float chain = 0.f;
 #pragma unroll 8
         for (int g = 0; g < G; ++g) chain += terms[g * 32];
-        inv = row_inv(chain, p.K, p.ln_eps);
+        const float inv = row_inv(chain, p.K, p.ln_eps);
         if (lane == 0) *row_scale = inv;
       }
       named_bar_sync(kConvBar, kTeam * 32);
-      inv = *row_scale;
-      if (total > kConvBatch * kTeam) load(ti);
-    }
-    for (int i0 = ti; i0 < total; i0 += kConvBatch * kTeam) {
-      if (i0 != ti) load(i0);
+      const float inv = *row_scale;
+      if (G > kConvBatch * kTeam) load(ti);
+      for (int i0 = ti; i0 < G; i0 += kConvBatch * kTeam) {
+        if (i0 != ti) load(i0);
 #pragma unroll
-      for (int j = 0; j < kConvBatch; ++j) {
-        const int i = i0 + j * kTeam;
-        if (i < total) {
-          const int g = group_of(i), slot = norm ? cache_slot(g) : i;
-          if (norm) {
+        for (int j = 0; j < kConvBatch; ++j) {
+          const int g = i0 + j * kTeam;
+          if (g < G) {
+            const int slot = cache_slot(g);
             rv[j] = normalise(rv[j], wv[j], inv);
             if (p.xn_out && g % gridDim.x == blockIdx.x) reinterpret_cast<uint2*>(p.xn_out + g * kGroup)[lane] = rv[j];
+            if (slot < cnt)
+              convert_group(rv[j], bq + slot * b_slot, b_lbo, 0, reinterpret_cast<float*>(xsinv) + 2 * slot, 1, lane);
           }
-          if (slot < cnt)
-            convert_group(rv[j], bq + slot * b_slot, b_lbo, 0, reinterpret_cast<float*>(xsinv) + 2 * slot, 1, lane);
         }
-      }
-      // publish the batch, one fence for all of it: B was written through the generic proxy, the tensor core reads it
-      // through the async one
-      fence_proxy_async();
-      __syncwarp();
-      const int i = i0 + lane * kTeam;
-      if (lane < kConvBatch && i < total) {
-        const int slot = norm ? cache_slot(i) : i;
-        __threadfence_block();
-        if (slot < cnt) *reinterpret_cast<volatile uint32_t*>(ready + slot) = 1u;
+        const int g = i0 + lane * kTeam, slot = cache_slot(g);
+        publish(lane < kConvBatch && g < G && slot < cnt ? slot : -1);
       }
     }
     __syncwarp();
@@ -1509,10 +1528,10 @@ int cache_groups_for(int tiles, int G, int grid) {
   return per_cta < G ? per_cta : G;
 }
 
-template <int MT, int WB, bool COMM>
+template <int MT, int WB, bool COMM, bool NORM = false>
 int launch_kernel(const SkinnyParams& p, int grid, cudaStream_t st, int smem);
 
-template <int MT, int WB, bool COMM>
+template <int MT, int WB, bool COMM, bool NORM = false>
 int launch_cfg(SkinnyParams& p, int grid, cudaStream_t st, int smem_optin) {
   constexpr int kStageBytes = Fmt<WB>::kStage;
   constexpr bool kStream = Geo<MT>::kStream;
@@ -1542,7 +1561,7 @@ int launch_cfg(SkinnyParams& p, int grid, cudaStream_t st, int smem_optin) {
     return launch_kernel<MT, WB, COMM>(p, grid, st, smem);
   }
   p.b_bytes = groups * 384 * p.M + 256;
-  if (p.ln_w) p.b_bytes = std::max(p.b_bytes, p.G * kChainBytes);
+  if constexpr (NORM) p.b_bytes = std::max(p.b_bytes, p.G * kChainBytes);
   p.xs_bytes = groups * MT * 8;
   p.bdepth = 0;
   p.bshift = 0;
@@ -1551,24 +1570,24 @@ int launch_cfg(SkinnyParams& p, int grid, cudaStream_t st, int smem_optin) {
   // uses would belong to different warps, and a warp that runs ahead could take "the other warp's copy has
   // not landed yet" for "my copy has landed".
   p.depth = config().depth;
-  int smem = total_smem<MT>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
+  int smem = total_smem<MT, NORM>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
   while (smem > limit && p.depth > 2) {
     p.depth -= 2;
-    smem = total_smem<MT>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
+    smem = total_smem<MT, NORM>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
   }
   if (smem > smem_optin)
     return fail(W4A16_EINVAL, "decode kernel needs %d bytes of shared memory for in_f = %d, M = %d; the device offers %d",
                 smem, p.K, p.M, smem_optin);
-  return launch_kernel<MT, WB, COMM>(p, grid, st, smem);
+  return launch_kernel<MT, WB, COMM, NORM>(p, grid, st, smem);
 }
 
-template <int MT, int WB, bool COMM>
+template <int MT, int WB, bool COMM, bool NORM>
 int launch_kernel(const SkinnyParams& p, int grid, cudaStream_t st, int smem) {
   static int attr_set[64] = {};
   int dev = 0;
   W4_CUDA(cudaGetDevice(&dev));
   if (attr_set[dev & 63] < smem) {
-    W4_CUDA(cudaFuncSetAttribute(k_skinny<MT, WB, COMM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    W4_CUDA(cudaFuncSetAttribute(k_skinny<MT, WB, COMM, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     attr_set[dev & 63] = smem;
   }
   cudaLaunchConfig_t cfg = {};
@@ -1581,7 +1600,7 @@ int launch_kernel(const SkinnyParams& p, int grid, cudaStream_t st, int smem) {
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = (config().pdl && !p.ordered) ? 1 : 0;
-  W4_CUDA(cudaLaunchKernelEx(&cfg, k_skinny<MT, WB, COMM>, p));
+  W4_CUDA(cudaLaunchKernelEx(&cfg, k_skinny<MT, WB, COMM, NORM>, p));
   return W4A16_OK;
 }
 
@@ -1654,6 +1673,8 @@ int layer_of(LayerRef& L, const w4a16_w8_weights_t* w) {
 
 template <int WB, bool COMM>
 int launch_batch_c(SkinnyParams& q, int grid, cudaStream_t st, int smem_optin) {
+  if constexpr (WB == 4 && !COMM)  // the norm is an option of w4a16_linear_fused alone
+    if (q.ln_w && !q.dig) return launch_cfg<1, WB, COMM, true>(q, grid, st, smem_optin);
   switch (instance_for(q.dig ? std::max(q.M, 2) : q.M)) {
     case 1: return launch_cfg<1, WB, COMM>(q, grid, st, smem_optin);
     case 2: return launch_cfg<2, WB, COMM>(q, grid, st, smem_optin);    // token sets 1, 1
