@@ -128,7 +128,16 @@ struct Geo {
   //   M = 15  28.2 / 19.6 / 16.5 / 12.2   28.0 / 19.1 / 16.2 / 11.6   27.5 / 17.1 / 15.5 / 10.3
   // and earlier M = 8 80 -> 64 22.4 / 14.3 / - / 10.1 -> 22.7 / 14.0 / - / 9.2, M = 16 72 -> 64 30.5 / 19.1 / - / 12.7 -> 28.9 / 17.1 / - / 11.1
   // (those with 17408 x 5120 in the second place).
-  static constexpr int kBoundThreads = MT == 8 || MT == 12 || MT >= 15 ? 1024 : (MT == 6 ? 896 : kThreads);
+  // Int8 weights keep 80 at M = 6 and 15: their instances spill more (M = 15 4 bytes of stores at 80, 36 at 64; M = 6 12 and, at 72,
+  // 36), and they serve heads, where the room for the next pre-pass counts for little. Heads of 248320 x 5120 / 131072 x 4096 /
+  // 65536 x 2048 / 32768 x 1024 (rows x columns) in us: M = 15, 64 -> 80: 212.0 / 98.4 / 36.5 / 19.0 -> 207.2 / 95.1 / 35.2 / 18.7 (a
+  // layer of 5120 x 6144 11.2 -> 12.4); M = 6, 72 -> 80: 190.6 / 86.6 / 30.6 / 14.2 -> 190.4 / 86.4 / 30.5 / 14.1.
+  template <int WB>
+  static constexpr int bound_threads() {
+    if (MT == 8 || MT == 12 || MT == 16) return 1024;
+    if (WB == 4 && MT == 15) return 1024;
+    return WB == 4 && MT == 6 ? 896 : kThreads;
+  }
   // int32 -> fp32 of the sums by the conversion instruction (exact below 2^24, the same floats) instead of an integer add of a magic
   // constant and a packed subtraction: fewer instructions, on a slower pipe. 34816 x 5120 / 5120 x 17408 / 16384 x 5120 / 5120 x 6144 in us, magic -> conversion:
   //   M = 6 (72 registers) 20.7 / 13.6 / 12.3 / 8.4 -> 20.1 / 13.2 / 12.0 / 8.2    M = 8 22.2 / 14.6 / 13.1 / 9.4 -> 21.2 / 14.1 / 12.6 / 9.1
@@ -473,7 +482,7 @@ __device__ __forceinline__ uint2 normalise(uint2 q, uint2 w, float inv) {
 // they ran without it. NORM (M = 1, int4): so is the RMSNorm of x, whose code as a branch of the plain kernel cost the
 // small GEMVs 5 to 14 %: 4096 x 1024 4.02 us without, 4.2 to 4.45 with it, 2048 x 2048 4.6 and 4.9 to 5.3.
 template <int MT, int WB, bool COMM, bool NORM = false>
-__global__ void __launch_bounds__(Geo<MT>::kBoundThreads, 1) k_skinny(const SkinnyParams p) {
+__global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_skinny(const SkinnyParams p) {
   using GE = Geo<MT>;
   constexpr int kBlock = Fmt<WB>::kBlock, kStageBytes = Fmt<WB>::kStage;
   constexpr int N = GE::N, AD2 = GE::AD2, DD2 = GE::DD2, ND = GE::ND;
