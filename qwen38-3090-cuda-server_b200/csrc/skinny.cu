@@ -72,10 +72,6 @@ struct Fmt {
   static constexpr int kBlock = WB == 4 ? kTileGroupBytes : kW8BlockBytes;  // bytes per (row tile, group)
   static constexpr int kStage = kStepGroups * kBlock;                        // 17152 / 33280
 };
-constexpr int kSideSteps = 16;             // (scale, zp) side ring, in steps: a slot is rewritten by the unpack warps
-                                           // A-ring + D-ring depths (at most 4 + 8 steps) after the fix-up read it. A power of
-                                           // two: the remainder by 12 was 2 % of the time at M = 9 (every warp takes it every step)
-constexpr int kSide = kSideSteps * 2;      // in groups
 constexpr int kTable = 64;                 // step table entries (ring)
 constexpr uint32_t kSpinLimit = 1u << 20;  // polls before a wait gives up
 constexpr uint32_t kPieceTag = 0x7A6B5C4Du;  // upper half of a published (sum, tag) word of a split tile's piece
@@ -128,10 +124,10 @@ struct Geo {
   //   M = 15  28.2 / 19.6 / 16.5 / 12.2   28.0 / 19.1 / 16.2 / 11.6   27.5 / 17.1 / 15.5 / 10.3
   // and earlier M = 8 80 -> 64 22.4 / 14.3 / - / 10.1 -> 22.7 / 14.0 / - / 9.2, M = 16 72 -> 64 30.5 / 19.1 / - / 12.7 -> 28.9 / 17.1 / - / 11.1
   // (those with 17408 x 5120 in the second place).
-  // Int8 weights keep 80 at M = 6 and 15: their instances spill more (M = 15 4 bytes of stores at 80, 36 at 64; M = 6 12 and, at 72,
+  // Int8 weights keep 80 at M = 6 and 15: their instances spill more (M = 15 4 bytes of stores at 80, 76 at 64; M = 6 12 and, at 72,
   // 36), and they serve heads, where the room for the next pre-pass counts for little. Heads of 248320 x 5120 / 131072 x 4096 /
-  // 65536 x 2048 / 32768 x 1024 (rows x columns) in us: M = 15, 64 -> 80: 212.0 / 98.4 / 36.5 / 19.0 -> 207.2 / 95.1 / 35.2 / 18.7 (a
-  // layer of 5120 x 6144 11.2 -> 12.4); M = 6, 72 -> 80: 190.6 / 86.6 / 30.6 / 14.2 -> 190.4 / 86.4 / 30.5 / 14.1.
+  // 65536 x 2048 / 32768 x 1024 (rows x columns) in us: M = 15, 64 -> 80: 223.2 / 102.7 / 36.8 / 18.0 -> 200.1 / 93.2 / 35.3 / 17.1 (a
+  // layer of 5120 x 6144 12.7 -> 12.4); M = 6, 72 -> 80: 190.6 / 86.6 / 30.6 / 14.2 -> 190.4 / 86.4 / 30.5 / 14.1.
   template <int WB>
   static constexpr int bound_threads() {
     if (MT == 8 || MT == 12 || MT == 16) return 1024;
@@ -162,8 +158,22 @@ struct Geo {
   static_assert(3 * TM <= CB && FW * CB <= N, "token sets must fit their column blocks");
   static_assert(kDCol0 + DD2 * kDColsS <= kTmemCols, "tensor memory budget");
   static_assert(AD2 <= ND && DD2 <= ND && DD2 % 2 == 0, "ring depths");  // even: a slot belongs to one issuer
-  static_assert(AD2 + DD2 <= kSideSteps, "a (scale, zp) slot must have been read before the unpack warps reuse it");
 };
+
+// (scale, zp) side ring, in steps: a slot is rewritten by the unpack warps A-ring + D-ring depths (at most 4 + 8 steps) after the
+// fix-up read it. A power of two: the remainder by 12 was 2 % of the time at M = 9 (every warp takes it every step). With int8
+// weights and N = 48 it is twelve: the 4 KB (193 KB of shared memory at in_f = 1024, 197 with them) made launches of small heads
+// slower; it is the size that counts, twelve steps walked in sixteen's memory gained nothing. Heads of 65536 x 2048 / 32768 x 1024 / 16384 x 1024 in us, sixteen -> twelve: M = 9 32.1 / 15.4 / 12.6 -> 30.9 / 14.5 / 11.7, M = 12
+// 32.7 / 16.8 / 13.6 -> 31.4 / 15.6 / 12.5, M = 16 33.4 / 18.0 / 14.8 -> 31.8 / 16.5 / 13.3; wide heads the same.
+template <int MT, int WB>
+__host__ __device__ constexpr int side_steps() {
+  static_assert(Geo<MT>::AD2 + Geo<MT>::DD2 <= 12, "a (scale, zp) slot must have been read before the unpack warps reuse it");
+  return WB == 8 && Geo<MT>::N == 48 ? 12 : 16;
+}
+template <int MT, int WB>
+__host__ __device__ constexpr int side_bytes() {
+  return side_steps<MT, WB>() * kStepGroups * kTileRows * 4;
+}
 
 struct SkinnyParams {
   const uint8_t* stream;  // weight stream, Fmt<WB>::kBlock bytes per (row tile, group)
@@ -386,7 +396,7 @@ __device__ __forceinline__ float small_int_to_float(uint32_t v) {
 }
 
 // dynamic shared memory:
-//   [weight ring: depth x 17152][B region: b_bytes][(scale,zp) ring: kSide x 128 x 4][(sum, 2^-p): xs_bytes]
+//   [weight ring: depth x 17152][B region: b_bytes][(scale,zp) ring: side_bytes][(sum, 2^-p): xs_bytes]
 //   [step table: kTable x 8][ready flags: 256 x 4][M = 1: mailbox; with the norm: its scale, 16 B][mbarriers][tmem base, flag]
 // The B operand of one k group is eight 16-k chunks, 48 M bytes apart, each holding the 3 M digit rows in
 // use as consecutive 16-byte rows (an 8-row core matrix every 128 bytes). The rows the tensor core reads
@@ -405,9 +415,9 @@ template <int MT>
 __host__ __device__ constexpr int bar_count(int depth, int bdepth) {
   return 2 * depth + Geo<MT>::AD2 + Geo<MT>::ND + Geo<MT>::DD2 + 2 + (Geo<MT>::kStream ? 2 * bdepth : 0) + 1 + (tile_end_helper<MT>() ? 2 * CW : 0);
 }
-template <int MT, bool NORM = false>
+template <int MT, int WB, bool NORM = false>
 __host__ __device__ inline int total_smem(int depth, int stage_bytes, int b_bytes, int xs_bytes, int bdepth) {
-  return depth * stage_bytes + b_bytes + kSide * kTileRows * 4 + xs_bytes + kTable * 8 + 256 * 4 +
+  return depth * stage_bytes + b_bytes + side_bytes<MT, WB>() + xs_bytes + kTable * 8 + 256 * 4 +
          (tile_end_helper<MT>() ? kMailWords * 4 : 0) + (NORM ? 16 : 0) + bar_count<MT>(depth, bdepth) * 8 + 16;
 }
 
@@ -485,6 +495,7 @@ template <int MT, int WB, bool COMM, bool NORM = false>
 __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_skinny(const SkinnyParams p) {
   using GE = Geo<MT>;
   constexpr int kBlock = Fmt<WB>::kBlock, kStageBytes = Fmt<WB>::kStage;
+  constexpr int kSideSteps = side_steps<MT, WB>();
   constexpr int N = GE::N, AD2 = GE::AD2, DD2 = GE::DD2, ND = GE::ND;
   constexpr bool kStream = GE::kStream;
   constexpr int SLOT = kTileRows * MT;  // floats per partial tile
@@ -494,7 +505,7 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
   uint8_t* ring = smem;
   uint8_t* bq = ring + DS * kStageBytes;
   uint8_t* side = bq + p.b_bytes;
-  uint8_t* xsinv = side + kSide * kTileRows * 4;
+  uint8_t* xsinv = side + side_bytes<MT, WB>();
   uint2* table = reinterpret_cast<uint2*>(xsinv + p.xs_bytes);
   uint32_t* ready = reinterpret_cast<uint32_t*>(table + kTable);  // M = 1, [slot]: the group's digit rows are written
   float* mail = reinterpret_cast<float*>(ready + 256);  // [2 entries][lane quarter][kMailStride] (helper instances only)
@@ -1558,7 +1569,7 @@ int launch_cfg(SkinnyParams& p, int grid, cudaStream_t st, int smem_optin) {
       p.bshift = c[1] == 8 ? 3 : (c[1] == 4 ? 2 : 1);
       p.b_bytes = p.bdepth * kStepGroups * p.db_bytes;
       p.xs_bytes = (p.G * Geo<MT>::kPairBytes + 15) & ~15;
-      smem = total_smem<MT>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, p.bdepth);
+      smem = total_smem<MT, WB>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, p.bdepth);
       if (smem <= limit) {
         found = true;
         break;
@@ -1579,10 +1590,10 @@ int launch_cfg(SkinnyParams& p, int grid, cudaStream_t st, int smem_optin) {
   // uses would belong to different warps, and a warp that runs ahead could take "the other warp's copy has
   // not landed yet" for "my copy has landed".
   p.depth = config().depth;
-  int smem = total_smem<MT, NORM>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
+  int smem = total_smem<MT, WB, NORM>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
   while (smem > limit && p.depth > 2) {
     p.depth -= 2;
-    smem = total_smem<MT, NORM>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
+    smem = total_smem<MT, WB, NORM>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
   }
   if (smem > smem_optin)
     return fail(W4A16_EINVAL, "decode kernel needs %d bytes of shared memory for in_f = %d, M = %d; the device offers %d",
@@ -1615,8 +1626,9 @@ int launch_kernel(const SkinnyParams& p, int grid, cudaStream_t st, int smem) {
 
 // M = 1: the digit rows of `groups` k groups (384 B + one pair per group) must fit beside a two-stage
 // weight ring.
-bool gemv_cache_fits(int groups, int stage_bytes, int smem_optin) {
-  const int fixed = 2 * stage_bytes + kSide * kTileRows * 4 + kTable * 8 + 256 * 4 + (kMailWords + 4) * 4 + 64 * 8 + 16 + 256;
+template <int WB>
+bool gemv_cache_fits(int groups, int smem_optin) {
+  const int fixed = 2 * Fmt<WB>::kStage + side_bytes<1, WB>() + kTable * 8 + 256 * 4 + (kMailWords + 4) * 4 + 64 * 8 + 16 + 256;
   return groups * (384 + 8) <= smem_optin - fixed;
 }
 
@@ -1739,8 +1751,8 @@ int launch_skinny(SkinnyParams& p, const LayerRef* w, const uint16_t* x, int M, 
   const bool in_place = p.ln_w != nullptr && yb != nullptr && yb < xb + 2LL * M * p.K && xb < yb + 2LL * M * p.ldy;
   const bool prepass = M >= 2 || in_place;
   if (!prepass) {
-    if (!gemv_cache_fits(cache_groups_for(p.tiles, p.G, grid), w->wbits == 4 ? Fmt<4>::kStage : Fmt<8>::kStage,
-                         di->smem_optin))
+    const int groups = cache_groups_for(p.tiles, p.G, grid);
+    if (!(w->wbits == 4 ? gemv_cache_fits<4>(groups, di->smem_optin) : gemv_cache_fits<8>(groups, di->smem_optin)))
       return fail(W4A16_EINVAL, "in_f = %d is too wide for the decode kernel's activation cache", w->in_f);
   } else {
     // the pre-pass: digit rows of all M tokens, once per call, into the scratch (behind the argmax pairs)
