@@ -42,7 +42,8 @@ const DeviceInfo* device_info();
 // stores of the kernel in front of them are visible. So every entry that writes weight buffers notes its
 // stream, and the next matmul call on that stream is enqueued without the programmatic-serialisation
 // attribute: fully ordered behind the write. take_weight_write is true once per noted stream; with no write
-// pending it costs one relaxed atomic load.
+// pending it costs one relaxed atomic load. It is called when nothing can refuse the call any more, and a launch that
+// fails notes the stream again.
 void note_weight_write(cudaStream_t st);
 bool take_weight_write(cudaStream_t st);
 bool pdl_enabled();  // programmatic dependent launch (default on; W4A16_PDL=0 turns it off)

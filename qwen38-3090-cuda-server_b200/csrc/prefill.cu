@@ -692,15 +692,18 @@ int launch_prefill(PrefillParams& p, uint16_t* C, const w4a16_weights_t* w, cons
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
   cluster_config(cfg, at, plan.splits, plan.clusters, plan.smem);
-  if (!take_weight_write(static_cast<cudaStream_t>(stream)) && pdl_enabled()) {
+  const bool behind_write = take_weight_write(static_cast<cudaStream_t>(stream));
+  if (!behind_write && pdl_enabled()) {
     // (behind a weight write the launch is fully ordered: the weights are read before the wait)
     at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = 2;
   }
   cfg.stream = static_cast<cudaStream_t>(stream);
-  W4_CUDA(cudaLaunchKernelEx(&cfg, k_prefill, p));
-  return W4A16_OK;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_prefill, p);
+  if (e == cudaSuccess) return W4A16_OK;
+  if (behind_write) note_weight_write(static_cast<cudaStream_t>(stream));
+  return fail(W4A16_ECUDA, "gemm_prefill: launch: %s", cudaGetErrorString(e));
 }
 }  // namespace
 

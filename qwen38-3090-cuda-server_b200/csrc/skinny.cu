@@ -1714,6 +1714,31 @@ int launch_batch(SkinnyParams& q, int grid, cudaStream_t st, int smem_optin) {
                                          : launch_batch_c<WB, false>(q, grid, st, smem_optin);
 }
 
+// The launches of a call whose arguments have passed every check but the instance's own shared-memory budget.
+int enqueue_skinny(SkinnyParams& p, const LayerRef* w, bool prepass, const DeviceInfo* di, int grid, cudaStream_t st) {
+  if (prepass) {
+    // the pre-pass: digit rows of all M tokens, once per call, into the scratch
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.ln_w ? p.M * ((p.G + 3) / 4) : (p.G * p.M + 3) / 4);
+    cfg.blockDim = dim3(128);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    // the first launch of the call carries the ordering behind a weight write; the main kernel may then overlap
+    // with this one as usual
+    cfg.numAttrs = (config().pdl && !p.ordered) ? 1 : 0;
+    p.ordered = 0;
+    const DigitGeometry dg = digit_geometry(std::max(p.M, 2));
+    p.db_bytes = 128 * dg.nrows;
+    const unsigned* wait_block = p.comm_wait ? p.comm_local : nullptr;
+    W4_CUDA(cudaLaunchKernelEx(&cfg, p.ln_w ? k_digits<true> : k_digits<false>, p.x, const_cast<uint8_t*>(p.dig), p.M, p.K, p.G,
+                               p.db_bytes, dg.tm, dg.cb, dg.tp, dg.sets, wait_block, p.comm_n, p.status, p.ln_w, p.ln_eps, p.xn_out));
+  }
+  return w->wbits == 4 ? launch_batch<4>(p, grid, st, di->smem_optin) : launch_batch<8>(p, grid, st, di->smem_optin);
+}
+
 int launch_skinny(SkinnyParams& p, const LayerRef* w, const uint16_t* x, int M, w4a16_scratch_t* s,
                   cudaStream_t st) {
   W4_REQUIRE(x != nullptr && (reinterpret_cast<uintptr_t>(x) & 15) == 0, "x null or not 16-byte aligned");
@@ -1722,7 +1747,6 @@ int launch_skinny(SkinnyParams& p, const LayerRef* w, const uint16_t* x, int M, 
   W4_REQUIRE(w->num_groups <= 256, "in_f = %d is wider than the decode kernel supports (32768)", w->in_f);
   const DeviceInfo* di = device_info();
   if (!di) return W4A16_ECUDA;
-  p.ordered = take_weight_write(st) ? 1 : 0;
   const int TR = tile_rows();
   p.stream = w->stream;
   p.N = w->out_f;
@@ -1755,30 +1779,14 @@ int launch_skinny(SkinnyParams& p, const LayerRef* w, const uint16_t* x, int M, 
     if (!(w->wbits == 4 ? gemv_cache_fits<4>(groups, di->smem_optin) : gemv_cache_fits<8>(groups, di->smem_optin)))
       return fail(W4A16_EINVAL, "in_f = %d is too wide for the decode kernel's activation cache", w->in_f);
   } else {
-    // the pre-pass: digit rows of all M tokens, once per call, into the scratch (behind the argmax pairs)
-    uint8_t* dig = reinterpret_cast<uint8_t*>(s->xf) + pair_bytes(s->max_splits);
-    p.dig = dig;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.ln_w ? M * ((p.G + 3) / 4) : (p.G * M + 3) / 4);
-    cfg.blockDim = dim3(128);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    // the first launch of the call carries the ordering behind a weight write; the main kernel may then overlap
-    // with this one as usual
-    cfg.numAttrs = (config().pdl && !p.ordered) ? 1 : 0;
-    p.ordered = 0;
-    const DigitGeometry dg = digit_geometry(std::max(M, 2));
-    p.db_bytes = 128 * dg.nrows;
-    const unsigned* wait_block = p.comm_wait ? p.comm_local : nullptr;
-    W4_CUDA(cudaLaunchKernelEx(&cfg, p.ln_w ? k_digits<true> : k_digits<false>, x, dig, M, p.K, p.G, p.db_bytes, dg.tm, dg.cb, dg.tp, dg.sets, wait_block, p.comm_n, p.status,
-                               p.ln_w, p.ln_eps, p.xn_out));
+    p.dig = reinterpret_cast<uint8_t*>(s->xf) + pair_bytes(s->max_splits);  // behind the argmax pairs
   }
-  if (int rc = w->wbits == 4 ? launch_batch<4>(p, grid, st, di->smem_optin) : launch_batch<8>(p, grid, st, di->smem_optin))
-    return rc;
-  return W4A16_OK;
+  // A refused call leaves the note of a weight write to the next one, and so does a launch that fails.
+  const bool behind_write = take_weight_write(st);
+  p.ordered = behind_write ? 1 : 0;
+  const int rc = enqueue_skinny(p, w, prepass, di, grid, st);
+  if (rc != W4A16_OK && behind_write) note_weight_write(st);
+  return rc;
 }
 
 }  // namespace
