@@ -1,4 +1,6 @@
 """Helpers shared by the GPU parity tests."""
+import ctypes as C
+
 import numpy as np
 import torch
 
@@ -45,3 +47,30 @@ class Guarded:
         es = self.raw.element_size()
         lo, hi = b[: self.band * es], b[(self.band + self.n) * es:]
         return bool((lo == 0x5A).all().item() and (hi == 0x5A).all().item())
+
+
+class _EdgeData(C.Structure):
+    _fields_ = [("from_port", C.c_ubyte), ("to_port", C.c_ubyte), ("type", C.c_ubyte), ("reserved", C.c_ubyte * 5)]
+
+
+def captured_edges(fn):
+    """Edge kinds, first to last, of the chain of nodes that `fn(stream)` captures
+    (CUgraphDependencyType: 0 full, 1 programmatic)."""
+    cuda = C.CDLL("libcuda.so.1")
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=stream):
+        fn(stream)
+    handle, n = C.c_void_p(graph.raw_cuda_graph()), C.c_size_t(0)
+    assert cuda.cuGraphGetEdges_v2(handle, None, None, None, C.byref(n)) == 0
+    if n.value == 0:
+        return []
+    src, dst, data = (C.c_void_p * n.value)(), (C.c_void_p * n.value)(), (_EdgeData * n.value)()
+    assert cuda.cuGraphGetEdges_v2(handle, src, dst, data, C.byref(n)) == 0
+    nxt = {src[i]: (dst[i], data[i].type) for i in range(n.value)}
+    assert len(nxt) == n.value, "not a chain"
+    node, kinds = next(iter(set(nxt) - {d for d, _ in nxt.values()})), []
+    while node in nxt:
+        node, kind = nxt[node]
+        kinds.append(kind)
+    return kinds

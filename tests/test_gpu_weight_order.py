@@ -3,40 +3,15 @@
 The matmul kernels read weights before they wait for the kernel in front of them, so a call straight behind a repack must be a
 fully ordered launch, whatever was refused in between, and any other call may be a programmatic one. The kind of ordering
 is read from captured graphs; the results are compared bit for bit with runs that synchronise after every call."""
-import ctypes as C
-
 import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
+from gpu_util import captured_edges  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
 FULL, PROGRAMMATIC = 0, 1  # CUgraphDependencyType
-
-
-class _EdgeData(C.Structure):
-    _fields_ = [("from_port", C.c_ubyte), ("to_port", C.c_ubyte), ("type", C.c_ubyte), ("reserved", C.c_ubyte * 5)]
-
-
-def _edges(fn):
-    """Edge kinds, first to last, of the chain of nodes that `fn(stream)` captures."""
-    cuda = C.CDLL("libcuda.so.1")
-    stream = torch.cuda.Stream()
-    graph = torch.cuda.CUDAGraph(keep_graph=True)
-    with torch.cuda.graph(graph, stream=stream):
-        fn(stream)
-    handle, n = C.c_void_p(graph.raw_cuda_graph()), C.c_size_t(0)
-    assert cuda.cuGraphGetEdges_v2(handle, None, None, None, C.byref(n)) == 0
-    src, dst, data = (C.c_void_p * n.value)(), (C.c_void_p * n.value)(), (_EdgeData * n.value)()
-    assert cuda.cuGraphGetEdges_v2(handle, src, dst, data, C.byref(n)) == 0
-    nxt = {src[i]: (dst[i], data[i].type) for i in range(n.value)}
-    assert len(nxt) == n.value, "not a chain"
-    node, kinds = next(iter(set(nxt) - {d for d, _ in nxt.values()})), []
-    while node in nxt:
-        node, kind = nxt[node]
-        kinds.append(kind)
-    return kinds
 
 
 def _tensors(synth, N, K, seed):
@@ -90,7 +65,7 @@ def test_first_matmul_behind_a_repack_is_fully_ordered(pkg, layer, name):
         fn(st)
 
     # inside the first call, into the repack, into the call behind it, and from there on
-    assert _edges(chain) == [PROGRAMMATIC] * (n - 1) + [FULL, FULL] + [PROGRAMMATIC] * (2 * n - 1)
+    assert captured_edges(chain) == [PROGRAMMATIC] * (n - 1) + [FULL, FULL] + [PROGRAMMATIC] * (2 * n - 1)
 
 
 @pytest.mark.parametrize("name", ["gemv", "skinny", "prefill"])
@@ -106,4 +81,98 @@ def test_refused_call_leaves_the_ordering_to_the_next(pkg, layer, name, why):
             refused[why](st)
         fn(st)
 
-    assert _edges(chain) == [FULL] + [PROGRAMMATIC] * (n - 1)
+    assert captured_edges(chain) == [FULL] + [PROGRAMMATIC] * (n - 1)
+
+
+def _steps(pkg, layers, ws, scratch, b, stream):
+    """Prefill and decode calls in which every call reads what the one in front of it wrote, or writes what it read."""
+    w0, w1, w2 = layers
+    T = b["a"].shape[0]
+
+    def prefill(dst, w, src):
+        return lambda: pkg.gemm_w4a16(b[dst], w, b[src], T, ws, stream=stream)
+
+    return [
+        prefill("b", w0, "a"), prefill("c", w1, "b"), prefill("d", w2, "c"),  # C of one as A of the next
+        prefill("c", w0, "d"), prefill("d", w1, "c"),                         # C over the A of the call in front
+        lambda: pkg.gemm_small_w4a16(b["y"], w0, b["d"], 9, scratch, stream=stream),
+        lambda: pkg.gemv_w4a16(b["d"][3], w1, b["y"][8], scratch, stream=stream),  # decode into a row that ...
+        prefill("a", w2, "d"), prefill("c", w0, "a"),                         # ... the prefill behind it reads
+        lambda: pkg.gemm_small_w4a16(b["a"], w1, b["c"], 16, scratch, stream=stream),
+        lambda: pkg.gemv_w4a16(b["z"], w2, b["a"][15], scratch, stream=stream),
+        prefill("d", w1, "a"),
+    ]
+
+
+# few tiles with K split over clusters and most SMs idle; more tokens; an odd number of row tiles
+@pytest.mark.parametrize("H,T", [(1024, 77), (1024, 300), (640, 19), (2176, 130)])
+def test_chained_prefill_and_decode_calls(pkg, synth, H, T):
+    layers = [pkg.awq_repack(*_tensors(synth, H, H, 20 + i)) for i in range(3)]
+    scratch, ws = pkg.gemv_scratch_alloc(H, H, 128, 16), pkg.gemm_workspace_alloc(4096)
+    gen = torch.Generator(device="cuda").manual_seed(H + T)
+    x = torch.randn((T, H), device="cuda", generator=gen).to(torch.bfloat16)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def buffers():
+        b = {n: torch.zeros((T, H), dtype=torch.bfloat16, device="cuda") for n in "abcdy"}
+        b["z"] = torch.zeros(H, dtype=torch.bfloat16, device="cuda")
+        b["a"].copy_(x)
+        torch.cuda.synchronize()
+        return b
+
+    def same(b):
+        return all(torch.equal(b[n].view(torch.int16), want[n].view(torch.int16)) for n in b)
+
+    want = buffers()
+    for step in _steps(pkg, layers, ws, scratch, want, stream):
+        step()
+        torch.cuda.synchronize()
+    assert all(bool(torch.isfinite(t.float()).all()) for t in want.values())
+    for _ in range(10):
+        b = buffers()
+        for step in _steps(pkg, layers, ws, scratch, b, stream):
+            step()
+        torch.cuda.synchronize()
+        assert same(b)
+    b, graph = buffers(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        b["a"].copy_(x)
+        for step in _steps(pkg, layers, ws, scratch, b, stream):
+            step()
+    for _ in range(5):
+        for n in b:
+            b[n].zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert same(b)
+    assert pkg.device_status() == 0
+    pkg.gemv_scratch_free(scratch)
+    pkg.gemm_workspace_free(ws)
+    for w in layers:
+        pkg.awq_free(w)
+
+
+@pytest.mark.parametrize("T", [19, 300])
+def test_prefill_right_behind_a_repack(pkg, synth, T):
+    """The same container overwritten with new weights and multiplied at once, with no synchronisation in between."""
+    H = 1024
+    sources = [_tensors(synth, H, H, 30 + i) for i in range(6)]
+    w, ws = pkg.awq_alloc_fused(H, H), pkg.gemm_workspace_alloc(4096)
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn((T, H), device="cuda", generator=gen).to(torch.bfloat16)
+    early, settled = torch.empty_like(x), torch.empty_like(x)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for src in sources:
+        pkg.gemm_w4a16(settled, w, x, T, ws, stream=stream)  # a prefill in front of the write, as well as behind it
+        pkg.awq_repack_into(w, 0, *src, stream=stream)
+        pkg.gemm_w4a16(early, w, x, T, ws, stream=stream)
+        torch.cuda.synchronize()
+        pkg.gemm_w4a16(settled, w, x, T, ws, stream=stream)
+        torch.cuda.synchronize()
+        assert torch.equal(early.view(torch.int16), settled.view(torch.int16))
+    assert pkg.device_status() == 0
+    pkg.gemm_workspace_free(ws)
+    pkg.awq_free(w)
