@@ -199,8 +199,9 @@ int w4a16_w8_lm_head_argmax(int32_t* ids, uint16_t* logits, void* pairs, int row
  *                      y = bf16(g / (1 + exp(-g)) * u) with g, u the bf16-rounded gate and up outputs.
  *   W4A16_EPILOGUE_RESIDUAL  residual_add (elementwise.cu:35-38, model.cu:777,785): y [M][out_f] is the running
  *                      hidden state, updated in place: y = bf16(float(y) + float(bf16(W x))).
- * The scratch must have been allocated with max_m >= 2 whenever ln_weight is given (the norm runs in the
- * pre-pass kernel that otherwise only serves M >= 2). */
+ * The scratch must have been allocated with max_m >= 2 whenever ln_weight is given. At M = 1 the norm runs inside the
+ * decode kernel; at M >= 2, and when y overlaps x, in the pre-pass kernel, which reads all of x before any of y is written.
+ * So y may overlap x, with or without the norm and in the other calls of M <= 16 too. */
 #define W4A16_EPILOGUE_NONE 0
 #define W4A16_EPILOGUE_SWIGLU 1
 #define W4A16_EPILOGUE_RESIDUAL 2

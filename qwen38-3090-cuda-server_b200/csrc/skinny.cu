@@ -1769,10 +1769,10 @@ int launch_skinny(SkinnyParams& p, const LayerRef* w, const uint16_t* x, int M, 
   if ((M >= 2 || p.ln_w != nullptr) && (M > (s->max_m >= 2 ? s->max_m : 0) || p.G > s->max_groups))
     return fail(W4A16_ESCRATCH, "scratch: sized for max_m = %d and in_f <= %d, got M = %d, in_f = %d", s->max_m,
                 s->max_groups * kGroup, M, w->in_f);
-  // M = 1 converts (and normalises) x inside the decode kernel, while other CTAs may already be storing y. A normalised call whose
-  // y overlaps x (the residual added in place) takes the pre-pass, which has read all of x by then, and the two-token instance.
+  // M = 1 converts (and normalises) x inside the decode kernel, while other CTAs may already be storing y. A call whose y
+  // overlaps x (the residual added in place) takes the pre-pass, which has read all of x by then, and the two-token instance.
   const char *xb = reinterpret_cast<const char*>(x), *yb = static_cast<const char*>(p.y);
-  const bool in_place = p.ln_w != nullptr && yb != nullptr && yb < xb + 2LL * M * p.K && xb < yb + 2LL * M * p.ldy;
+  const bool in_place = yb != nullptr && yb < xb + 2LL * M * p.K && xb < yb + (p.y_f32 ? 4LL : 2LL) * M * p.ldy;
   const bool prepass = M >= 2 || in_place;
   if (!prepass) {
     const int groups = cache_groups_for(p.tiles, p.G, grid);
@@ -1780,6 +1780,14 @@ int launch_skinny(SkinnyParams& p, const LayerRef* w, const uint16_t* x, int M, 
       return fail(W4A16_EINVAL, "in_f = %d is too wide for the decode kernel's activation cache", w->in_f);
   } else {
     p.dig = reinterpret_cast<uint8_t*>(s->xf) + pair_bytes(s->max_splits);  // behind the argmax pairs
+    if (s->max_m < 2 || p.G > s->max_groups) {
+      // a plain M = 1 call in place, with a scratch that has no room for a pre-pass: the second half of the pieces'
+      // buffer, which is sized for twice the CTAs of the grid
+      const size_t half = s->partial_elems / 2 * sizeof(float);
+      if (half < prepass_bytes(p.G) || half < static_cast<size_t>(grid) * 2 * kTileRows * 2 * sizeof(unsigned long long))
+        return fail(W4A16_ESCRATCH, "scratch: partial buffer holds %zu floats, too few for a call in place", s->partial_elems);
+      p.dig = reinterpret_cast<uint8_t*>(s->partial) + half;
+    }
   }
   // A refused call leaves the note of a weight write to the next one, and so does a launch that fails.
   const bool behind_write = take_weight_write(st);

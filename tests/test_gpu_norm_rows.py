@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
-from gpu_util import host_bits  # noqa: E402
+from gpu_util import captured_edges, host_bits  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -109,5 +109,47 @@ def test_normalised_call_that_adds_to_its_own_input(pkg, synth, M):
     pkg.linear_fused(own, w, own, M, scratch, ln_weight=ln, epilogue=pkg.EPILOGUE_RESIDUAL)
     assert torch.equal(apart.view(torch.int16), own.view(torch.int16)) and not torch.equal(own, x)
     assert pkg.device_status() == 0
+    pkg.gemv_scratch_free(scratch)
+    pkg.awq_free(w)
+
+
+@pytest.mark.parametrize("max_m", [1, 16])
+@pytest.mark.parametrize("H", [128, 1152, 5120])
+def test_plain_calls_whose_output_overlaps_the_input(pkg, synth, H, max_m):
+    """The same for calls without a norm at M = 1, whatever the scratch has room for: a pre-pass kernel reads x first."""
+    w = pkg.weights_from_numpy(*synth.make_weights(H, H, seed=6))
+    scratch = pkg.gemv_scratch_alloc(H, H, 128, max_m)
+    gen = torch.Generator(device="cuda").manual_seed(H)
+    x = torch.randn(H, device="cuda", generator=gen).to(torch.bfloat16)
+    plain, res, wide = torch.empty_like(x), x.clone(), torch.empty(H, device="cuda")
+    torch.cuda.synchronize()
+    pkg.gemv_w4a16(plain, w, x, scratch)
+    pkg.gemv_w4a16_f32(wide, w, x, scratch)
+    pkg.linear_fused(res, w, x, 1, scratch, epilogue=pkg.EPILOGUE_RESIDUAL)
+    own = torch.zeros(2 * H, device="cuda", dtype=torch.bfloat16)  # x lies in the second half, which a y of 32 bits reaches
+    xo = own[H:]
+
+    def gemv(st):
+        pkg.gemv_w4a16(xo, w, xo, scratch, stream=st)
+
+    def gemv_static(st):
+        pkg.gemv_w4a16_static(xo, w, xo, stream=st)
+
+    def gemv_f32(st):
+        pkg.gemv_w4a16_f32(own.view(torch.float32), w, xo, scratch, stream=st)
+
+    def residual(st):
+        pkg.linear_fused(xo, w, xo, 1, scratch, epilogue=pkg.EPILOGUE_RESIDUAL, stream=st)
+
+    for call, got, want in ((gemv, xo, plain), (gemv_static, xo, plain), (gemv_f32, own.view(torch.float32), wide), (residual, xo, res)):
+        xo.copy_(x)
+        call(torch.cuda.current_stream())
+        assert torch.equal(got.view(torch.int16), want.view(torch.int16)), call.__name__
+        assert len(captured_edges(call)) == 1  # two kernels
+    assert len(captured_edges(lambda st: pkg.gemv_w4a16(plain, w, x, scratch, stream=st))) == 0
+    pkg.gemv_w4a16(plain, w, x, scratch)  # the scratch serves an ordinary call as before
+    xo.copy_(x)
+    gemv(torch.cuda.current_stream())
+    assert torch.equal(xo, plain) and pkg.device_status() == 0
     pkg.gemv_scratch_free(scratch)
     pkg.awq_free(w)
