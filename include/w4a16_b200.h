@@ -193,7 +193,8 @@ int w4a16_w8_lm_head_argmax(int32_t* ids, uint16_t* logits, void* pairs, int row
 /* A linear layer (M <= 16 tokens) with its elementwise neighbours fused in; every part is optional:
  *   ln_weight != NULL  RMSNorm in front (src/kernels/elementwise.cu:8-33, called at src/model/model.cu:681,774):
  *                      xn = bf16(x * rsqrt(mean(x^2) + ln_eps) * (1 + ln_weight)), the layer multiplies xn;
- *                      xn_out (may be NULL) receives xn [M][in_f] for callers that need it elsewhere.
+ *                      xn_out (may be NULL) receives xn [M][in_f] for callers that need it elsewhere;
+ *                      it must not overlap x (W4A16_EINVAL): rows are still read while others are stored.
  *   W4A16_EPILOGUE_SWIGLU    swiglu (elementwise.cu:40-49, model.cu:781): the weights hold gate and up rows
  *                      INTERLEAVED (w4a16_repack_into_swiglu), y is [M][out_f / 2]:
  *                      y = bf16(g / (1 + exp(-g)) * u) with g, u the bf16-rounded gate and up outputs.

@@ -1893,7 +1893,13 @@ int run_fused(uint16_t* y, const W* w, const uint16_t* x, int M, const Fusion& f
   p.ln_eps = f.ln_eps;
   p.xn_out = f.xn_out;
   p.epilogue = f.epilogue;
-  if (f.ln_w) W4_REQUIRE((reinterpret_cast<uintptr_t>(f.ln_w) & 7) == 0, "fused linear: norm weights not 8-byte aligned");
+  if (f.ln_w) {
+    W4_REQUIRE((reinterpret_cast<uintptr_t>(f.ln_w) & 7) == 0, "fused linear: norm weights not 8-byte aligned");
+    // every CTA sums a token's whole row, with no order between one that still reads x and one that already stores xn
+    const char *xb = reinterpret_cast<const char*>(x), *nb = reinterpret_cast<const char*>(f.xn_out);
+    const long long bytes = 2LL * M * L.in_f;
+    W4_REQUIRE(nb == nullptr || nb >= xb + bytes || xb >= nb + bytes, "fused linear: xn_out overlaps x");
+  }
   if (f.epilogue == kEpiSwiglu) {
     W4_REQUIRE(L.out_f % 32 == 0, "swiglu epilogue: out_f %d must be a multiple of 32 (gate, up interleaved)", L.out_f);
     p.ldy = L.out_f / 2;

@@ -153,3 +153,25 @@ def test_plain_calls_whose_output_overlaps_the_input(pkg, synth, H, max_m):
     assert torch.equal(xo, plain) and pkg.device_status() == 0
     pkg.gemv_scratch_free(scratch)
     pkg.awq_free(w)
+
+
+@pytest.mark.parametrize("M", [1, 3])
+def test_normalised_rows_must_not_go_over_the_input(pkg, synth, M):
+    H = 1024
+    w = pkg.weights_from_numpy(*synth.make_weights(H, H, seed=7))
+    scratch = pkg.gemv_scratch_alloc(H, H, 128, 16)
+    buf = torch.randn(3 * M * H, device="cuda").to(torch.bfloat16)
+    x, ln, y = buf[M * H:2 * M * H], torch.zeros(H, device="cuda", dtype=torch.bfloat16), torch.empty((M, H), device="cuda", dtype=torch.bfloat16)
+    before = buf.clone()
+    for at in (M * H, 8, 2 * M * H - 8):  # x itself, and one step of 16 bytes into either end
+        with pytest.raises(pkg.W4A16Error, match="overlaps"):
+            pkg.linear_fused(y, w, x, M, scratch, ln_weight=ln, xn_out=buf[at:at + M * H])
+    assert torch.equal(buf, before)
+    pkg.linear_fused(y, w, x, M, scratch, xn_out=x)  # without the norm nothing is stored there
+    for at in (0, 2 * M * H):  # right in front of x and right behind it
+        xn = buf[at:at + M * H]
+        pkg.linear_fused(y, w, x, M, scratch, ln_weight=ln, xn_out=xn)
+        assert torch.equal(x, before[M * H:2 * M * H]) and not torch.equal(xn, before[at:at + M * H])
+    assert pkg.device_status() == 0
+    pkg.gemv_scratch_free(scratch)
+    pkg.awq_free(w)
