@@ -1390,7 +1390,7 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
   if (COMM && p.comm_signal && !p.argmax && tid == 0) signal_cta_done(p.comm_local, p.comm_peers, p.comm_n, p.comm_rank);
 }
 
-// Pre-pass of the M >= 2 calls: one warp per (k group, token) turns the token's 128 bf16 values of the
+// Pre-pass of the M >= 2 calls, and of M = 1 calls whose output overlaps their input: one warp per (k group, token) turns the token's 128 bf16 values of the
 // group into three digit rows of the B operand, their sum and the scale 2^-p, laid out as the main kernel of this M
 // reads them: per group [8 chunks of 16 k][N rows] 16 B (N = 16, 32 or 48, a token set's rows in its own column block of `cb`;
 // db_bytes in all), and behind all groups' rows, per group and token set, `tp` sums and then `tp` scales. Small CTAs
@@ -1589,6 +1589,8 @@ int launch_cfg(SkinnyParams& p, int grid, cudaStream_t st, int smem_optin) {
   // an mbarrier only tells the current phase from the previous one: with an odd depth a stage's consecutive
   // uses would belong to different warps, and a warp that runs ahead could take "the other warp's copy has
   // not landed yet" for "my copy has landed".
+  // (Int8 weights with more than 30 groups per CTA get four stages, as at M = 2..4; six, where a smaller side ring let them fit,
+  // were slower: head 248320 x 5120 188.8 us against 182.1 at M = 1, 197.6 against 187.7 at M = 4.)
   p.depth = config().depth;
   int smem = total_smem<MT, WB, NORM>(p.depth, kStageBytes, p.b_bytes, p.xs_bytes, 0);
   while (smem > limit && p.depth > 2) {
