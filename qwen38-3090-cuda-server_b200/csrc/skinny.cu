@@ -190,7 +190,6 @@ struct SkinnyParams {
   int bdepth;        // M >= 2: steps in the digit ring (a power of two)
   int bshift;        //         and its log2
   unsigned long long mg_grid, mg_G;  // ceil(2^40 / d) for d = gridDim.x and G: exact division by multiply
-  uint32_t hint;     // suspend-time hint of the mbarrier waits, ns
   int depth;         // weight ring stages
   float* partial;
   unsigned* counters;  // [tiles * CW + 1], zero between launches
@@ -311,12 +310,6 @@ __device__ __forceinline__ uint32_t step_word(int slot0, int slot1, int ng, bool
 }
 
 // ---- PTX used only here ------------------------------------------------------------------
-// Bounded wait with a per-launch suspend hint: how long one try_wait may park the thread.
-__device__ __forceinline__ bool wait_h(uint32_t bar, uint32_t parity, uint32_t hint_ns, uint32_t limit) {
-  for (uint32_t i = 0; i < limit; ++i)
-    if (mbar_try_wait(bar, parity, hint_ns)) return true;
-  return false;
-}
 // Instruction descriptor for kind::i8: signed 8-bit A and B (both K-major), int32 accumulate.
 __host__ __device__ constexpr uint32_t umma_idesc_s8(int M, int N) {
   return (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(N >> 3) << 17) |
@@ -603,7 +596,7 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
           mbar_arrive(commrdy_a);
         }
         __syncwarp();
-      } else if (!wait_h(commrdy_a, 0, p.hint, 4 * kSpinLimit)) {
+      } else if (!mbar_wait_bounded(commrdy_a, 0, 4 * kSpinLimit)) {
         atomicExch(p.status, W4A16_ETIMEOUT);
       }
     }
@@ -702,7 +695,7 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
   constexpr uint32_t tmem = 0;
   const bool uses_tmem = warp < kWProducer || warp == kWMma || warp == kWMma2 || warp >= kWConv0;
   if (uses_tmem) {
-    if (!warp_agrees(wait_h(tmemrdy_a, 0, p.hint, kSpinLimit)) || *reinterpret_cast<volatile uint32_t*>(tmem_slot) != 0u) {
+    if (!warp_agrees(mbar_wait_bounded(tmemrdy_a, 0, kSpinLimit)) || *reinterpret_cast<volatile uint32_t*>(tmem_slot) != 0u) {
       atomicExch(p.status, W4A16_ETIMEOUT);
       team_ok = false;
     }
@@ -767,16 +760,16 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
         const int a = t & (AD2 - 1), d = t & (DD2 - 1);
         // A written (its writers also saw the step's weights and table entry landed), and the D slot this
         // step fills has been read out by every fix-up warp
-        if (!warp_agrees(wait_h(afull_a + a * 8, static_cast<uint32_t>(t / AD2) & 1u, p.hint, kSpinLimit) &&
+        if (!warp_agrees(mbar_wait_bounded(afull_a + a * 8, static_cast<uint32_t>(t / AD2) & 1u, kSpinLimit) &&
                          (!GE::kIssuerWaitsD || t < DD2 ||
-                          wait_h(dempty_a + d * 8, static_cast<uint32_t>(t / DD2 - 1) & 1u, p.hint, kSpinLimit)))) {
+                          mbar_wait_bounded(dempty_a + d * 8, static_cast<uint32_t>(t / DD2 - 1) & 1u, kSpinLimit)))) {
           atomicExch(p.status, W4A16_ETIMEOUT);
           break;
         }
         const uint32_t e = table[t & (kTable - 1)].x;
         if constexpr (kStream) {
           // the step's digit rows have landed in their ring slot (bulk copy: async proxy, as the MMA reads them)
-          if (!warp_agrees(wait_h(bfull_a + (t & (BD - 1)) * 8, static_cast<uint32_t>(t >> BS) & 1u, p.hint, kSpinLimit))) {
+          if (!warp_agrees(mbar_wait_bounded(bfull_a + (t & (BD - 1)) * 8, static_cast<uint32_t>(t >> BS) & 1u, kSpinLimit))) {
             atomicExch(p.status, W4A16_ETIMEOUT);
             break;
           }
@@ -794,7 +787,7 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
             break;
           }
           __threadfence_block();
-          all_ready = mbar_try_wait(bready_a, 0, 0);
+          all_ready = mbar_test_wait(bready_a, 0);
         }
         tc_fence_after();
         const uint32_t d_t = tmem + GE::kDCol0 + d * GE::kDColsS;
@@ -830,7 +823,7 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
     bool ok = team_ok;
     for (int t = pair; ok && t < T; t += 2) {
       const int a = t & (AD2 - 1);
-      if (!warp_agrees(wait_h(wfull_a + st * 8, wph, p.hint, kSpinLimit))) {
+      if (!warp_agrees(mbar_wait_bounded(wfull_a + st * 8, wph, kSpinLimit))) {
         atomicExch(p.status, W4A16_ETIMEOUT);
         break;
       }
@@ -852,10 +845,10 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
       load_row(base);
       // the A slot's previous step has been multiplied (whether the D slot is free is the issuer's concern: the
       // operand can be unpacked while the fix-up warps are still reading the sums of DD2 steps ago)
-      if (!warp_agrees((t < AD2 || wait_h(done_a + ((t - AD2) & (ND - 1)) * 8, static_cast<uint32_t>((t - AD2) / ND) & 1u,
-                                          p.hint, kSpinLimit)) &&
+      if (!warp_agrees((t < AD2 || mbar_wait_bounded(done_a + ((t - AD2) & (ND - 1)) * 8, static_cast<uint32_t>((t - AD2) / ND) & 1u,
+                                          kSpinLimit)) &&
                        (GE::kIssuerWaitsD || t < DD2 ||
-                        wait_h(dempty_a + (t & (DD2 - 1)) * 8, static_cast<uint32_t>(t / DD2 - 1) & 1u, p.hint, kSpinLimit)))) {
+                        mbar_wait_bounded(dempty_a + (t & (DD2 - 1)) * 8, static_cast<uint32_t>(t / DD2 - 1) & 1u, kSpinLimit)))) {
         atomicExch(p.status, W4A16_ETIMEOUT);
         break;
       }
@@ -1031,7 +1024,7 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
     const float2* xs_tab = reinterpret_cast<const float2*>(xsinv);  // M = 1: (sum, 2^-p) per cache slot
     if constexpr (kStream) {
       // the pair table of the call arrives once, by bulk copy
-      if (!warp_agrees(wait_h(bready_a, 0, p.hint, kSpinLimit))) {
+      if (!warp_agrees(mbar_wait_bounded(bready_a, 0, kSpinLimit))) {
         atomicExch(p.status, W4A16_ETIMEOUT);
         ok = false;
       }
@@ -1043,7 +1036,7 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
       int seg_tile = 0;
       if (helper) {
         const float* mslot = mail + (nmail * CW + q) * kMailStride;
-        if (!warp_agrees(wait_h(mailfull_a + (nmail * CW + q) * 8, 0, p.hint, 4 * kSpinLimit))) {
+        if (!warp_agrees(mbar_wait_bounded(mailfull_a + (nmail * CW + q) * 8, 0, 4 * kSpinLimit))) {
           atomicExch(p.status, W4A16_ETIMEOUT);
           break;
         }
@@ -1053,14 +1046,14 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
       } else {
       // A round is one or (M = 1) two steps (two unless the first ends its segment): one wait per issuer (a commit
       // covers everything its thread issued before), GB groups' tensor-memory loads in flight together.
-      if (!warp_agrees(wait_h(done_a + (t & (ND - 1)) * 8, static_cast<uint32_t>(t / ND) & 1u, p.hint, kSpinLimit))) {
+      if (!warp_agrees(mbar_wait_bounded(done_a + (t & (ND - 1)) * 8, static_cast<uint32_t>(t / ND) & 1u, kSpinLimit))) {
         atomicExch(p.status, W4A16_ETIMEOUT);
         ok = false;
         break;
       }
       const uint2 e0 = table[t & (kTable - 1)];  // written before the step's weights were requested
       const bool two = GE::kPairRounds && !((e0.x >> 17) & 1u) && t + 1 < T;
-      if (two && !warp_agrees(wait_h(done_a + ((t + 1) & (ND - 1)) * 8, static_cast<uint32_t>((t + 1) / ND) & 1u, p.hint, kSpinLimit))) {
+      if (two && !warp_agrees(mbar_wait_bounded(done_a + ((t + 1) & (ND - 1)) * 8, static_cast<uint32_t>((t + 1) / ND) & 1u, kSpinLimit))) {
         atomicExch(p.status, W4A16_ETIMEOUT);
         ok = false;
         break;
@@ -1504,16 +1497,13 @@ __global__ void k_pairs_reduce(int32_t* ids, const Pair* pairs, int nranks, int 
 struct Config {
   int depth;     // weight ring stages (two blocks, 17152 B, each); even
   int pdl;
-  int hint;      // suspend-time hint of the in-kernel mbarrier waits, ns
 };
 
 const Config& config() {
   static Config c = [] {
-    Config k{6, 1, 2000};
+    Config k{6, 1};
     if (const char* e = getenv("W4A16_DEPTH")) k.depth = atoi(e);
     if (const char* e = getenv("W4A16_PDL")) k.pdl = atoi(e) != 0;
-    if (const char* e = getenv("W4A16_HINT")) k.hint = atoi(e);
-    if (k.hint < 0) k.hint = 0;
     if (k.depth < 2) k.depth = 2;
     if (k.depth > 12) k.depth = 12;
     k.depth &= ~1;  // even: see the ring-depth note in launch_cfg
@@ -1759,7 +1749,6 @@ int launch_skinny(SkinnyParams& p, const LayerRef* w, const uint16_t* x, int M, 
   p.counters = reinterpret_cast<unsigned*>(s->xgsum);
   p.cta_pairs = s->xf;
   p.status = di->status;
-  p.hint = static_cast<uint32_t>(config().hint);
   const int grid = grid_for_shape(w->out_f, w->num_groups, di->sms);
   W4_REQUIRE(static_cast<long long>(p.tiles) * p.G * (grid + 1) < (1LL << 32), "out_f x in_f too large for the decode kernel");
   auto magic = [](long long d) { return static_cast<unsigned long long>(((1LL << 40) + d - 1) / d); };
