@@ -1220,31 +1220,34 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
               }
             }
             last = true;
-            constexpr int PB = TM <= 2 ? 4 : (TM <= 4 ? 2 : 1);  // pieces whose loads are in flight together
+            // A batch's loads are straight-line code, so that all of them are in flight together: what would be a token past M or
+            // a piece past the last reads the last one's words again. (Under a test each, every load waited for the one before:
+            // from the last sums to the end of a 5120 x 6144 launch 1.1 us at M = 2, 3.2 us at M = 4. Launches of 5120 x 6144 /
+            // 5120 x 17408 / 34816 x 5120 in us, before -> after: M = 1 6.17 / 10.57 / 16.63 -> 6.04 / 10.41 / 16.48, M = 4 8.84 / 13.65 /
+            // 18.56 -> 6.91 / 11.36 / 18.42, M = 9 9.05 / 16.08 / 22.58 -> 8.48 / 15.34 / 22.12, M = 12 at 5120 x 6144 10.54 -> 9.48.)
+            constexpr int PB = TM <= 2 ? 4 : (MT == 9 ? 2 : 1);  // pieces per batch: what fits the registers without spills
             for (int cb = c_first + 1; cb <= c_last && ok; cb += PB) {
               unsigned long long piece[PB][TM];
-              const unsigned long long* sl[PB];
+              unsigned long long* sl[PB];
 #pragma unroll
               for (int k = 0; k < PB; ++k) {
-                const int cc = cb + k <= c_last ? cb + k : c_last;
+                const int cc = min(cb + k, c_last);
                 const uint32_t cu0 = fdiv(Uu * static_cast<uint32_t>(cc), p.mg_grid);
                 const int wc = (static_cast<int>(fdiv(cu0, p.mg_G)) == tile) ? 0 : 1;
                 sl[k] = slots + (static_cast<size_t>(cc) * 2 + wc) * SLOT + r;
               }
               uint32_t spins = 0;
               for (;;) {
-                bool all = true;
 #pragma unroll
                 for (int k = 0; k < PB; ++k)
-                  if (cb + k <= c_last) {
 #pragma unroll
-                    for (int i = 0; i < TM; ++i)
-                      if (m0 + i < M) {
-                        piece[k][i] = ld_relaxed_gpu_u64(sl[k] + (m0 + i) * kTileRows);
-                        all = all && static_cast<uint32_t>(piece[k][i] >> 32) == kPieceTag;
-                      }
-                  }
-                if (__all_sync(0xffffffffu, all)) break;
+                  for (int i = 0; i < TM; ++i) piece[k][i] = ld_relaxed_gpu_u64(sl[k] + min(m0 + i, M - 1) * kTileRows);
+                uint32_t differ = 0;
+#pragma unroll
+                for (int k = 0; k < PB; ++k)
+#pragma unroll
+                  for (int i = 0; i < TM; ++i) differ |= static_cast<uint32_t>(piece[k][i] >> 32) ^ kPieceTag;
+                if (__all_sync(0xffffffffu, differ == 0u)) break;
                 if (++spins > kSpinLimit) {
                   atomicExch(p.status, W4A16_ETIMEOUT);
                   ok = false;
@@ -1255,11 +1258,10 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
               for (int k = 0; k < PB; ++k)
                 if (cb + k <= c_last) {
 #pragma unroll
-                  for (int i = 0; i < TM; ++i)
-                    if (m0 + i < M) {
-                      v[i] += __uint_as_float(static_cast<uint32_t>(piece[k][i]));
-                      st_relaxed_gpu_u64(const_cast<unsigned long long*>(sl[k]) + (m0 + i) * kTileRows, 0ull);
-                    }
+                  for (int i = 0; i < TM; ++i) {
+                    v[i] += __uint_as_float(static_cast<uint32_t>(piece[k][i]));
+                    if (m0 + i < M) st_relaxed_gpu_u64(sl[k] + (m0 + i) * kTileRows, 0ull);
+                  }
                 }
             }
           }
