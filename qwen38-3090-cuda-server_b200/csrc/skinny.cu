@@ -134,12 +134,17 @@ struct Geo {
     if (WB == 4 && MT == 15) return 1024;
     return WB == 4 && MT == 6 ? 896 : kThreads;
   }
-  // int32 -> fp32 of the sums by the conversion instruction (exact below 2^24, the same floats) instead of an integer add of a magic
-  // constant and a packed subtraction: fewer instructions, on a slower pipe. 34816 x 5120 / 5120 x 17408 / 16384 x 5120 / 5120 x 6144 in us, magic -> conversion:
-  //   M = 6 (72 registers) 20.7 / 13.6 / 12.3 / 8.4 -> 20.1 / 13.2 / 12.0 / 8.2    M = 8 22.2 / 14.6 / 13.1 / 9.4 -> 21.2 / 14.1 / 12.6 / 9.1
-  //   M = 9  23.3 / 16.2 / 13.7 / 9.3 -> 24.2 / 17.1 / 14.6 / 10.1                 M = 12 25.6 / 18.3 / 15.3 / 11.5 -> 26.0 / 19.4 / 15.8 / 12.1
-  //   M = 16 28.5 / 19.3 / 16.0 / 11.3 -> 27.5 / 19.3 / 16.0 / 11.5                M = 4 the same
-  static constexpr bool kConvert = MT == 6 || MT == 8 || MT == 16;
+  // How the three digits' int32 sums become D0 + 2^8 D1 + 2^16 D2 in fp32. Either all three by adding a magic constant as integers
+  // and taking it off again in packed fp32 (nine instructions for two tokens' sums, then two packed FMAs), or, kJoin, 256 D1 + D0 as an integer
+  // (below 2^30) and one conversion: fmaf(d1, 256, d0) of exact floats rounds the same number the same way, so the bits are
+  // the same. The conversion instruction is on a slower pipe, which is why it does not pay everywhere; kTopConvert: D2 by
+  // it as well. 34816 x 5120 / 16384 x 5120 / 5120 x 6144 in us, magic (M = 6, 8, 16: three conversions) -> now:
+  //   M = 4  18.40 /   -   /  6.91 -> 18.29 /   -   /  6.81    M = 6  19.15 / 11.48 / 7.86 -> 18.77 / 11.28 / 7.78
+  //   M = 8  20.37 / 12.24 /  8.26 -> 19.38 / 11.67 /  8.08    M = 15 26.26 / 15.17 / 10.16 -> 24.41 / 14.61 / 10.17
+  //   M = 16 26.43 / 15.46 / 10.27 -> 25.84 / 15.17 / 10.24
+  // and where it was not taken, magic -> kJoin: M = 9 22.14 / 12.98 / 8.57 -> 22.65 / 13.38 / 8.78, M = 12 23.98 / 14.08 / 9.42 -> 23.53 / 14.24 / 9.58.
+  static constexpr bool kJoin = MT == 4 || MT == 6 || MT == 8 || MT == 15 || MT == 16;
+  static constexpr bool kTopConvert = MT == 6 || MT == 16;
   static constexpr int N = !kStream ? 16 : ((FW * CB + 15) / 16) * 16;  // rows of the B operand the tensor core reads
   static constexpr int AD2 = N == 48 ? 2 : 4;
   static constexpr int DD2 = N == 16 ? 8 : 4;
@@ -1136,23 +1141,24 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
           for (int i = 0; i + 1 < TM; i += 2) {
             const unsigned long long sum2 = *reinterpret_cast<const unsigned long long*>(xs_g + i);
             const unsigned long long inv2 = *reinterpret_cast<const unsigned long long*>(xs_g + GE::TP + i);
-            auto to_float = [&](uint32_t lo, uint32_t hi) {
-              return GE::kConvert ? pack_f32x2(__int2float_rn(static_cast<int>(lo)), __int2float_rn(static_cast<int>(hi)))
-                                  : add_f32x2(magic_pair(lo, hi), off2);
+            auto by_instr = [](uint32_t lo, uint32_t hi) {
+              return pack_f32x2(__int2float_rn(static_cast<int>(lo)), __int2float_rn(static_cast<int>(hi)));
             };
-            const unsigned long long d0 = to_float(d[3 * i], d[3 * i + 3]);
-            const unsigned long long d1 = to_float(d[3 * i + 1], d[3 * i + 4]);
-            const unsigned long long d2 = to_float(d[3 * i + 2], d[3 * i + 5]);
-            const unsigned long long dot = fma_f32x2(d2, k16, fma_f32x2(d1, k8, d0));
+            auto by_magic = [&](uint32_t lo, uint32_t hi) { return add_f32x2(magic_pair(lo, hi), off2); };
+            unsigned long long low, top;
+            if constexpr (GE::kJoin) low = by_instr(d[3 * i + 1] * 256u + d[3 * i], d[3 * i + 4] * 256u + d[3 * i + 3]);
+            else low = fma_f32x2(by_magic(d[3 * i + 1], d[3 * i + 4]), k8, by_magic(d[3 * i], d[3 * i + 3]));
+            if constexpr (GE::kTopConvert) top = by_instr(d[3 * i + 2], d[3 * i + 5]);
+            else top = by_magic(d[3 * i + 2], d[3 * i + 5]);
+            const unsigned long long dot = fma_f32x2(top, k16, low);
             const unsigned long long acc = fma_f32x2(mul_f32x2(s2, inv2), fma_f32x2(nz2, sum2, dot), pack_f32x2(fin[i], fin[i + 1]));
             unpack_f32x2(acc, fin[i], fin[i + 1]);
           }
           if constexpr (TM & 1) {
             constexpr int i = TM - 1;
-            const float d0 = small_int_to_float(d[3 * i]);
-            const float d1 = small_int_to_float(d[3 * i + 1]);
-            const float d2 = small_int_to_float(d[3 * i + 2]);
-            const float dot = fmaf(d2, 65536.f, fmaf(d1, 256.f, d0));
+            const float low = GE::kJoin ? __int2float_rn(static_cast<int>(d[3 * i + 1] * 256u + d[3 * i]))
+                                        : fmaf(small_int_to_float(d[3 * i + 1]), 256.f, small_int_to_float(d[3 * i]));
+            const float dot = fmaf(small_int_to_float(d[3 * i + 2]), 65536.f, low);
             fin[i] = fmaf(s * xs_g[GE::TP + i], fmaf(-z, xs_g[i], dot), fin[i]);
           }
         };
