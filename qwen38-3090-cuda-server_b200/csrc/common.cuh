@@ -175,6 +175,13 @@ __device__ __forceinline__ bool mbar_wait_bounded_relaxed(uint32_t bar, uint32_t
 // they have to agree. A warp that gave up sets the status word, does no more work and still reaches every barrier
 // that other warps wait at.
 __device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok); }
+// A warp's wait on two barriers at once: the tests are in flight together, so that barriers that have completed cost one
+// test's latency and not the sum.
+__device__ __forceinline__ bool warp_waits(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t limit) {
+  const bool r0 = mbar_try_wait(b0, p0), r1 = mbar_try_wait(b1, p1);
+  if (warp_agrees(r0 & r1)) return true;
+  return warp_agrees((r0 || mbar_wait_bounded(b0, p0, limit)) && (r1 || mbar_wait_bounded(b1, p1, limit)));
+}
 // 1-D bulk async copy global -> this CTA's shared memory, completion on an mbarrier.
 // dst, src 16-byte aligned; bytes a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes,

@@ -11,8 +11,8 @@
 //     group stages of activations instead of two;
 //   * a producer thread per CTA streams the packed int4 blocks of its row tile through a ring of
 //     shared-memory stages with 1-D bulk async copies (cp.async.bulk + mbarrier);
-//   * sixteen dequant warps per CTA (one output row and half a k group per thread; two teams take alternate
-//     groups) turn 32 bytes of nibbles into bf16 weights in registers - (128+q) by LOP3,
+//   * sixteen dequant warps per CTA (one output row per thread; four teams take the k groups in
+//     turn) turn 64 bytes of nibbles into bf16 weights in registers - (128+q) by LOP3,
 //     minus (128+zp) and times the group scale with packed bf16 arithmetic, which is exactly
 //     bf16(float(q-zp)*float(s)), the value w4a16_dequant_rows produces - and store them as the A operand
 //     into tensor memory (tcgen05.st);
@@ -48,7 +48,7 @@
 namespace w4a16 {
 namespace {
 
-constexpr int PW = 16;                      // dequant warps: 4 TMEM lane quarters x 2 halves of a k group x 2 groups
+constexpr int PW = 16;                      // dequant warps: 4 TMEM lane quarters x 4 groups
 constexpr int EW = 8;                       // epilogue warps: two per lane quarter, each half of the tokens
 constexpr int kWEpi0 = PW, kWWeights = PW + EW, kWIssue = kWWeights + 1, kWActs = kWIssue + 1;
 constexpr int kPWarps = kWActs + 1;
@@ -61,6 +61,7 @@ constexpr int kPMaxWD = 16;                 // weight ring stages (one k group e
 constexpr uint32_t kPTmemCols = 512;
 constexpr uint32_t kPSpin = 1u << 20;
 constexpr uint32_t kMagicP = 0x43004300u, kNibMaskP = 0x000F000Fu;
+constexpr int kPTeams = 4;                  // teams of dequant warps
 constexpr int kPMaxA = 6;                   // A slots, at most
 constexpr int kPBars = 2 * kPMaxWD + kPDone + kPMaxA + kPSteps + 2;
 // Tensor memory: the accumulator's TN columns, the rest are slots of the A operand, 64 columns per k group.
@@ -72,7 +73,7 @@ struct PrefillParams {
   const uint8_t* stream;
   uint16_t* C;        // [M][ldc] bf16; this launch's rows land in columns [col0, col0 + N)
   int M, N, K, G, row_tiles, pairs;  // pairs: row tiles in twos (an odd last one repeats the last tile and stores nothing)
-  int tn, splits, wdepth;            // wdepth is even: a stage is always read by the same dequant warps
+  int tn, splits, wdepth;            // wdepth is a multiple of four: a stage is always read by the same dequant warps
   int full_tt, tiles;                // token tiles of TN tokens; tiles in all (the ragged token tile's come last)
   long long ldc;
   int wide;                          // C (and every peer's) takes 16-byte stores: base, ldc and col0 are multiples of that
@@ -184,21 +185,21 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
   const int na = a_slots(p.tn);
   const uint32_t ring_a = smem_u32(ring), xbuf_a = smem_u32(xbuf);
   const uint32_t wfull_a = smem_u32(bars);               // [WD] weights of a group landed
-  const uint32_t wempty_a = wfull_a + kPMaxWD * 8;       // [WD] read by the 8 dequant warps
+  const uint32_t wempty_a = wfull_a + kPMaxWD * 8;       // [WD] read by the 4 dequant warps
   const uint32_t done_a = wempty_a + kPMaxWD * 8;        // [kPDone] group j % 8 multiplied (both CTAs get the commit)
   const uint32_t dfull_a = done_a + kPDone * 8;          // accumulator complete (both CTAs)
-  const uint32_t afull_a = dfull_a + 8;                  // [na] leader: a group's A operand written (8 warps of each CTA)
+  const uint32_t afull_a = dfull_a + 8;                  // [na] leader: a group's A operand written (4 warps of each CTA)
   const uint32_t xfull_a = afull_a + kPMaxA * 8;         // [kPSteps] leader: both CTAs' activations of a group landed
   const uint32_t dempty_a = xfull_a + kPSteps * 8;       // leader: accumulator read out (the epilogue warps of both CTAs)
 
   if (tid == 0) {
     for (int i = 0; i < kPMaxWD; ++i) {
       mbar_init(wfull_a + i * 8, 1);
-      mbar_init(wempty_a + i * 8, 8);
+      mbar_init(wempty_a + i * 8, 4);
     }
     for (int i = 0; i < kPDone; ++i) mbar_init(done_a + i * 8, 1);
     for (int i = 0; i < kPSteps; ++i) mbar_init(xfull_a + i * 8, 1);
-    for (int i = 0; i < kPMaxA; ++i) mbar_init(afull_a + i * 8, 16);
+    for (int i = 0; i < kPMaxA; ++i) mbar_init(afull_a + i * 8, 8);
     mbar_init(dfull_a, 1);
     mbar_init(dempty_a, 2 * EW);
     fence_mbar_init();
@@ -258,8 +259,7 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
         if (!warp_agrees(mbar_wait_bounded(dempty_a, dph, kPSpin))) dead = true;  // (passes on the first tile)
         for (int g = g0; !dead && g < g1; ++g, ++j) {
           const uint32_t st = j & (kPSteps - 1);
-          if (!warp_agrees(mbar_wait_bounded(xfull_a + st * 8, (j / kPSteps) & 1u, kPSpin) &&
-                           mbar_wait_bounded(afull_a + a * 8, aph, kPSpin))) {
+          if (!warp_waits(xfull_a + st * 8, (j / kPSteps) & 1u, afull_a + a * 8, aph, kPSpin)) {
             dead = true;
             break;
           }
@@ -316,35 +316,42 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
   } else if (warp < PW) {
     // ================================================================ dequant warps
     // The walk over tiles does not matter here: the groups come in the order of the weight ring.
-    // Two teams of eight warps take alternate groups: one group's waits, shared-memory loads and tensor-memory stores
-    // run beside the other's arithmetic. (Ring depths are even, so a barrier's consecutive phases belong to one team;
-    // a parity wait could not tell them apart otherwise.)
-    const int q = warp & 3, odd = (warp >> 2) & 1, team = warp >> 3;  // odd: takes the second half (64 k) of its groups
+    // Four teams of four warps (one output row per thread) take the groups in turn: one group's waits, shared-memory loads and
+    // tensor-memory stores run beside the others' arithmetic. (The weight ring's depth is a multiple of four and the ring of
+    // "group multiplied" barriers has eight, so a barrier's consecutive phases belong to one team; a parity wait could
+    // not tell them apart otherwise.)
+    // A team of eight warps with half a row each paid every wait, vote and arrival twice: 34816 x 5120 at M = 17 / 77 31.8 / 36.0 us
+    // with two teams of eight, 29.6 / 34.7 with four of four (M = 777, four layers of a block: 546 and 533).
+    const int q = warp & 3, team = warp >> 2;
     const int row = q * 32 + lane;
-    const uint32_t a_t = tmem_a + (static_cast<uint32_t>(q * 32) << 16) + odd * 32;
+    const uint32_t a_t = tmem_a + (static_cast<uint32_t>(q * 32) << 16);
     const uint32_t afull_l = map_to_rank(afull_a, leader);
     const int ntiles = cluster < p.tiles ? (p.tiles - 1 - cluster) / nclusters + 1 : 0;
     const uint32_t ngroups = static_cast<uint32_t>(ntiles) * static_cast<uint32_t>(g1 - g0);
-    const uint32_t off0 = 2 * odd * kChunkBytes + weight_slot(row, 0) * 16, off1 = (2 * odd + 1) * kChunkBytes + weight_slot(row, 1) * 16;
+    const uint32_t off_e = weight_slot(row, 0) * 16, off_o = kChunkBytes + weight_slot(row, 1) * 16;  // even and odd 32-k chunks
     int st = team, a = team;  // weight stage and A slot
     uint32_t wph = 0;
-    for (uint32_t j = team; j < ngroups; j += 2) {
+    for (uint32_t j = team; j < ngroups; j += kPTeams) {
       const bool landed = mbar_wait_bounded(wfull_a + st * 8, wph, kPSpin);
       const uint8_t* blk = ring + st * kTileGroupBytes;
-      const uint4 w0 = *reinterpret_cast<const uint4*>(blk + off0), w1 = *reinterpret_cast<const uint4*>(blk + off1);
+      const uint4 w[4] = {*reinterpret_cast<const uint4*>(blk + off_e), *reinterpret_cast<const uint4*>(blk + off_o),
+                          *reinterpret_cast<const uint4*>(blk + off_e + 2 * kChunkBytes),
+                          *reinterpret_cast<const uint4*>(blk + off_o + 2 * kChunkBytes)};
       const uint32_t zp = blk[kTgZpOff + row];
       const uint32_t sc = reinterpret_cast<const uint16_t*>(blk + kTgScaleOff)[row];
       const uint32_t zpair = __byte_perm(zp, 0x43434343u, 0x4040);  // bf16 pair (128+zp, 128+zp)
       const uint32_t spair = sc | (sc << 16);
-      const uint32_t w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-      uint32_t v[2][16];
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
+      auto expand = [&](const uint4& c, uint32_t(&v)[16]) {
+        const uint32_t cw[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int pp = 0; pp < 4; ++pp)
-            v[c][4 * i + pp] = mul_bf16x2(sub_bf16x2(((w[4 * c + i] >> (4 * pp)) & kNibMaskP) | kMagicP, zpair), spair);
+            v[4 * i + pp] = mul_bf16x2(sub_bf16x2(((cw[i] >> (4 * pp)) & kNibMaskP) | kMagicP, zpair), spair);
+      };
+      uint32_t v0[16], v1[16];
+      expand(w[0], v0);
+      expand(w[1], v1);
       // (the vote is also what tells lane 0 that the whole warp has read the stage)
       if (!warp_agrees(landed)) {
         dead = true;
@@ -359,14 +366,18 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
         break;
       }
       tc_fence_after();
-      tmem_st16(a_t + a * 64, v[0]);
-      tmem_st16(a_t + a * 64 + 16, v[1]);
+      tmem_st16(a_t + a * 64, v0);
+      tmem_st16(a_t + a * 64 + 16, v1);
+      expand(w[2], v0);
+      tmem_st16(a_t + a * 64 + 32, v0);
+      expand(w[3], v1);
+      tmem_st16(a_t + a * 64 + 48, v1);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(afull_l + a * 8);
-      if ((a += 2) >= na) a -= na;
-      if ((st += 2) >= WD) {
+      if ((a += kPTeams) >= na) a -= na;
+      if ((st += kPTeams) >= WD) {
         st -= WD;
         wph ^= 1;
       }
@@ -550,7 +561,7 @@ PrefillPlan plan_prefill(int M, int pairs, int G, const int* device_clusters, in
     }
   }
   best.wdepth = kPMaxWD;
-  while (best.wdepth > 2 && prefill_smem(best.tn, best.wdepth) > smem_optin) best.wdepth -= 2;
+  while (best.wdepth > kPTeams && prefill_smem(best.tn, best.wdepth) > smem_optin) best.wdepth -= kPTeams;
   best.smem = prefill_smem(best.tn, best.wdepth);
   return best;
 }
@@ -611,7 +622,7 @@ const int* cluster_slots(int dev, const DeviceInfo* di) {
     for (int S = 1; S <= kPMaxSplit && e == cudaSuccess; ++S) {
       cudaLaunchConfig_t cfg = {};
       cudaLaunchAttribute at[1];
-      cluster_config(cfg, at, S, 1, prefill_smem(kPMaxTN, 2));
+      cluster_config(cfg, at, S, 1, prefill_smem(kPMaxTN, kPTeams));
       e = cudaOccupancyMaxActiveClusters(&s.n[S], k_prefill, &cfg);
     }
     if (e != cudaSuccess || s.n[1] < 1) {
