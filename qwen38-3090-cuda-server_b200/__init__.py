@@ -158,14 +158,23 @@ def check(rc: int):
         raise W4A16Error(rc, lib().w4a16_last_error().decode())
 
 
+# The per-call conversions are plain integers (the signatures above turn them into pointers) and the stream is asked for by its
+# raw handle, without a torch.cuda.Stream around it: an eager GEMV of 5120 x 6144 is bound by the host.
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
+
+
+_torch = None
 
 
 def _stream(stream=None):
-    import torch
-    s = torch.cuda.current_stream() if stream is None else stream
-    return C.c_void_p(s.cuda_stream)
+    global _torch
+    if stream is not None:
+        return stream.cuda_stream
+    if _torch is None:
+        import torch
+        _torch = torch
+    return _torch._C._cuda_getCurrentRawStream(_torch.cuda.current_device())
 
 
 # --------------------------------------------------------------------- weights

@@ -37,6 +37,7 @@ int fail(int code, const char* fmt, ...) {
 constexpr int kMaxDevices = 64;
 static DeviceInfo g_dev[kMaxDevices];
 static std::mutex g_dev_mu;
+static std::atomic<bool> g_dev_ready[kMaxDevices];  // g_dev[i] is filled in and does not change any more
 static std::mutex g_ww_mu;
 static std::vector<cudaStream_t> g_ww_streams;  // streams with a weight write no matmul call has followed yet
 static std::atomic<int> g_ww_count{0};
@@ -49,8 +50,9 @@ const DeviceInfo* device_info() {
     set_error("no current CUDA device");
     return nullptr;
   }
-  std::lock_guard<std::mutex> lk(g_dev_mu);
   DeviceInfo& d = g_dev[dev];
+  if (g_dev_ready[dev].load(std::memory_order_acquire)) return &d;
+  std::lock_guard<std::mutex> lk(g_dev_mu);
   if (d.device != dev) {
     int sms = 0, smem = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
@@ -67,6 +69,7 @@ const DeviceInfo* device_info() {
     d.smem_optin = smem;
     d.status = st;
     d.device = dev;
+    g_dev_ready[dev].store(true, std::memory_order_release);
   }
   return &d;
 }
