@@ -158,6 +158,11 @@ struct Geo {
   // shallow one (4 steps) the wait is on the critical loop and belongs to the issuer, so that the operand is
   // already unpacked when the slot comes free.
   static constexpr bool kIssuerWaitsD = DD2 < 8;
+  // The issuers' three tests of a step in flight together (one that is over already costs 74 cycles). 34816 x 5120 / 16384 x 5120 / 5120 x 6144 /
+  // 5120 x 17408 at M = 16 in us: 25.94 / 15.46 / 10.29 / 18.23 ->
+  // 25.35 / 14.87 / 9.94 / 17.62, heads the same. At the other token counts the longer code costs as much or more (M = 8 19.37 / 11.75 / 8.07 -> 19.98 / 12.09 / 8.16).
+  static constexpr bool kTogether = MT == 16;
+  static_assert(!kTogether || kIssuerWaitsD, "three waits");
   // A round of the fix-up warps is one step, except at M = 1, where two steps' loads are in flight together.
   static constexpr bool kPairRounds = MT == 1;
   static_assert(3 * TM <= CB && FW * CB <= N, "token sets must fit their column blocks");
@@ -763,6 +768,21 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
       const uint32_t step16 = (2 * b_lbo) >> 4, slot16 = static_cast<uint32_t>(b_slot) >> 4;
       for (int t = mine; ok && t < T; t += 2) {
         const int a = t & (AD2 - 1), d = t & (DD2 - 1);
+        uint32_t e;
+        if constexpr (GE::kTogether) {
+          // the waits of the branch below, their tests in flight together
+          const uint32_t bar_a = afull_a + a * 8, par_a = static_cast<uint32_t>(t / AD2) & 1u;
+          const uint32_t bar_b = bfull_a + (t & (BD - 1)) * 8, par_b = static_cast<uint32_t>(t >> BS) & 1u;
+          const uint32_t bar_d = dempty_a + d * 8, par_d = static_cast<uint32_t>(t / DD2 - 1) & 1u;
+          const bool ra = mbar_try_wait(bar_a, par_a), rb = mbar_try_wait(bar_b, par_b), rd = t < DD2 || mbar_try_wait(bar_d, par_d);
+          if (!warp_agrees(ra & rb & rd) &&
+              !warp_agrees((rd || mbar_wait_bounded(bar_d, par_d, kSpinLimit)) && (rb || mbar_wait_bounded(bar_b, par_b, kSpinLimit)) &&
+                           (ra || mbar_wait_bounded(bar_a, par_a, kSpinLimit)))) {
+            atomicExch(p.status, W4A16_ETIMEOUT);
+            break;
+          }
+          e = 2u * (t & (BD - 1)) * 0x101u + 0x100u;  // the two halves of digit-ring slot t % BD
+        } else {
         // A written (its writers also saw the step's weights and table entry landed), and the D slot this
         // step fills has been read out by every fix-up warp
         if (!warp_agrees(mbar_wait_bounded(afull_a + a * 8, static_cast<uint32_t>(t / AD2) & 1u, kSpinLimit) &&
@@ -771,7 +791,7 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
           atomicExch(p.status, W4A16_ETIMEOUT);
           break;
         }
-        const uint32_t e = table[t & (kTable - 1)].x;
+        e = table[t & (kTable - 1)].x;
         if constexpr (kStream) {
           // the step's digit rows have landed in their ring slot (bulk copy: async proxy, as the MMA reads them)
           if (!warp_agrees(mbar_wait_bounded(bfull_a + (t & (BD - 1)) * 8, static_cast<uint32_t>(t >> BS) & 1u, kSpinLimit))) {
@@ -793,6 +813,7 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
           }
           __threadfence_block();
           all_ready = mbar_test_wait(bready_a, 0);
+        }
         }
         tc_fence_after();
         const uint32_t d_t = tmem + GE::kDCol0 + d * GE::kDColsS;
