@@ -28,8 +28,7 @@
 //
 // What bounds it: long prompts run at the tensor cores' rate under the power cap (256 x 256 x 16 per 128 cycles: 1024
 // cycles per k group; tensor pipe 87.5 % active over a 4096-token launch), short ones at the expansion of the weights: a
-// CTA and k group is about 2400 warp instructions, 600 cycles if every issue slot were taken, and about 850 as it runs (0.62
-// of the slots, ALU pipe 54 to 68 % active), where HBM would allow 386.
+// CTA and k group takes 640 to 700 cycles (ALU pipe 53 to 66 % active, issue slots about half), where HBM would allow 386.
 // In us, weights cold, against one CTA per tile of 128 x 256 with eight dequant warps:
 //   34816 x 5120, M = 4096: 1264 -> 922 (1583 TFLOP/s); 5120 x 17408, M = 4096: 698 -> 488 (1497)
 //   34816 x 5120, M = 777:   300 -> 202;                5120 x 8192, M = 777:   110 -> 57
@@ -86,6 +85,12 @@ struct PrefillParams {
   unsigned* comm_peers[8];
   int comm_n, comm_rank;
 };
+
+__device__ __forceinline__ uint32_t fma_bf16x2(uint32_t a, uint32_t b, uint32_t c) {
+  uint32_t d;
+  asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
 
 // ---- CTA pairs and clusters --------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -344,7 +349,26 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
       const uint32_t sc = reinterpret_cast<const uint16_t*>(blk + kTgScaleOff)[row];
       const uint32_t zpair = __byte_perm(zp, 0x43434343u, 0x4040);  // bf16 pair (128+zp, 128+zp)
       const uint32_t spair = sc | (sc << 16);
+      // Nibbles 0 and 4 of a word become (128 + q) - (128 + zp) by one OR and a subtraction. Nibbles 1 and 5 are left where they
+      // are: as a bf16 pair w & 0x00F000F0 is q 2^-129 (subnormals, and the first normal binade goes on where they end), so
+      // one packed FMA makes (q - zp) / 4 of it, exactly, and 4 s is exact too: the same product, rounded once. The ALU pipe
+      // (shifts and LOP3) is the busiest: 80 of its instructions per row and group instead of 112. Four layers of a block at M = 30 /
+      // 77: 77.7 / 85.0 us with a shift per nibble position, 76.5 / 83.8 with this (74.1 / 81.7 without the test for large scales).
+      const uint32_t zquarter = fma_bf16x2(zpair, 0xBE80BE80u, 0x42004200u);  // -zp / 4 = 32 - (128 + zp) / 4
+      const uint32_t s4 = mul_bf16x2(spair, 0x40804080u);
       auto expand = [&](const uint4& c, uint32_t(&v)[16]) {
+        const uint32_t cw[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t w8 = cw[i] >> 8;
+          v[4 * i] = mul_bf16x2(sub_bf16x2((cw[i] & kNibMaskP) | kMagicP, zpair), spair);
+          v[4 * i + 1] = mul_bf16x2(fma_bf16x2(cw[i] & 0x00F000F0u, 0x7F007F00u, zquarter), s4);
+          v[4 * i + 2] = mul_bf16x2(sub_bf16x2((w8 & kNibMaskP) | kMagicP, zpair), spair);
+          v[4 * i + 3] = mul_bf16x2(fma_bf16x2(w8 & 0x00F000F0u, 0x7F007F00u, zquarter), s4);
+        }
+      };
+      // ... unless 4 s overflows, from 2^126 on
+      auto expand_large = [&](const uint4& c, uint32_t(&v)[16]) {
         const uint32_t cw[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -355,11 +379,17 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
       uint32_t v0[16], v1[16];
       expand(w[0], v0);
       expand(w[1], v1);
-      // (the vote is also what tells lane 0 that the whole warp has read the stage)
-      if (!warp_agrees(landed)) {
-        dead = true;
-        break;
+      bool large = false;
+      if (!warp_agrees(landed && (sc & 0x7FFFu) - 0x7E80u >= 0x100u)) {
+        if (!warp_agrees(landed)) {
+          dead = true;
+          break;
+        }
+        large = true;
+        expand_large(w[0], v0);
+        expand_large(w[1], v1);
       }
+      // (the votes are also what tells lane 0 that the whole warp has read the stage)
       if (lane == 0) mbar_arrive(wempty_a + st * 8);
       // only now the wait for the A slot: the MMAs that read it last, na groups ago, must have completed
       const uint32_t jd = j - na;
@@ -371,9 +401,14 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
       tc_fence_after();
       tmem_st16(a_t + a * 64, v0);
       tmem_st16(a_t + a * 64 + 16, v1);
-      expand(w[2], v0);
+      if (large) {
+        expand_large(w[2], v0);
+        expand_large(w[3], v1);
+      } else {
+        expand(w[2], v0);
+        expand(w[3], v1);
+      }
       tmem_st16(a_t + a * 64 + 32, v0);
-      expand(w[3], v1);
       tmem_st16(a_t + a * 64 + 48, v1);
       tmem_wait_st();
       tc_fence_before();

@@ -112,3 +112,28 @@ def test_several_tiles_per_cluster(N, K, M):
 def test_output_not_16_byte_aligned(skew):
     _check(400, 384, 77, skew=skew)
     _check(2048, 1024, 300, skew=skew)
+
+
+@pytest.mark.parametrize("exponent", [-126, -20, 125, 126, 127])
+def test_scales_at_both_ends(exponent):
+    """The product with scales up to the largest powers of two (from 2^126 on four times the scale is no number) against fp64 on
+    the dequantised rows, weights within +-1 of their zero points, activations that bring the sums back to ordinary size."""
+    N, K, M = 144, 640, 40
+    rng = np.random.Generator(np.random.PCG64(5))
+    z = rng.integers(1, 15, (N, K // 128), dtype=np.uint8)
+    q = (np.repeat(z, 128, axis=1).astype(np.int64) + rng.integers(-1, 2, (N, K))).astype(np.uint8)
+    scale = synth.f32_to_bf16_bits(np.full((N, K // 128), np.ldexp(1.5, exponent), np.float32))
+    scale[::3, 1] = synth.f32_to_bf16_bits(np.array([0.25], np.float32))[0]  # rows of both kinds in a warp
+    w = pkg.weights_from_numpy(synth.pack_weight(q), scale, synth.pack_zero_point(z))
+    deq = torch.empty((N, K), dtype=torch.bfloat16, device="cuda")
+    pkg.w4a16_dequant_rows(deq, w, 0, N)
+    x = torch.randn((M, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(5))
+    x = (x * 2.0 ** (-60 if exponent > 0 else 20)).to(torch.bfloat16)
+    ws = pkg.gemm_workspace_alloc(4096)
+    c = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+    pkg.gemm_w4a16(c, w, x, M, ws)
+    ref, mag = x.double() @ deq.double().t(), x.double().abs() @ deq.double().abs().t()
+    assert pkg.device_status() == 0 and bool(torch.isfinite(c).all())
+    assert bool(((c.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + K * 2.0 ** -24 * mag).all())
+    pkg.gemm_workspace_free(ws)
+    pkg.awq_free(w)
