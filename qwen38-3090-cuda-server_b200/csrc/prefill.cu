@@ -389,7 +389,9 @@ __global__ void __launch_bounds__(kPWarps * 32, 1) k_prefill(const __grid_consta
         expand_large(w[0], v0);
         expand_large(w[1], v1);
       }
-      // (the votes are also what tells lane 0 that the whole warp has read the stage)
+      // The second half of the row is in registers but used only below: a vote orders no memory accesses, __syncwarp does, so
+      // that the next bulk copy into the stage cannot pass another lane's loads.
+      __syncwarp();
       if (lane == 0) mbar_arrive(wempty_a + st * 8);
       // only now the wait for the A slot: the MMAs that read it last, na groups ago, must have completed
       const uint32_t jd = j - na;
