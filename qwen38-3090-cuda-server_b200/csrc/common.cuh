@@ -41,9 +41,10 @@ const DeviceInfo* device_info();
 // The matmul kernels start fetching weights before griddepcontrol.wait, and only that wait guarantees that the
 // stores of the kernel in front of them are visible. So every entry that writes weight buffers notes its
 // stream, and the next matmul call on that stream is enqueued without the programmatic-serialisation
-// attribute: fully ordered behind the write. take_weight_write is true once per noted stream; with no write
-// pending it costs one relaxed atomic load. It is called when nothing can refuse the call any more, and a launch that
-// fails notes the stream again.
+// attribute: fully ordered behind the write. take_weight_write is true once per noted stream, and besides once in every capture of
+// that stream's calls: a call that is only captured runs later, if at all, so it leaves the note to the next one that is executed (the
+// graph's other calls may be programmatic, as there is one in front of them). With no write pending it costs one relaxed
+// atomic load. It is called when nothing can refuse the call any more, and a launch that fails notes the stream again.
 void note_weight_write(cudaStream_t st);
 bool take_weight_write(cudaStream_t st);
 bool pdl_enabled();  // programmatic dependent launch (default on; W4A16_PDL=0 turns it off)

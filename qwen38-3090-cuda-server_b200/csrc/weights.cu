@@ -39,7 +39,12 @@ static DeviceInfo g_dev[kMaxDevices];
 static std::mutex g_dev_mu;
 static std::atomic<bool> g_dev_ready[kMaxDevices];  // g_dev[i] is filled in and does not change any more
 static std::mutex g_ww_mu;
-static std::vector<cudaStream_t> g_ww_streams;  // streams with a weight write no matmul call has followed yet
+// Streams with a weight write that no executed matmul call has followed yet, and the last capture in which a call has.
+struct WeightWrite {
+  cudaStream_t stream;
+  unsigned long long followed_in;
+};
+static std::vector<WeightWrite> g_ww;
 static std::atomic<int> g_ww_count{0};
 
 __device__ int g_status_word = 0;
@@ -189,20 +194,40 @@ __global__ void k_wait_timeout_selftest(int* status, uint32_t polls) {
 
 }  // namespace
 
+// The capture that the stream's calls go to, or 0: they are executed. (An error says that the legacy stream cannot be used while
+// another one is captured; the launch that follows reports it and the note comes back.)
+static unsigned long long capture_of(cudaStream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusNone ? 0 : id;
+}
+
 void note_weight_write(cudaStream_t st) {
   std::lock_guard<std::mutex> lk(g_ww_mu);
-  for (cudaStream_t q : g_ww_streams)
-    if (q == st) return;
-  g_ww_streams.push_back(st);
-  g_ww_count.store(static_cast<int>(g_ww_streams.size()), std::memory_order_release);
+  for (WeightWrite& w : g_ww)
+    if (w.stream == st) {
+      w.followed_in = 0;
+      return;
+    }
+  g_ww.push_back({st, 0});
+  g_ww_count.store(static_cast<int>(g_ww.size()), std::memory_order_release);
 }
 bool take_weight_write(cudaStream_t st) {
   if (g_ww_count.load(std::memory_order_relaxed) == 0) return false;
   std::lock_guard<std::mutex> lk(g_ww_mu);
-  for (size_t i = 0; i < g_ww_streams.size(); ++i)
-    if (g_ww_streams[i] == st) {
-      g_ww_streams.erase(g_ww_streams.begin() + static_cast<long>(i));
-      g_ww_count.store(static_cast<int>(g_ww_streams.size()), std::memory_order_release);
+  for (size_t i = 0; i < g_ww.size(); ++i)
+    if (g_ww[i].stream == st) {
+      if (const unsigned long long capture = capture_of(st)) {
+        const bool first = g_ww[i].followed_in != capture;
+        g_ww[i].followed_in = capture;
+        return first;
+      }
+      g_ww.erase(g_ww.begin() + static_cast<long>(i));
+      g_ww_count.store(static_cast<int>(g_ww.size()), std::memory_order_release);
       return true;
     }
   return false;

@@ -53,11 +53,11 @@ class _EdgeData(C.Structure):
     _fields_ = [("from_port", C.c_ubyte), ("to_port", C.c_ubyte), ("type", C.c_ubyte), ("reserved", C.c_ubyte * 5)]
 
 
-def captured_edges(fn):
+def captured_edges(fn, stream=None):
     """Edge kinds, first to last, of the chain of nodes that `fn(stream)` captures
     (CUgraphDependencyType: 0 full, 1 programmatic)."""
     cuda = C.CDLL("libcuda.so.1")
-    stream = torch.cuda.Stream()
+    stream = stream or torch.cuda.Stream()
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph, stream=stream):
         fn(stream)

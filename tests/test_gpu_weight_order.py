@@ -84,6 +84,61 @@ def test_refused_call_leaves_the_ordering_to_the_next(pkg, layer, name, why):
     assert captured_edges(chain) == [FULL] + [PROGRAMMATIC] * (n - 1)
 
 
+@pytest.mark.parametrize("name", ["gemv", "skinny", "prefill"])
+def test_captured_calls_leave_the_ordering_to_the_next_executed_one(pkg, layer, name):
+    """What a later call would get is read from a capture, of which only the edges count: the first matmul behind the write is
+    fully ordered in every capture, however many there are, until a call on the stream has been executed."""
+    src, w, calls, _ = layer
+    fn, n = calls[name]
+    stream, rows = torch.cuda.Stream(), torch.empty((w.out_f, w.in_f), dtype=torch.bfloat16, device="cuda")
+
+    def chain(st):
+        pkg.w4a16_dequant_rows(rows, w, 0, w.out_f, stream=st)  # the node in front of the first matmul
+        fn(st)
+        fn(st)
+
+    ordered, free = [FULL] + [PROGRAMMATIC] * (2 * n - 1), [PROGRAMMATIC] * (2 * n)
+    assert captured_edges(chain, stream) == free
+    pkg.awq_repack_into(w, 0, *src, stream=stream)
+    assert captured_edges(chain, stream) == ordered
+    assert captured_edges(chain, stream) == ordered
+    fn(stream)
+    assert captured_edges(chain, stream) == free
+    # a write that is captured itself: the matmul behind it, and the next executed one
+    assert captured_edges(lambda st: (pkg.awq_repack_into(w, 0, *src, stream=st), chain(st)), stream) == [FULL] + ordered
+    fn(stream)
+    assert captured_edges(chain, stream) == free
+    torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("name", ["gemv", "skinny", "prefill"])
+def test_executed_call_behind_a_repack_and_a_capture(pkg, synth, layer, name):
+    """Repack, a matmul that is only captured, the same matmul executed: the new weights' bits."""
+    src, w, calls, _ = layer
+    other = _tensors(synth, w.out_f, w.in_f, 9)
+    stream = torch.cuda.Stream()
+    x = torch.randn((80, w.in_f), device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)).to(torch.bfloat16)
+    y = [torch.zeros((80, w.out_f), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    block, ws = pkg.gemv_scratch_alloc(w.in_f, w.out_f, 128, 16), pkg.gemm_workspace_alloc(4096)
+    call = {"gemv": lambda out: pkg.gemv_w4a16(out, w, x, block, stream=stream),
+            "skinny": lambda out: pkg.gemm_small_w4a16(out, w, x, 9, block, stream=stream),
+            "prefill": lambda out: pkg.gemm_w4a16(out, w, x, 77, ws, stream=stream)}[name]
+    torch.cuda.synchronize()
+    for tensors in (other, src) * 4:
+        call(y[0])  # the old weights' call in front
+        pkg.awq_repack_into(w, 0, *tensors, stream=stream)
+        with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=stream):
+            call(y[1])
+        call(y[0])
+        torch.cuda.synchronize()
+        call(y[1])
+        torch.cuda.synchronize()
+        assert torch.equal(y[0].view(torch.int16), y[1].view(torch.int16))
+    assert pkg.device_status() == 0
+    pkg.gemv_scratch_free(block)
+    pkg.gemm_workspace_free(ws)
+
+
 def _steps(pkg, layers, ws, scratch, b, stream):
     """Prefill and decode calls in which every call reads what the one in front of it wrote, or writes what it read."""
     w0, w1, w2 = layers
