@@ -1252,7 +1252,16 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
             // from the last sums to the end of a 5120 x 6144 launch 1.1 us at M = 2, 3.2 us at M = 4. Launches of 5120 x 6144 /
             // 5120 x 17408 / 34816 x 5120 in us, before -> after: M = 1 6.17 / 10.57 / 16.63 -> 6.04 / 10.41 / 16.48, M = 4 8.84 / 13.65 /
             // 18.56 -> 6.91 / 11.36 / 18.42, M = 9 9.05 / 16.08 / 22.58 -> 8.48 / 15.34 / 22.12, M = 12 at 5120 x 6144 10.54 -> 9.48.)
-            constexpr int PB = TM <= 2 ? 4 : (MT == 9 ? 2 : 1);  // pieces per batch: what fits the registers without spills
+            // Int8 weights keep the tests at M = 2 and 13 to 15: straight-line loads raise what their instances spill from 4 and 24 bytes
+            // (stores and loads) to 8 and 60, and from 4 and 16 to 44 and 40, part of it in the loop over steps. Straight -> tested in us, M = 2:
+            // 2048 x 2048 5.12 -> 4.93, heads of 32768 x 1024 11.28 -> 11.02, 131072 x 4096 82.5 both; M = 15: heads of 248320 x 5120
+            // 211.2 -> 201.9, 131072 x 4096 98.4 -> 93.1, 32768 x 1024 16.71 -> 16.38, and 5120 x 6144 11.34 -> 11.64, the one layer that loses. (In
+            // two straight batches, of three tokens and two: 203.2, 94.6, 16.86 and 12.84.)
+            constexpr bool kStraight = !(WB == 8 && (MT == 2 || MT == 15));
+            // Pieces per batch: what fits the registers. Two at three tokens and more, stores / loads spilled with int4 weights: M = 6 24 / 88 bytes,
+            // M = 8 and 16 52 / 48, M = 12 40 / 56, M = 15 250 / 276; at M = 9, whose limit is 80, none: 5120 x 6144 / 16384 x 5120 / 5120 x 17408
+            // with one piece 9.00 / 13.29 / 15.74 us, with two 8.52 / 12.87 / 15.31.
+            constexpr int PB = TM <= 2 ? 4 : (MT == 9 ? 2 : 1);
             for (int cb = c_first + 1; cb <= c_last && ok; cb += PB) {
               unsigned long long piece[PB][TM];
               unsigned long long* sl[PB];
@@ -1265,15 +1274,26 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
               }
               uint32_t spins = 0;
               for (;;) {
-#pragma unroll
-                for (int k = 0; k < PB; ++k)
-#pragma unroll
-                  for (int i = 0; i < TM; ++i) piece[k][i] = ld_relaxed_gpu_u64(sl[k] + min(m0 + i, M - 1) * kTileRows);
                 uint32_t differ = 0;
+                if constexpr (kStraight) {
 #pragma unroll
-                for (int k = 0; k < PB; ++k)
+                  for (int k = 0; k < PB; ++k)
 #pragma unroll
-                  for (int i = 0; i < TM; ++i) differ |= static_cast<uint32_t>(piece[k][i] >> 32) ^ kPieceTag;
+                    for (int i = 0; i < TM; ++i) piece[k][i] = ld_relaxed_gpu_u64(sl[k] + min(m0 + i, M - 1) * kTileRows);
+#pragma unroll
+                  for (int k = 0; k < PB; ++k)
+#pragma unroll
+                    for (int i = 0; i < TM; ++i) differ |= static_cast<uint32_t>(piece[k][i] >> 32) ^ kPieceTag;
+                } else {
+#pragma unroll
+                  for (int k = 0; k < PB; ++k)
+#pragma unroll
+                    for (int i = 0; i < TM; ++i)
+                      if (cb + k <= c_last && m0 + i < M) {
+                        piece[k][i] = ld_relaxed_gpu_u64(sl[k] + (m0 + i) * kTileRows);
+                        differ |= static_cast<uint32_t>(piece[k][i] >> 32) ^ kPieceTag;
+                      }
+                }
                 if (__all_sync(0xffffffffu, differ == 0u)) break;
                 if (++spins > kSpinLimit) {
                   atomicExch(p.status, W4A16_ETIMEOUT);
@@ -1286,7 +1306,7 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
                 if (cb + k <= c_last) {
 #pragma unroll
                   for (int i = 0; i < TM; ++i) {
-                    v[i] += __uint_as_float(static_cast<uint32_t>(piece[k][i]));
+                    if (kStraight || m0 + i < M) v[i] += __uint_as_float(static_cast<uint32_t>(piece[k][i]));
                     if (m0 + i < M) st_relaxed_gpu_u64(sl[k] + (m0 + i) * kTileRows, 0ull);
                   }
                 }

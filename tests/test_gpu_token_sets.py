@@ -33,3 +33,25 @@ def test_rows_equal_the_single_row_kernel(pkg, synth, N, K):
     assert pkg.device_status() == 0
     pkg.gemv_scratch_free(scratch)
     pkg.awq_free(w)
+
+
+# int8 weights: tiles of two to about twenty pieces, whose reader differs by token count; twice, so that the second launch finds
+# the words that the first one has zeroed
+@pytest.mark.parametrize("N,K", [(272, 4096), (1024, 16384), (5120, 640)])
+@pytest.mark.parametrize("M", [2, 3, 4, 8, 12, 13, 14, 15, 16])
+def test_int8_rows_of_split_tiles(pkg, N, K, M):
+    gen = torch.Generator(device="cuda").manual_seed(N + K)
+    w = pkg.quantize_w8a16((torch.randn((N, K), device="cuda", generator=gen) * 0.02).to(torch.bfloat16))
+    scratch = pkg.gemv_scratch_alloc(K, N, 128, 16)
+    x = torch.randn((M, K), device="cuda", generator=gen).to(torch.bfloat16)
+    rows, y = (torch.empty((M, N), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    for m in range(M):
+        pkg.gemv_w8a16(rows[m], w, x[m], scratch)
+    for _ in range(2):
+        y.zero_()
+        pkg.gemm_small_w8a16(y, w, x, M, scratch)
+        assert torch.equal(y.view(torch.int16), rows.view(torch.int16))
+    assert pkg.device_status() == 0
+    pkg.gemv_scratch_free(scratch)
+    pkg.w8a16_free(w)
