@@ -247,8 +247,9 @@ int w4a16_shard_rows(int out_f, int nranks, int rank, int* row_begin, int* row_e
  * blocks[rank] is the local one. All ranks must issue
  * the same sequence of signalling launches on a communicator (every w4a16_*_gather / *_sharded call below
  * signals once). Zero the blocks and make that visible on every rank (a host barrier) before the first
- * call. Every wait is bounded (about a second): on expiry the waiting kernel records W4A16_ETIMEOUT in
- * the device status word and carries on. No reference counterpart (the reference is single-GPU). */
+ * call. Every wait is bounded: for another rank's flag about a second, for the kernel's own hand-overs one to four
+ * seconds, longer than what they may stand behind (at the most 17 s, where one stands behind the wait for a flag). On
+ * expiry the waiting kernel records W4A16_ETIMEOUT in the device status word and carries on. No reference counterpart (the reference is single-GPU). */
 typedef struct w4a16_comm {
   uint32_t* blocks[8];
   int nranks, rank;

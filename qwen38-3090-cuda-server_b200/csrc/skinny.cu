@@ -73,7 +73,8 @@ struct Fmt {
   static constexpr int kStage = kStepGroups * kBlock;                        // 17152 / 33280
 };
 constexpr int kTable = 64;                 // step table entries (ring)
-constexpr uint32_t kSpinLimit = 1u << 20;  // polls before a wait gives up
+constexpr uint32_t kSpinLimit = 1u << 20;  // tests before a wait gives up: about four seconds on a barrier, one for a piece of a split tile
+constexpr uint32_t kReadyLimit = 1u << 25; // polls of shared memory: over two seconds, more than the wait for a rank's flag in front of it
 constexpr uint32_t kPieceTag = 0x7A6B5C4Du;  // upper half of a published (sum, tag) word of a split tile's piece
 constexpr int kFixBar = 1;                 // named barrier of the fix-up warps
 constexpr int kConvBar = 2;                // named barrier of the converting warps
@@ -804,10 +805,10 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
           const uint32_t s0 = e & 0xFFu, s1 = (e >> 8) & 0xFFu, need = static_cast<uint32_t>(M);
           uint32_t spins = 0;
           while (rdy[s0] < need || rdy[s1] < need) {
-            if (++spins > kSpinLimit) break;
+            if (++spins > kReadyLimit) break;
             __nanosleep(40);
           }
-          if (!warp_agrees(spins <= kSpinLimit)) {
+          if (!warp_agrees(spins <= kReadyLimit)) {
             atomicExch(p.status, W4A16_ETIMEOUT);
             break;
           }

@@ -9,6 +9,8 @@ one rank) is covered by the multi-GPU worker.
 The wait that runs out: a communicator of two ranks of which only one ever signals. The bounded
 wait gives up after about a second, the status word reads W4A16_ETIMEOUT, nothing hangs or faults.
 """
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -123,6 +125,37 @@ def test_chained_layers_wait_for_the_previous_gather(pkg, oracle, synth, M):
     pkg.gemv_scratch_free(s)
     pkg.awq_free(A)
     pkg.awq_free(B)
+
+
+@pytest.mark.parametrize("M", [1, 9])
+def test_wait_for_a_rank_that_signals_late(pkg, synth, M):
+    """Nearly half of the second that a flag is waited for: nothing else in the kernel may give up before that wait does. The other
+    rank's signal is a copy from the host, so no kernel waits for another one."""
+    N, K = 2048, 1024
+    w = pkg.weights_from_numpy(*synth.make_weights(N // 2, K, seed=83))
+    s = pkg.gemv_scratch_alloc(K, N, 128, 16)
+    x = dev_bf16(synth.make_activations(M, K, seed=83))
+    want = torch.empty((M, N // 2), dtype=torch.bfloat16, device="cuda")
+    pkg.gemm_small_w4a16(want, w, x, M, s)
+    ys = [torch.zeros((M, N), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    flags, ptrs = _blocks(2)
+    flags[0, 0], flags[0, 16] = 65536, 1  # one launch so far, and this rank's part of it is there
+    signal = torch.full((1,), 65536, dtype=torch.int32).pin_memory()
+    run, copy = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    pkg.gemm_skinny_gather([y.data_ptr() for y in ys], pkg.make_comm(ptrs, 0), N, 0, w, x, M, s, wait_prev=True, stream=run)
+    time.sleep(0.4)
+    assert not run.query()
+    with torch.cuda.stream(copy):
+        flags[0, 1:2].copy_(signal, non_blocking=True)
+    torch.cuda.synchronize()
+    status = pkg.device_status()
+    pkg.device_status_clear()
+    assert status == 0
+    for y in ys:
+        assert torch.equal(y[:, : N // 2].view(torch.int16), want.view(torch.int16))
+    pkg.gemv_scratch_free(s)
+    pkg.awq_free(w)
 
 
 def test_wait_for_a_rank_that_never_signals_runs_out(pkg, synth):
