@@ -155,7 +155,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait: gives up after `limit` tests (each may block for the time above) and returns
+// Bounded wait: gives up after `limit` tests (each may block for the time above: 2^20 of them last about four seconds) and returns
 // false; never spins forever.
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity, uint32_t limit) {
   for (uint32_t i = 0; i < limit; ++i)

@@ -27,14 +27,15 @@
 //     are added through distributed shared memory, always in split order (bitwise reproducible).
 //
 // What bounds it: long prompts run at the tensor cores' rate under the power cap (256 x 256 x 16 per 128 cycles: 1024
-// cycles per k group; tensor pipe 87.5 % active over a 4096-token launch), short ones at the expansion of the weights: a
-// CTA and k group takes 640 to 700 cycles (ALU pipe 53 to 66 % active, issue slots about half), where HBM would allow 386.
-// In us, weights cold, against one CTA per tile of 128 x 256 with eight dequant warps:
+// cycles per k group; tensor pipe 87 % active over a 4096-token launch), short ones by no single role: a CTA and k group takes
+// 640 to 700 cycles (5120 x 17408 at M = 77: issue slots 52 %, ALU pipe 41 % on average and 52 % on the busiest SM, tensor pipe 43 % of active
+// cycles), where HBM would allow 386.
+// In us, weights cold, against one CTA per tile of 128 x 256 with eight dequant warps (by box and temperature: 2 to 10 %):
 //   34816 x 5120, M = 4096: 1264 -> 922 (1583 TFLOP/s); 5120 x 17408, M = 4096: 698 -> 488 (1497)
-//   34816 x 5120, M = 777:   300 -> 202;                5120 x 8192, M = 777:   110 -> 57
-//   34816 x 5120, M = 77:     73 -> 37;                 5120 x 17408, M = 77:   105 -> 25;     8192 x 5120, M = 77: 45 -> 20
+//   34816 x 5120, M = 777:   300 -> 208;                5120 x 8192, M = 777:   110 -> 54
+//   34816 x 5120, M = 77:     73 -> 34;                 5120 x 17408, M = 77:   105 -> 23;     8192 x 5120, M = 77: 45 -> 13
 // and on the way, 34816 x 5120 at M = 4096 on one device: half groups as the unit of every hand-off 1134 (the first shape; the
-// issuing thread is the limit), whole groups 1063, two teams of dequant warps and C through shared memory 890. A warp's vote on
+// issuing thread is the limit), whole groups 1063, two teams of dequant warps (four since) and C through shared memory 890. A warp's vote on
 // its waits took another 9 % off short prompts (34816 x 5120 at M = 77: 40.8 -> 37.1) by keeping the loops warp-uniform.
 // Programmatic dependent launch (the next launch sets up, streams and expands its first weights as this one's CTAs leave) took
 // the four layers of a block from 104.8 to 96.5 us at M = 77 (5120 -> 8192, 6144 -> 5120, MLP) and from 562.5 to 546.7 at M = 777.
@@ -578,12 +579,13 @@ int prefill_smem(int tn, int wdepth) {
 // (4 TN cycles per group for a pair) and the expansion of the weights (kExpand cycles per group), plus
 // what is paid once per tile (pipeline fill, read-out of the accumulator, the exchange of split K). Tiles go to
 // the clusters in turn, dearest first, so cluster 0 has the longest list: its total is what is minimised.
-// The constants rank the shapes, they do not predict times: a group of a short prompt takes twice kExpand (see above).
-// Against every other (TN, S), on 20 shapes of 1024..34816 rows, 4096..17408 columns and 24..1500 tokens: the choice was the
-// fastest on 18. 5120 x 17408 at M = 24: 32 tokens and three splits 23.6 us, two 31.5, four 36.8, one 55.1; 6144 x 5120 at
-// M = 100: two splits 17.7, one 22.0; 34816 x 5120 at M = 520: 192 tokens 137, 224 148, 160 152, 128 176. Where kExpand misleads
-// it, tiles come out too narrow: 34816 x 5120 at M = 1024 128 tokens 284 us, 224 277; 12288 x 4096 at M = 200 96 tokens 32.1
-// us, 224 25.2.
+// The constants rank the shapes, they do not predict times: a group of a short prompt takes about one and a half times kExpand (see
+// above). Against every other (TN, S), on 22 shapes of 1024..34816 rows, 4096..17408 columns and 17..1500 tokens: the choice was the
+// fastest on 17. 5120 x 17408 at M = 24: 32 tokens and three splits 20.1 us, two 25.7, one 45.0; 6144 x 5120 at M = 100: two
+// splits 13.2, one 15.7; 34816 x 5120 at M = 520: 192 tokens 141, 224 149, 160 161, 128 182. Where kExpand misleads it, tiles
+// come out too narrow: 12288 x 4096 at M = 200 96 tokens 30.7 us, 224 23.2; 8192 x 5120 at M = 777 96 tokens 69.1, 224 55.1; 34816 x 5120
+// at M = 1024 128 tokens 285, 256 271; 1024 x 4096 at M = 64 32 tokens in four splits 6.6, 64 tokens 5.8. Too wide: 34816 x 5120 at M = 777
+// 224 tokens 208, 160 203.
 // `only` > 0 asks for that number of splits. The choice goes by what a B200 of 148 SMs runs (index S: clusters of 2 S CTAs
 // at once, as cudaOccupancyMaxActiveClusters answers on two of them), not by what this device's GPCs happen to fit, so that a
 // row has the same bits on every GPU; the device only rules out clusters it cannot run at all and sizes the grid.
@@ -618,6 +620,9 @@ PrefillPlan plan_prefill(int M, int pairs, int G, const int* device_clusters, in
       }
     }
   }
+  // A multiple of the teams: tiles of 224 tokens keep four stages of the six that would fit, of 128 twelve of fourteen. Two teams and six
+  // (fourteen) stages -> four teams and four (twelve), in us: 34816 x 5120 at M = 200 55.8 -> 55.4, 16384 x 5120 at M = 210 28.48 -> 28.43, 5120 x
+  // 17408 at M = 209 35.3 -> 34.8; at 128 tokens 16384 x 5120 at M = 112 20.0 -> 19.1, 34816 x 5120 at M = 128 39.4 -> 37.7.
   best.wdepth = kPMaxWD;
   while (best.wdepth > kPTeams && prefill_smem(best.tn, best.wdepth) > smem_optin) best.wdepth -= kPTeams;
   best.smem = prefill_smem(best.tn, best.wdepth);

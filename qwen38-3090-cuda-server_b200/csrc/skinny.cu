@@ -115,8 +115,9 @@ struct Geo {
   static constexpr int kThreads = kWarps * 32;
   // The block size the compiler plans for sets the register limit: 80 (24 warps), 72 (asked for with 896 threads) or 64 (with
   // 1024). The pre-pass's CTAs of the NEXT call want to sit beside this kernel's (4096 registers each): 24 warps
-  // of 80 leave room for one, of 72 for two, of 64 for four. Taken is what was fastest over the layers (M = 15 spills 36 bytes at
-  // 64 and gains all the same). 34816 x 5120 / 5120 x 17408 / 16384 x 5120 / 5120 x 6144 in us:
+  // of 80 leave room for one, of 72 for two, of 64 for four. Taken is what was fastest over the layers, on the build before the waits lost
+  // their hint and the split tiles' reader its tests (M = 15 then spilled 36 bytes at 64; now no int4 instance spills, M = 6, 9 and 12 take
+  // 66, 75 and 61 registers, and M = 9 would spill 20 and 80 bytes at 72). 34816 x 5120 / 5120 x 17408 / 16384 x 5120 / 5120 x 6144 in us:
   //           80 registers                72                          64
   //   M = 4   19.1 / 14.2 / 11.8 /  9.7   19.3 / 14.4 / 11.9 /  9.6   19.5 / 14.5 / 12.0 /  9.5
   //   M = 6   20.5 / 14.2 / 12.2 /  8.2   20.7 / 13.6 / 12.3 /  8.4   20.6 / 13.6 / 12.3 /  8.3
@@ -125,10 +126,11 @@ struct Geo {
   //   M = 15  28.2 / 19.6 / 16.5 / 12.2   28.0 / 19.1 / 16.2 / 11.6   27.5 / 17.1 / 15.5 / 10.3
   // and earlier M = 8 80 -> 64 22.4 / 14.3 / - / 10.1 -> 22.7 / 14.0 / - / 9.2, M = 16 72 -> 64 30.5 / 19.1 / - / 12.7 -> 28.9 / 17.1 / - / 11.1
   // (those with 17408 x 5120 in the second place).
-  // Int8 weights keep 80 at M = 6 and 15: their instances spill more (M = 15 4 bytes of stores at 80, 76 at 64; M = 6 12 and, at 72,
-  // 36), and they serve heads, where the room for the next pre-pass counts for little. Heads of 248320 x 5120 / 131072 x 4096 /
-  // 65536 x 2048 / 32768 x 1024 (rows x columns) in us: M = 15, 64 -> 80: 223.2 / 102.7 / 36.8 / 18.0 -> 200.1 / 93.2 / 35.3 / 17.1 (a
-  // layer of 5120 x 6144 12.7 -> 12.4); M = 6, 72 -> 80: 190.6 / 86.6 / 30.6 / 14.2 -> 190.4 / 86.4 / 30.5 / 14.1.
+  // Int8 weights keep 80 at M = 6 and 15: their instances spill more (bytes of stores and loads: M = 15 4 and 16 at 80, 48 and 44 at
+  // 64; M = 6 8 and 48, at 72 24 and 84), and they serve heads, where the room for the next pre-pass counts for little. Heads of
+  // 248320 x 5120 / 131072 x 4096 / 65536 x 2048 / 32768 x 1024 (rows x columns) in us, on that earlier build: M = 15, 64 -> 80:
+  // 223.2 / 102.7 / 36.8 / 18.0 -> 200.1 / 93.2 / 35.3 / 17.1 (a layer of 5120 x 6144 12.7 -> 12.4); M = 6, 72 -> 80: 190.6 / 86.6 / 30.6 / 14.2 ->
+  // 190.4 / 86.4 / 30.5 / 14.1.
   template <int WB>
   static constexpr int bound_threads() {
     if (MT == 8 || MT == 12 || MT == 16) return 1024;
@@ -143,6 +145,8 @@ struct Geo {
   //   M = 4  18.40 /   -   /  6.91 -> 18.29 /   -   /  6.81    M = 6  19.15 / 11.48 / 7.86 -> 18.77 / 11.28 / 7.78
   //   M = 8  20.37 / 12.24 /  8.26 -> 19.38 / 11.67 /  8.08    M = 15 26.26 / 15.17 / 10.16 -> 24.41 / 14.61 / 10.17
   //   M = 16 26.43 / 15.46 / 10.27 -> 25.84 / 15.17 / 10.24
+  // and with int8 weights, heads of 248320 x 5120 / 131072 x 4096 / 32768 x 1024 / a layer of 5120 x 6144, three conversions -> now at M = 8
+  // 193.17 / 86.92 / 14.01 / 9.67 -> 192.48 / 86.50 / 13.93 / 9.60, at M = 16 200.99 / 93.85 / 16.19 / 10.94 -> 200.64 / 93.61 / 16.00 / 10.79;
   // and where it was not taken, magic -> kJoin: M = 9 22.14 / 12.98 / 8.57 -> 22.65 / 13.38 / 8.78, M = 12 23.98 / 14.08 / 9.42 -> 23.53 / 14.24 / 9.58.
   static constexpr bool kJoin = MT == 4 || MT == 6 || MT == 8 || MT == 15 || MT == 16;
   static constexpr bool kTopConvert = MT == 6 || MT == 16;
@@ -161,7 +165,10 @@ struct Geo {
   static constexpr bool kIssuerWaitsD = DD2 < 8;
   // The issuers' three tests of a step in flight together (one that is over already costs 74 cycles). 34816 x 5120 / 16384 x 5120 / 5120 x 6144 /
   // 5120 x 17408 at M = 16 in us: 25.94 / 15.46 / 10.29 / 18.23 ->
-  // 25.35 / 14.87 / 9.94 / 17.62, heads the same. At the other token counts the longer code costs as much or more (M = 8 19.37 / 11.75 / 8.07 -> 19.98 / 12.09 / 8.16).
+  // 25.35 / 14.87 / 9.94 / 17.62, heads the same. M = 8 loses (19.37 / 11.75 / 8.07 -> 19.98 / 12.09 / 8.16); M = 6, 9 and 12 gain nothing (first, third
+  // and fourth of these layers: M = 6 18.82 / 7.84 / 12.62 -> 18.89 / 7.90 / 12.59, M = 9 22.11 / 8.52 / 15.31 -> 22.13 / 8.54 / 15.19, M = 12 24.00 / 9.45 /
+  // 15.34 -> 23.93 / 9.51 / 15.33; int8 head of 248320 x 5120 at M = 9 197.2 -> 199.0). M = 13 to 15 would gain as well, it was measured later and is
+  // not taken so far: M = 15 24.59 / 14.79 / 10.25 / 16.20 -> 24.60 / 14.31 / 10.02 / 15.76, int8 head 202.1 -> 202.7.
   static constexpr bool kTogether = MT == 16;
   static_assert(!kTogether || kIssuerWaitsD, "three waits");
   // A round of the fix-up warps is one step, except at M = 1, where two steps' loads are in flight together.
@@ -312,7 +319,7 @@ struct SegIter {
   }
 };
 
-// Step table entry, written by the producer, read by the MMA issuers and the fix-up warps:
+// Step table entry, written by the producer, read by the fix-up warps and (M < 16; at M = 16 the slots follow from the step) the MMA issuers:
 //   x = slot0 | slot1 << 8 | (groups - 1) << 16 | last step of its segment << 17 | whole tile << 18 | first k group << 19
 //   y = row tile
 __device__ __forceinline__ uint32_t step_word(int slot0, int slot1, int ng, bool seg_last, bool whole, int g0) {
@@ -784,37 +791,37 @@ __global__ void __launch_bounds__(Geo<MT>::template bound_threads<WB>(), 1) k_sk
           }
           e = 2u * (t & (BD - 1)) * 0x101u + 0x100u;  // the two halves of digit-ring slot t % BD
         } else {
-        // A written (its writers also saw the step's weights and table entry landed), and the D slot this
-        // step fills has been read out by every fix-up warp
-        if (!warp_agrees(mbar_wait_bounded(afull_a + a * 8, static_cast<uint32_t>(t / AD2) & 1u, kSpinLimit) &&
-                         (!GE::kIssuerWaitsD || t < DD2 ||
-                          mbar_wait_bounded(dempty_a + d * 8, static_cast<uint32_t>(t / DD2 - 1) & 1u, kSpinLimit)))) {
-          atomicExch(p.status, W4A16_ETIMEOUT);
-          break;
-        }
-        e = table[t & (kTable - 1)].x;
-        if constexpr (kStream) {
-          // the step's digit rows have landed in their ring slot (bulk copy: async proxy, as the MMA reads them)
-          if (!warp_agrees(mbar_wait_bounded(bfull_a + (t & (BD - 1)) * 8, static_cast<uint32_t>(t >> BS) & 1u, kSpinLimit))) {
+          // A written (its writers also saw the step's weights and table entry landed), and the D slot this
+          // step fills has been read out by every fix-up warp
+          if (!warp_agrees(mbar_wait_bounded(afull_a + a * 8, static_cast<uint32_t>(t / AD2) & 1u, kSpinLimit) &&
+                           (!GE::kIssuerWaitsD || t < DD2 ||
+                            mbar_wait_bounded(dempty_a + d * 8, static_cast<uint32_t>(t / DD2 - 1) & 1u, kSpinLimit)))) {
             atomicExch(p.status, W4A16_ETIMEOUT);
             break;
           }
-        } else if (!all_ready) {
-          // the digit rows of this step's two slots (all M tokens each) must be in shared memory
-          const volatile uint32_t* rdy = ready;
-          const uint32_t s0 = e & 0xFFu, s1 = (e >> 8) & 0xFFu, need = static_cast<uint32_t>(M);
-          uint32_t spins = 0;
-          while (rdy[s0] < need || rdy[s1] < need) {
-            if (++spins > kReadyLimit) break;
-            __nanosleep(40);
+          e = table[t & (kTable - 1)].x;
+          if constexpr (kStream) {
+            // the step's digit rows have landed in their ring slot (bulk copy: async proxy, as the MMA reads them)
+            if (!warp_agrees(mbar_wait_bounded(bfull_a + (t & (BD - 1)) * 8, static_cast<uint32_t>(t >> BS) & 1u, kSpinLimit))) {
+              atomicExch(p.status, W4A16_ETIMEOUT);
+              break;
+            }
+          } else if (!all_ready) {
+            // the digit rows of this step's two slots (all M tokens each) must be in shared memory
+            const volatile uint32_t* rdy = ready;
+            const uint32_t s0 = e & 0xFFu, s1 = (e >> 8) & 0xFFu, need = static_cast<uint32_t>(M);
+            uint32_t spins = 0;
+            while (rdy[s0] < need || rdy[s1] < need) {
+              if (++spins > kReadyLimit) break;
+              __nanosleep(40);
+            }
+            if (!warp_agrees(spins <= kReadyLimit)) {
+              atomicExch(p.status, W4A16_ETIMEOUT);
+              break;
+            }
+            __threadfence_block();
+            all_ready = mbar_test_wait(bready_a, 0);
           }
-          if (!warp_agrees(spins <= kReadyLimit)) {
-            atomicExch(p.status, W4A16_ETIMEOUT);
-            break;
-          }
-          __threadfence_block();
-          all_ready = mbar_test_wait(bready_a, 0);
-        }
         }
         tc_fence_after();
         const uint32_t d_t = tmem + GE::kDCol0 + d * GE::kDColsS;
