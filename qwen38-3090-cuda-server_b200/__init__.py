@@ -164,17 +164,19 @@ def _ptr(t):
     return t.data_ptr() if t is not None else None
 
 
-_torch = None
+_torch = _raw_stream = None
 
 
 def _stream(stream=None):
-    global _torch
+    global _torch, _raw_stream
     if stream is not None:
         return stream.cuda_stream
-    if _torch is None:
+    if _raw_stream is None:
         import torch
         _torch = torch
-    return _torch._C._cuda_getCurrentRawStream(_torch.cuda.current_device())
+        # a private function of torch; where it is missing, the stream's object has the handle
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda dev: torch.cuda.current_stream(dev).cuda_stream)
+    return _raw_stream(_torch.cuda.current_device())
 
 
 # --------------------------------------------------------------------- weights

@@ -1,6 +1,7 @@
 """The C-ABI library loads on a machine without a GPU and exports every declared entry point."""
 import ctypes
 import re
+import types
 
 import pytest
 
@@ -49,3 +50,18 @@ def test_struct_layouts_match_header(pkg):
     assert ctypes.sizeof(pkg.Scratch) == 56
     assert ctypes.sizeof(pkg.Workspace) == 32
     assert ctypes.sizeof(pkg.W8Weights) == 32   # 2 pointers + 4 ints
+
+
+@pytest.mark.parametrize("private", [True, False])
+def test_current_stream_with_and_without_torchs_private_function(pkg, monkeypatch, private):
+    torch = pytest.importorskip("torch")
+    if private:
+        monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda dev: 1000 + dev, raising=False)
+    else:
+        monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+        monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: types.SimpleNamespace(cuda_stream=1000 + dev))
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(pkg, "_raw_stream", None)
+    monkeypatch.setattr(pkg, "_torch", None)
+    assert pkg._stream() == 1003
+    assert pkg._stream(types.SimpleNamespace(cuda_stream=7)) == 7
